@@ -1433,7 +1433,6 @@ int ark_autotune(ark_ctx *ctx, int steps_per_candidate, int *choice) {
         else if (which == 4) ctx->x1_lines = v;
         else ctx->p1_chunk = v;
     };
-    if (ctx->x1_lines <= 0) ctx->x1_lines = x_lines_per_warp(ctx->g, !fp32);
     for (int which = 0; which < 6; ++which) {
         // segment lengths: the steps between also move the blocks' last wave
         const int segs[8] = {8, 12, 16, 20, 24, 32, 48, 64};

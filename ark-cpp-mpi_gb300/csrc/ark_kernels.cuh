@@ -1702,15 +1702,20 @@ __device__ __forceinline__ int zface(int s, int C3, bool periodic) {
 // generation fcur, new faces go to fcur^1.
 
 template <class T>
-__device__ __forceinline__ void sweep_x_body(const DevState<T> &S, int con, int fcur, int glines, const BIx &bx) {
+__device__ __forceinline__ void sweep_x_body(const DevState<T> &S, int con, int fcur, int glines, const BIx &bx, int nch = 0) {
     const Geom g = S.g;
     const int lane = threadIdx.x & 31;
     const int nlines = g.C2 * g.C3;
-    const int first = (bx.x * 4 + (threadIdx.x >> 5)) * glines; // the warp's first line
+    const int wq = bx.x * 4 + (threadIdx.x >> 5);
+    // nch > 0: the warp takes nch chunks of the stream of all lines' positions, from position
+    // wq * (32 nch - 1): its first position is the last one of the warp before, computed again
+    // for the face between the two
+    const int start = wq * (32 * nch - 1);
+    const int first = nch ? start / (g.C1 + 2) : wq * glines; // the warp's first line
     if (first >= nlines) return;
-    const int nl = nlines - first < glines ? nlines - first : glines;
+    const int nl = nch ? nlines - first : nlines - first < glines ? nlines - first : glines;
     const int nd = g.C1 + 1, npos = g.C1 + 2; // cells 0..C1+1 of a line
-    const int total = nl * npos;              // positions of the warp's stream
+    const int total = nch ? 32 * nch : nl * npos; // positions of the warp's stream
     const SweepSrc<T> R = sweep_src(S, con, fcur, 0);
     const FaceOut<T> W = sweep_out(S, fcur, 0);
     const NCell<T> N = {R.nN, R.nA, R.nB, R.nR, R.nc};
@@ -1749,8 +1754,9 @@ __device__ __forceinline__ void sweep_x_body(const DevState<T> &S, int con, int 
         deltas(P);
     };
     Pos cp;
-    cp.li = lane / npos;
-    cp.s = lane - cp.li * npos;
+    cp.s = (nch ? start - first * npos : 0) + lane;
+    cp.li = cp.s / npos;
+    cp.s -= cp.li * npos;
     cp.c0 = cp.f0 = 0;
     if (cp.li < nl) locate(cp);
     deltas(cp);
@@ -1771,6 +1777,7 @@ __device__ __forceinline__ void sweep_x_body(const DevState<T> &S, int con, int 
     for (int p0 = 0; p0 < total; p0 += 32) {
         const bool act = cp.li < nl;
         const int s = cp.s, c0 = cp.c0, f0 = cp.f0, dc = cp.dc, db = cp.db, dp = cp.dp;
+        const bool lead = p0 == 0 && lane == 0; // nothing behind it in this warp
         Pos np = cp;
         advance(np);
         if (np.li < nl) {
@@ -1784,7 +1791,7 @@ __device__ __forceinline__ void sweep_x_body(const DevState<T> &S, int con, int 
         rqb.r = __shfl_up_sync(0xffffffffu, rqf.r, 1);
         rqb.q = __shfl_up_sync(0xffffffffu, rqf.q, 1);
         if (lane == 0) rqb = carry_rq;
-        if (act && s == 0) rqb = face_rq(R.FN[ARK_CK(f0 + db, R.nf)], R.FP[ARK_CK(f0 + db, R.nf)], q);
+        if (act && (s == 0 || lead)) rqb = face_rq(R.FN[ARK_CK(f0 + s + db, R.nf)], R.FP[ARK_CK(f0 + s + db, R.nf)], q);
         carry_rq.r = __shfl_sync(0xffffffffu, rqf.r, 31);
         carry_rq.q = __shfl_sync(0xffffffffu, rqf.q, 31);
         Ext<T> e = {};
@@ -1824,7 +1831,7 @@ __device__ __forceinline__ void sweep_x_body(const DevState<T> &S, int con, int 
         carry.bf = __shfl_sync(0xffffffffu, e.bf, 31);
         carry_u = __shfl_sync(0xffffffffu, cur.nN, 31);
         carry_fl = (uint8_t)__shfl_sync(0xffffffffu, (int)cur.fl, 31);
-        if (act && s >= 1)
+        if (act && s >= 1 && !lead)
             face_update<T, false>(N, W, c0 + s - 1 + dp, c0 + s + dc, f0 + s, flb, cur.fl, ucb, cur.nN, prev, e, uA_b,
                                   uB_b, q);
         cur = nxt;
@@ -1836,8 +1843,8 @@ __device__ __forceinline__ void sweep_x_body(const DevState<T> &S, int con, int 
 
 template <class T>
 __global__ void __launch_bounds__(128, sizeof(T) == 4 ? 6 : 3)
-    k_sweep_x(const __grid_constant__ DevState<T> S, int con, int fcur, int glines) {
-    sweep_x_body<T>(S, con, fcur, glines, bix_here());
+    k_sweep_x(const __grid_constant__ DevState<T> S, int con, int fcur, int glines, int nch) {
+    sweep_x_body<T>(S, con, fcur, glines, bix_here(), nch);
 }
 
 // The x faces that Phase1 + stress with the x1 sweep folded in leaves (stg::phase1_tma_body
@@ -2498,28 +2505,76 @@ template <class T> void Launch<T>::use_forces(const DevState<T> &S, int ncon, cu
     k_use_forces<T><<<cell_grid(S.g), dim3(kCellBX, kCellBY), 0, st>>>(S, ncon);
 }
 
-// Segments of at most 32 faces, balanced so no thread gets a short tail.
-// segments of at most `target` faces, balanced
-inline int sweep_segment(int nd, int target, int *nseg) {
-    const int n = (nd + target - 1) / target;
-    *nseg = n;
-    return (nd + n - 1) / n;
+// How the sweeps of a small grid are cut.  With few lines the fixed cuts (segments of 16-20 faces,
+// warps of 3-4 whole x lines) leave most SMs idle behind a serial chain of cells (about 3 us per
+// cell and warp in FP64): 64x32x32 in FP64 ran x1 on 64 blocks of nine 32-position chunks (34 us)
+// and x2 / x3 on 32 blocks of 18 cells (67 / 58 us).  A cut costs the work of the SM with the most
+// blocks: (blocks per SM) x (cells or chunks a block marches through, the overlap cell of a segment
+// included).  An SM's rate hardly drops with one or two blocks on it (FP64: one block of 4 warps
+// alone takes 1.4 times its share; FP32, waiting on memory, needs three): sm_load's least.
+inline double sm_load(long long blocks, bool fp64) {
+    const long long per = (blocks + 151) / 152;
+    const double least = fp64 ? 1.4 : 3.0;
+    return per > least ? (double)per : least;
+}
+// Chunks of 32 positions per warp of the x1 sweep (0: whole lines, gl per warp): taken where they
+// cost at least 5% less.  FP64, us: 64x32x32 34 -> 13 (2 chunks; 1 chunk 16, 3 chunks 18),
+// 200x60x1 136 -> 17 (1 chunk), 128x64x64 83 -> 71; 256x128x128 keeps its lines.
+inline int x_chunk_blocks(const Geom &g, int nch) {
+    const long long total = (long long)g.C2 * g.C3 * (g.C1 + 2), per = 32 * nch - 1;
+    return (int)(((total - 1 + per - 1) / per + 3) / 4);
+}
+inline int x_chunks_per_warp(const Geom &g, int gl, bool fp64) {
+    const int lines = g.C2 * g.C3;
+    const double whole = sm_load((lines + 4 * gl - 1) / (4 * gl), fp64) * ((gl * (g.C1 + 2) + 31) / 32);
+    double best = 0.95 * whole;
+    int nch = 0;
+    for (int n = 1; n <= 12; ++n) {
+        const double cost = sm_load(x_chunk_blocks(g, n), fp64) * (n + 0.1);
+        if (cost < best) {
+            best = cost;
+            nch = n;
+        }
+    }
+    return nch;
+}
+// Segments of the x2 / x3 sweeps: of at most `target` faces, balanced so no thread gets a short
+// tail; where those are fewer than two waves (four blocks of 4 warps per SM), FP64 takes the count
+// with the least load instead.  us: 64x32x32 66 / 56 -> 23 / 16 (2 faces; 1 face 27 / 19, 4 faces
+// 26 / 18), 200x60x1 x2 153 -> 28 (1 face), 96x64x64 89 / 77 -> 69 / 61.
+inline int sweep_segment(int nd, int target, int blocks, bool fp64, int *nseg) {
+    int n = (nd + target - 1) / target;
+    if (fp64 && (long long)blocks * n < 2 * 4 * 152) {
+        double best = sm_load((long long)blocks * n, true) * ((nd + n - 1) / n + 1);
+        for (int m = n + 1; m <= nd; ++m) {
+            const double cost = sm_load((long long)blocks * m, true) * ((nd + m - 1) / m + 1);
+            if (cost < best) {
+                best = cost;
+                n = m;
+            }
+        }
+    }
+    const int seg = (nd + n - 1) / n;
+    *nseg = (nd + seg - 1) / seg;
+    return seg;
 }
 
 template <class T>
 void Launch<T>::sweep(const DevState<T> &S, int con, int fcur, int axis, cudaStream_t st, int target, int xlines) {
     if (axis == 0) {
         const int lines_x = S.g.C2 * S.g.C3, gl = xlines > 0 ? xlines : x_lines_per_warp(S.g, sizeof(T) == 8);
-        const dim3 grid((lines_x + 4 * gl - 1) / (4 * gl)); // 4 warps of gl lines
-        k_sweep_x<T><<<grid, 128, 0, st>>>(S, con, fcur, gl);
+        const int nch = xlines > 0 ? 0 : x_chunks_per_warp(S.g, gl, sizeof(T) == 8);
+        // 4 warps of nch chunks, or of gl lines
+        const dim3 grid(nch ? x_chunk_blocks(S.g, nch) : (lines_x + 4 * gl - 1) / (4 * gl));
+        k_sweep_x<T><<<grid, 128, 0, st>>>(S, con, fcur, gl, nch);
     } else if (axis == 1) {
         int nseg;
-        const int seg = sweep_segment(S.g.C2 + 1, target, &nseg);
+        const int seg = sweep_segment(S.g.C2 + 1, target, col_sweep_blocks(S.g, 1), sizeof(T) == 8, &nseg);
         const dim3 grid(col_sweep_blocks(S.g, 1), 1, nseg);
         k_sweep_col<T, 1><<<grid, 128, 0, st>>>(S, con, fcur, seg);
     } else {
         int nseg;
-        const int seg = sweep_segment(S.g.C3 + 1, target, &nseg);
+        const int seg = sweep_segment(S.g.C3 + 1, target, col_sweep_blocks(S.g, 2), sizeof(T) == 8, &nseg);
         const dim3 grid(col_sweep_blocks(S.g, 2), 1, nseg);
         k_sweep_col<T, 2><<<grid, 128, 0, st>>>(S, con, fcur, seg);
     }
