@@ -441,14 +441,8 @@ template <class T> struct EngineT : Engine {
         const int xg = ctx->p2mode >= 1 && ctx->p2mode <= 3 ? 1 : 0;
         const bool nofill = skip_phase2_fill();
         if (!ev) {
-            // captured: the ghost fill (the "Con" level's ghosts) beside dt (the partial slots
-            // and the scalars): independent work, both done before Phase1
-            cudaEventRecord(ctx->fill_fork, st);
-            cudaStreamWaitEvent(ctx->fill, ctx->fill_fork, 0);
-            Launch<T>::wrap_con(S, y, xg ? 2 : nofill ? 0 : 1, ctx->fill);
-            cudaEventRecord(ctx->fill_join, ctx->fill);
-            Launch<T>::finalize_dt(S, 1, st);
-            cudaStreamWaitEvent(st, ctx->fill_join, 0);
+            // captured: dt and the ghost fill of the "Con" level in one launch
+            Launch<T>::step_begin(S, y, xg ? 2 : nofill ? 0 : 1, st);
         } else { // timed one launch after the other
             Launch<T>::finalize_dt(S, 1, st);
             mark();
@@ -691,8 +685,6 @@ ark_ctx *ark_create(const ark_params *params, int *status) {
     cudaDeviceGetStreamPriorityRange(&prio_low, &prio_high);
     if (cudaStreamCreateWithPriority(&ctx->st, cudaStreamNonBlocking, prio_high) != cudaSuccess ||
         cudaStreamCreateWithPriority(&ctx->fill, cudaStreamNonBlocking, prio_high) != cudaSuccess ||
-        cudaEventCreateWithFlags(&ctx->fill_fork, cudaEventDisableTiming) != cudaSuccess ||
-        cudaEventCreateWithFlags(&ctx->fill_join, cudaEventDisableTiming) != cudaSuccess ||
         cudaEventCreateWithFlags(&ctx->seam_fork, cudaEventDisableTiming) != cudaSuccess ||
         cudaEventCreateWithFlags(&ctx->seam_join, cudaEventDisableTiming) != cudaSuccess) {
         *status = fail(ARK_ERR_CUDA, "cudaStreamCreate failed");
@@ -771,8 +763,6 @@ int ark_destroy(ark_ctx *ctx) {
         cudaStreamSynchronize(ctx->fill);
         cudaStreamDestroy(ctx->fill);
     }
-    if (ctx->fill_fork) cudaEventDestroy(ctx->fill_fork);
-    if (ctx->fill_join) cudaEventDestroy(ctx->fill_join);
     if (ctx->seam_fork) cudaEventDestroy(ctx->seam_fork);
     if (ctx->seam_join) cudaEventDestroy(ctx->seam_join);
     for (int b = 0; b < 2; ++b) {

@@ -84,7 +84,7 @@ __device__ __forceinline__ BIx decode(const WorkList &W, int q, int b) {
 
 using DS = DevState<float>;
 
-__global__ void __launch_bounds__(1024) kb_finalize(const DS *__restrict__ inst, int advance) {
+__global__ void __launch_bounds__(kBuckets) kb_finalize(const DS *__restrict__ inst, int advance) {
     finalize_dt_body<float>(inst[blockIdx.x], advance);
 }
 
@@ -600,10 +600,10 @@ void ens_step(ark_ensemble *E, int x, int fc, cudaEvent_t *ev) {
         cudaStreamWaitEvent(E->fill, E->fill_fork, 0);
         kb_wrap<<<grid_of(E, WL_WRAP), 128, 0, E->fill>>>(E->d_inst, E->d_jobs + (size_t)y * E->n, wl(E, WL_WRAP));
         cudaEventRecord(E->fill_join, E->fill);
-        kb_finalize<<<E->n, 1024, 0, E->st>>>(E->d_inst, 1);
+        kb_finalize<<<E->n, kBuckets, 0, E->st>>>(E->d_inst, 1);
         cudaStreamWaitEvent(E->st, E->fill_join, 0);
     } else { // timed one launch after the other
-        kb_finalize<<<E->n, 1024, 0, E->st>>>(E->d_inst, 1);
+        kb_finalize<<<E->n, kBuckets, 0, E->st>>>(E->d_inst, 1);
         mark(0);
         kb_wrap<<<grid_of(E, WL_WRAP), 128, 0, E->st>>>(E->d_inst, E->d_jobs + (size_t)y * E->n, wl(E, WL_WRAP));
         mark(1);

@@ -329,6 +329,8 @@ template <class T> struct Launch {
     static void finalize_dt(const DevState<T> &S, int advance_time, cudaStream_t st);
     // with_ro: 1 also roCon on z, 2 on x and z (for the one-kernel Phase2 forms)
     static void wrap_con(const DevState<T> &S, int con, int with_ro, cudaStream_t st);
+    // finalize_dt (advancing the time) and wrap_con in one launch
+    static void step_begin(const DevState<T> &S, int con, int with_ro, cudaStream_t st);
     // xlines: also the x ghosts (the one-kernel Phase2 forms read them; the x1 sweep does not)
     static void wrap_phase2(const DevState<T> &S, int con, int fcur, cudaStream_t st, int xlines = 0);
     // kch: planes per block of the staged and face-centric forms (0: their default)
