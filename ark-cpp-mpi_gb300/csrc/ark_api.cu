@@ -666,6 +666,26 @@ size_t ark_face_count(const ark_params *p) {
     return p ? (size_t)(p->n1_cells + 3) * (p->n2_cells + 3) * (p->n3_cells + 3) : 0;
 }
 
+// The TMA-staged tile (march 6: 128 x 2, 4: 64 x 4, 5: 32 x 8 cells) for a plane of C1 x C2 cells:
+// the least padded area, each tile's weighted by what it costs on a plane that it fills (w128, w64,
+// w32: Phase1 + stress with the sweeps 1 : 1.016 : 1.08 at 512x256x256, mostly the tile seams).  At
+// 150x67x93 the 128-wide tile leaves 41% of its lanes idle: the step takes 121 us on it, 94 on 32 x 8
+// tiles (Phase1 + stress with the sweeps 62 -> 46, the second Phase1 28 -> 23).
+static int tile_shape(int C1, int C2, double w128, double w64, double w32) {
+    const double w[3] = {w128, w64, w32};
+    int best = 0;
+    double least = 1e300;
+    for (int q = 0; q < 3; ++q) {
+        const int tx = 128 >> q, ty = 2 << q;
+        const double area = w[q] * ((C1 + tx - 1) / tx * tx) * (double)((C2 + ty - 1) / ty * ty);
+        if (area < least) {
+            least = area;
+            best = q;
+        }
+    }
+    return best == 0 ? 6 : best == 1 ? 4 : 5;
+}
+
 ark_ctx *ark_create(const ark_params *params, int *status) {
     int dummy;
     if (!status) status = &dummy;
@@ -713,14 +733,15 @@ ark_ctx *ark_create(const ark_params *params, int *status) {
         // 1.032 ms and the seams 0.055 + 0.029 ms, against 0.538 + 0.421 + 0.374 for the three
         // kernels.  On 64 x 4 tiles: 2.012 ms.  Smaller grids (form 5 on 64 x 4 / 128 x 2 tiles
         // against form 0, ms per step): 256x128x128 0.329 / 0.324 against 0.353, 128x64x64
-        // 0.0606 / 0.0595 against 0.0734, 64x48x48 0.0451 / 0.0461 against 0.0522
+        // 0.0606 / 0.0595 against 0.0734, 64x48x48 0.0451 / 0.0461 against 0.0522.  Where the
+        // widths leave lanes idle, the tile with the least padding (tile_shape)
         ctx->p2mode = 5;
-        if (params->n1_cells >= 128) ctx->march[0] = 6;
+        ctx->march[0] = tile_shape(params->n1_cells, params->n2_cells, 1.0, 1.016, 1.08);
     }
     // x2/x3 segments: 20 faces for FP64 (0.531 / 0.508 -> 0.513 / 0.492 ms at 256x128x128 against
     // 32), 16 for FP32 (what the autotuner picks at 512x256x256)
     ctx->seg_target = params->precision == ARK_FP32 ? 16 : 20;
-    ctx->march[1] = params->precision == ARK_FP32 ? 4 : 3;
+    ctx->march[1] = params->precision == ARK_FP32 ? tile_shape(params->n1_cells, params->n2_cells, 1e9, 1.0, 1.03) : 3;
     if (const char *e = std::getenv("ARK_PHASE1_MARCH")) { // "ab": a for Phase1 with stress, b without
         // 0: one cell per thread, 1: marching, 2: planes staged in shared memory (FP32 only),
         // 3: face quantities computed once (FP64 only), 4: staged with TMA copies (FP32 only),
@@ -1477,7 +1498,7 @@ int ark_autotune(ark_ctx *ctx, int steps_per_candidate, int *choice) {
         choice[1] = ctx->march[1];
         choice[2] = ctx->seg_target;
         choice[3] = (int)std::lround(best);
-        choice[4] = ctx->p2mode;
+        choice[4] = std::min(ctx->p2mode, 4); // 4: folded, the x1 sweep alone or with the x3 sweep
     }
     return ARK_OK;
 }

@@ -203,12 +203,37 @@ inline int staged_chunk(const Geom &g) {
     return (int)k;
 }
 inline dim3 staged_grid(const Geom &g, int kch) { return dim3(tiles_x(g), (g.C2 + SY - 1) / SY, (g.C3 + kch - 1) / kch); }
-// The same for a TSX x TSY tile of the TMA form.
-template <int TSX, int TSY> inline int tile_chunk(const Geom &g) {
-    const long long cols = (long long)((g.C1 + TSX - 1) / TSX) * ((g.C2 + TSY - 1) / TSY);
-    long long k = (long long)g.C3 * cols / (152 * 2 * 8);
-    k = k < 8 ? 8 : (k > 64 ? 64 : k);
-    return (int)k;
+// Planes per block of the TMA form on `tiles` tiles: the chunk length with the least load, a wave of
+// 304 blocks (two per SM) taking the time of kch planes and of its halo planes (`halo` planes'
+// worth: the plane below is velocities and flags only, the one above those and the z faces).  A
+// GPU that holds at most one block per SM runs a plane in 0.8 of the time.  A small grid is cut
+// finely enough to fill the SMs once (64x48x48: 2 planes, 288 blocks, Phase1 + stress with the
+// sweeps 19 -> 11 us, second Phase1 9.3 -> 7.2, against 8 planes on 72 blocks; 1 plane 13, 3 planes
+// 13), a larger one in whole waves (256x128x128: 19 planes, 2.95 waves, 322 -> 295 us per step;
+// 8 planes 317, 26 planes 325).  From eight waves of 16 planes on, blocks drift apart too far for
+// whole waves to matter: about eight waves, 64 planes at most (512x256x256: 53 planes 1.966 ms; 43
+// and 64, the least by the count, 1.999 and 1.990).
+inline int fit_planes(long long tiles, int C3, double halo) {
+    const long long eight = tiles * C3 / (304 * 8);
+    if (eight >= 16) return (int)(eight < 64 ? eight : 64);
+    double best = 1e300;
+    int kbest = C3;
+    for (int n = 1; n <= C3; ++n) {
+        const int kch = (C3 + n - 1) / n;
+        if ((C3 + kch - 1) / kch != n) continue; // the same chunks as a smaller n
+        const long long blocks = tiles * n;
+        const double waves = blocks <= 152 ? 0.8 : (double)((blocks + 303) / 304);
+        const double cost = waves * (kch + halo);
+        if (cost < 0.999 * best) {
+            best = cost;
+            kbest = kch;
+        }
+    }
+    return kbest;
+}
+// The same for a TSX x TSY tile of a grid.
+template <int TSX, int TSY> inline int tile_chunk(const Geom &g, bool stress) {
+    return fit_planes((long long)((g.C1 + TSX - 1) / TSX) * ((g.C2 + TSY - 1) / TSY), g.C3, stress ? 1.0 : 0.5);
 }
 template <int TSX, int TSY> inline dim3 tile_grid(const Geom &g, int kch) {
     return dim3((g.C1 + TSX - 1) / TSX, (g.C2 + TSY - 1) / TSY, (g.C3 + kch - 1) / kch);
@@ -990,7 +1015,7 @@ inline void launch_staged_tma(const DevState<float> &S, int src, int dst, int fc
         launch_staged<MODE>(S, src, dst, fcur, st, kch_in);
         return;
     }
-    const int kch = kch_in > 0 ? (kch_in < S.g.C3 ? kch_in : S.g.C3) : tile_chunk<TSX, TSY>(S.g);
+    const int kch = kch_in > 0 ? (kch_in < S.g.C3 ? kch_in : S.g.C3) : tile_chunk<TSX, TSY>(S.g, TLayout<MODE, TSX, TSY>::STRESS);
     k_phase1_tma<MODE, TSX, TSY><<<tile_grid<TSX, TSY>(S.g, kch), dim3(TSX * TSY + 32), TLayout<MODE, TSX, TSY>::SMEM + 128, st>>>(
         S, A, src, dst, kch, fcur, XSeams{});
 }
@@ -1001,7 +1026,7 @@ template <int MODE, int TSX, int TSY, int XS>
 inline bool launch_staged_tma_xs(const DevState<float> &S, int src, int dst, int fcur, XSeams &X, cudaStream_t st, int kch_in) {
     TmaArgs A;
     if (!tma_args<MODE, TSX, TSY>(A, S, src, fcur)) return false;
-    const int kch = kch_in > 0 ? (kch_in < S.g.C3 ? kch_in : S.g.C3) : tile_chunk<TSX, TSY>(S.g);
+    const int kch = kch_in > 0 ? (kch_in < S.g.C3 ? kch_in : S.g.C3) : tile_chunk<TSX, TSY>(S.g, TLayout<MODE, TSX, TSY>::STRESS);
     X.tw = TSX;
     X.kch = kch;
     k_phase1_tma<MODE, TSX, TSY, XS>
@@ -1017,7 +1042,7 @@ inline bool launch_staged_tma_unmet(const DevState<float> &S, int src, int dst, 
     TmaArgs A;
     if (!tma_args<MODE, 64, 4>(A, S, src, fcur)) return false;
     for (unsigned kind = DOWN; kind <= TOP; kind <<= 1) A.m.bytes[kind] += extra;
-    const int kch = tile_chunk<64, 4>(S.g);
+    const int kch = tile_chunk<64, 4>(S.g, true);
     k_phase1_tma<MODE, 64, 4><<<tile_grid<64, 4>(S.g, kch), dim3(64 * 4 + 32), TLayout<MODE, 64, 4>::SMEM + 128, st>>>(S, A, src,
                                                                                                            dst, kch, fcur,
                                                                                                            XSeams{});

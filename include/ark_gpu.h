@@ -347,7 +347,8 @@ int ark_set_closure(ark_ctx *ctx, const ark_mlp *mlp, double u_tau);
  * candidate timed three times (best kept).  The results do not depend on the shapes.  choice
  * (5 ints, may be NULL): the chosen {shape 1, shape 2, segment, microseconds per step, Phase2
  * form: 0 sweep kernels, 1 one sweep kernel (only by ARK_PHASE2_FUSED=1), 2 sweeps and second
- * Phase1 in one kernel, 3 the same with TMA copies, 4 the x1 sweep folded into Phase1 + stress}. */
+ * Phase1 in one kernel, 3 the same with TMA copies, 4 the x1 sweep (or the x1 and x3 sweeps)
+ * folded into Phase1 + stress}. */
 int ark_autotune(ark_ctx *ctx, int steps_per_candidate, int *choice);
 
 /* ---- ensembles: many independent channels in one launch per phase ------------------------

@@ -47,7 +47,7 @@ def test_fp64_small_grids_match_oracle(ark, port, C, px, pz):
 
 
 @pytest.mark.parametrize("px,pz", [(1, 1), (0, 1), (1, 0)])
-@pytest.mark.parametrize("C", [(5, 3, 2), (30, 4, 9), (48, 20, 24), (70, 33, 5)])
+@pytest.mark.parametrize("C", [(5, 3, 2), (30, 4, 9), (48, 20, 24), (70, 33, 5), (150, 10, 31), (256, 5, 3)])
 def test_fp32_separate_sweeps_equal_folded_on_small_grids(ark, port, monkeypatch, C, px, pz):
     p = port.channel_params(*C, seed=23)
     st = port.channel_state(p)
