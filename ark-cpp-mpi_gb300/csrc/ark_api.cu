@@ -480,28 +480,19 @@ template <class T> struct EngineT : Engine {
             Launch<T>::phase2_fused(S, y, fcur, st);
             for (int ax = 0; ax < 3; ++ax) mark();
         } else {
-            // the seam faces of the folded sweeps: only the second Phase1 reads the x and z faces,
-            // so (captured) they are written beside the x2 sweep (and the x3 sweep), on the second
-            // stream
-            const bool beside = xs && !ev;
-            if (beside) {
-                cudaEventRecord(ctx->seam_fork, st);
-                cudaStreamWaitEvent(ctx->fill, ctx->seam_fork, 0);
-                Launch<T>::sweep_x_seams(S, y, fcur, seams, ctx->fill);
-                if (zs) Launch<T>::sweep_z_seams(S, y, fcur, seams.kch, ctx->fill);
-                cudaEventRecord(ctx->seam_join, ctx->fill);
-            }
+            // captured, the seam faces of the folded sweeps go with the x2 sweep in one launch
+            const bool merged = xs && !ev;
+            if (merged) Launch<T>::sweep_y_seams(S, y, fcur, seams, zs, st, ctx->seg_target);
             for (int ax = 0; ax < 3; ++ax) {
                 if (ax == 0 && xs) {
-                    if (!beside) Launch<T>::sweep_x_seams(S, y, fcur, seams, st);
+                    if (!merged) Launch<T>::sweep_x_seams(S, y, fcur, seams, st);
                 } else if (ax == 2 && zs) {
-                    if (!beside) Launch<T>::sweep_z_seams(S, y, fcur, seams.kch, st);
-                } else if (ax > 0 || !fold) {
+                    if (!merged) Launch<T>::sweep_z_seams(S, y, fcur, seams.kch, st);
+                } else if (ax == 1 ? !merged : ax > 0 || !fold) {
                     Launch<T>::sweep(S, y, fcur, ax, st, ctx->seg_target, ctx->x1_lines);
                 }
                 mark();
             }
-            if (beside) cudaStreamWaitEvent(st, ctx->seam_join, 0);
         }
         Launch<T>::phase1(S, x, y, fcur ^ 1, P1_FORCES | P1_RSUM, ctx->march[1], st, ctx->p1_chunk);
         mark();
@@ -703,10 +694,7 @@ ark_ctx *ark_create(const ark_params *params, int *status) {
     // learned closure's inference) only takes SMs the step's kernels leave idle
     int prio_low = 0, prio_high = 0;
     cudaDeviceGetStreamPriorityRange(&prio_low, &prio_high);
-    if (cudaStreamCreateWithPriority(&ctx->st, cudaStreamNonBlocking, prio_high) != cudaSuccess ||
-        cudaStreamCreateWithPriority(&ctx->fill, cudaStreamNonBlocking, prio_high) != cudaSuccess ||
-        cudaEventCreateWithFlags(&ctx->seam_fork, cudaEventDisableTiming) != cudaSuccess ||
-        cudaEventCreateWithFlags(&ctx->seam_join, cudaEventDisableTiming) != cudaSuccess) {
+    if (cudaStreamCreateWithPriority(&ctx->st, cudaStreamNonBlocking, prio_high) != cudaSuccess) {
         *status = fail(ARK_ERR_CUDA, "cudaStreamCreate failed");
         return nullptr;
     }
@@ -780,12 +768,6 @@ int ark_destroy(ark_ctx *ctx) {
     }
     if (ctx->fork) cudaEventDestroy(ctx->fork);
     if (ctx->join) cudaEventDestroy(ctx->join);
-    if (ctx->fill) {
-        cudaStreamSynchronize(ctx->fill);
-        cudaStreamDestroy(ctx->fill);
-    }
-    if (ctx->seam_fork) cudaEventDestroy(ctx->seam_fork);
-    if (ctx->seam_join) cudaEventDestroy(ctx->seam_join);
     for (int b = 0; b < 2; ++b) {
         if (ctx->io_dev[b]) cudaFree(ctx->io_dev[b]);
         if (ctx->io_host[b]) cudaFreeHost(ctx->io_host[b]);

@@ -2028,6 +2028,36 @@ __global__ void __launch_bounds__(128) k_sweep_z_seams(const __grid_constant__ D
     sweep_col_body<T, 2>(S, con, fcur, 1, bx);
 }
 
+// What is left of Phase2 after Phase1 + stress with the x1 (and x3) sweeps folded in, in one launch of
+// independent blocks: the x2 sweep (ny blocks, yc to a segment), the z seams (nz, zc to a seam plane)
+// and the x seams (nx).  The seam faces are 2-3% of the faces, scattered and bound by latency.  As
+// two launches on a second stream they were the longer branch of a small grid's step (64x48x48: 12
+// us beside an x2 sweep of 13.6; 32.5 -> 28.7 us per step in one launch).  A grid that fits the SMs
+// at once (first = 1) has them first, beside everything; a larger one last, where they fill the x2
+// sweep's last wave (512x256x256 with them first 2.4 us slower per step than last).
+template <class T>
+__global__ void __launch_bounds__(128, 9) k_sweep_y_seams(const __grid_constant__ DevState<T> S, int con, int fcur, int seg, int ny,
+                                                          int yc, const __grid_constant__ XSeams X, int nx, int nz, int zc, int first) {
+    int b = (int)blockIdx.x - (first ? nx + nz : 0);
+    BIx bx = {0, 0, 0, 0, 0};
+    if (b >= 0 && b < ny) {
+        bx.z = b / yc;
+        bx.x = b - bx.z * yc;
+        sweep_col_body<T, 1>(S, con, fcur, seg, bx);
+        return;
+    }
+    b = first ? (int)blockIdx.x : b - ny; // x seams, then z seams
+    if (b < nx) {
+        sweep_x_seams_body<T>(S, con, fcur, X, b * 128 + (int)threadIdx.x);
+    } else {
+        b -= nx;
+        const int p = b / zc, nch = (S.g.C3 + X.kch - 1) / X.kch;
+        bx.x = b - p * zc;
+        bx.z = p < nch ? p * X.kch : S.g.C3;
+        sweep_col_body<T, 2>(S, con, fcur, 1, bx);
+    }
+}
+
 // ---------------------------------------------------------------------------------------
 // Phase2 with the three sweeps fused.  The sweeps are independent (each reads its own face
 // set and the two cell levels, and writes its own new face generation), so one kernel can do
@@ -2231,6 +2261,62 @@ template <class T> __global__ void __launch_bounds__(256) k_mean_profile(DevStat
 // ---------------------------------------------------------------------------------------
 // launchers
 // ---------------------------------------------------------------------------------------
+
+// How the sweeps of a small grid are cut.  With few lines the fixed cuts (segments of 16-20 faces,
+// warps of 3-4 whole x lines) leave most SMs idle behind a serial chain of cells (about 3 us per
+// cell and warp in FP64): 64x32x32 in FP64 ran x1 on 64 blocks of nine 32-position chunks (34 us)
+// and x2 / x3 on 32 blocks of 18 cells (67 / 58 us).  A cut costs the work of the SM with the most
+// blocks: (blocks per SM) x (cells or chunks a block marches through, the overlap cell of a segment
+// included).  A few blocks on an SM take as long as one: sm_load's `least` (FP64: a block of 4 warps alone takes
+// 1.4 times its share; FP32, waiting on memory, is as fast with three x1 blocks, five x2 / x3 ones).
+inline double sm_load(long long blocks, double least) {
+    const long long per = (blocks + 151) / 152;
+    return per > least ? (double)per : least;
+}
+// Chunks of 32 positions per warp of the x1 sweep (0: whole lines, gl per warp): taken where they
+// cost at least 5% less.  FP64, us: 64x32x32 34 -> 13 (2 chunks; 1 chunk 16, 3 chunks 18),
+// 200x60x1 136 -> 17 (1 chunk), 128x64x64 83 -> 71; 256x128x128 keeps its lines.
+inline int x_chunk_blocks(const Geom &g, int nch) {
+    const long long total = (long long)g.C2 * g.C3 * (g.C1 + 2), per = 32 * nch - 1;
+    return (int)(((total - 1 + per - 1) / per + 3) / 4);
+}
+inline int x_chunks_per_warp(const Geom &g, int gl, bool fp64) {
+    const int lines = g.C2 * g.C3;
+    const double least = fp64 ? 1.4 : 3.0;
+    const double whole = sm_load((lines + 4 * gl - 1) / (4 * gl), least) * ((gl * (g.C1 + 2) + 31) / 32);
+    double best = 0.95 * whole;
+    int nch = 0;
+    for (int n = 1; n <= 12; ++n) {
+        const double cost = sm_load(x_chunk_blocks(g, n), least) * (n + 0.1);
+        if (cost < best) {
+            best = cost;
+            nch = n;
+        }
+    }
+    return nch;
+}
+// Segments of the x2 / x3 sweeps: of at most `target` faces, balanced so no thread gets a short
+// tail; where those are fewer than two waves of four blocks per SM (FP32: one wave of nine), the
+// count with the least load instead, if it is larger.  FP64, us: 64x32x32 66 / 56 -> 23 / 16 (2 faces; 1 face 27 /
+// 19, 4 faces 26 / 18), 200x60x1 x2 153 -> 28 (1 face), 96x64x64 89 / 77 -> 69 / 61.  FP32: 64x48x48
+// x2 13.6 -> 5.5 (2 faces instead of 13), 150x67x93 17.7 -> 15 (8 instead of 14).
+inline int sweep_segment(int nd, int target, int blocks, bool fp64, int *nseg) {
+    const double least = fp64 ? 1.4 : 5.0;
+    int n = (nd + target - 1) / target;
+    if ((long long)blocks * n < (fp64 ? 2 * 4 : 9) * 152) {
+        double best = sm_load((long long)blocks * n, least) * ((nd + n - 1) / n + 1);
+        for (int m = n + 1; m <= nd; ++m) {
+            const double cost = sm_load((long long)blocks * m, least) * ((nd + m - 1) / m + 1);
+            if (cost < best) {
+                best = cost;
+                n = m;
+            }
+        }
+    }
+    const int seg = (nd + n - 1) / n;
+    *nseg = (nd + seg - 1) / seg;
+    return seg;
+}
 
 inline int grid_for(int64_t n, int block, int cap) {
     int64_t b = (n + block - 1) / block;
@@ -2481,6 +2567,19 @@ template <class T> void Launch<T>::sweep_z_seams(const DevState<T> &S, int con, 
 }
 
 
+template <class T>
+void Launch<T>::sweep_y_seams(const DevState<T> &S, int con, int fcur, const XSeams &X, bool z, cudaStream_t st, int target) {
+    if constexpr (std::is_same<T, float>::value) {
+        const int yc = col_sweep_blocks(S.g, 1), zc = col_sweep_blocks(S.g, 2);
+        int nseg;
+        const int seg = sweep_segment(S.g.C2 + 1, target, yc, false, &nseg);
+        const int nx = (int)((seam_slots(S.g, X.tw) + 127) / 128);
+        const int nz = z ? zc * ((S.g.C3 + X.kch - 1) / X.kch + 1) : 0;
+        const int ny = yc * nseg, blocks = nx + nz + ny;
+        k_sweep_y_seams<T><<<blocks, 128, 0, st>>>(S, con, fcur, seg, ny, yc, X, nx, nz, zc, blocks <= 9 * 152);
+    }
+}
+
 template <class T> void Launch<T>::prepare() {
     if constexpr (std::is_same<T, double>::value) {
         constexpr int fb = fcs::face_smem<double>();
@@ -2539,60 +2638,6 @@ template <class T> void Launch<T>::stress(const DevState<T> &S, int con, int bul
 
 template <class T> void Launch<T>::use_forces(const DevState<T> &S, int ncon, cudaStream_t st) {
     k_use_forces<T><<<cell_grid(S.g), dim3(kCellBX, kCellBY), 0, st>>>(S, ncon);
-}
-
-// How the sweeps of a small grid are cut.  With few lines the fixed cuts (segments of 16-20 faces,
-// warps of 3-4 whole x lines) leave most SMs idle behind a serial chain of cells (about 3 us per
-// cell and warp in FP64): 64x32x32 in FP64 ran x1 on 64 blocks of nine 32-position chunks (34 us)
-// and x2 / x3 on 32 blocks of 18 cells (67 / 58 us).  A cut costs the work of the SM with the most
-// blocks: (blocks per SM) x (cells or chunks a block marches through, the overlap cell of a segment
-// included).  An SM's rate hardly drops with one or two blocks on it (FP64: one block of 4 warps
-// alone takes 1.4 times its share; FP32, waiting on memory, needs three): sm_load's least.
-inline double sm_load(long long blocks, bool fp64) {
-    const long long per = (blocks + 151) / 152;
-    const double least = fp64 ? 1.4 : 3.0;
-    return per > least ? (double)per : least;
-}
-// Chunks of 32 positions per warp of the x1 sweep (0: whole lines, gl per warp): taken where they
-// cost at least 5% less.  FP64, us: 64x32x32 34 -> 13 (2 chunks; 1 chunk 16, 3 chunks 18),
-// 200x60x1 136 -> 17 (1 chunk), 128x64x64 83 -> 71; 256x128x128 keeps its lines.
-inline int x_chunk_blocks(const Geom &g, int nch) {
-    const long long total = (long long)g.C2 * g.C3 * (g.C1 + 2), per = 32 * nch - 1;
-    return (int)(((total - 1 + per - 1) / per + 3) / 4);
-}
-inline int x_chunks_per_warp(const Geom &g, int gl, bool fp64) {
-    const int lines = g.C2 * g.C3;
-    const double whole = sm_load((lines + 4 * gl - 1) / (4 * gl), fp64) * ((gl * (g.C1 + 2) + 31) / 32);
-    double best = 0.95 * whole;
-    int nch = 0;
-    for (int n = 1; n <= 12; ++n) {
-        const double cost = sm_load(x_chunk_blocks(g, n), fp64) * (n + 0.1);
-        if (cost < best) {
-            best = cost;
-            nch = n;
-        }
-    }
-    return nch;
-}
-// Segments of the x2 / x3 sweeps: of at most `target` faces, balanced so no thread gets a short
-// tail; where those are fewer than two waves (four blocks of 4 warps per SM), FP64 takes the count
-// with the least load instead.  us: 64x32x32 66 / 56 -> 23 / 16 (2 faces; 1 face 27 / 19, 4 faces
-// 26 / 18), 200x60x1 x2 153 -> 28 (1 face), 96x64x64 89 / 77 -> 69 / 61.
-inline int sweep_segment(int nd, int target, int blocks, bool fp64, int *nseg) {
-    int n = (nd + target - 1) / target;
-    if (fp64 && (long long)blocks * n < 2 * 4 * 152) {
-        double best = sm_load((long long)blocks * n, true) * ((nd + n - 1) / n + 1);
-        for (int m = n + 1; m <= nd; ++m) {
-            const double cost = sm_load((long long)blocks * m, true) * ((nd + m - 1) / m + 1);
-            if (cost < best) {
-                best = cost;
-                n = m;
-            }
-        }
-    }
-    const int seg = (nd + n - 1) / n;
-    *nseg = (nd + seg - 1) / seg;
-    return seg;
 }
 
 template <class T>

@@ -347,6 +347,8 @@ template <class T> struct Launch {
     static void sweep_x_seams(const DevState<T> &S, int con, int fcur, const XSeams &X, cudaStream_t st);
     // the z faces it leaves with the x3 sweep folded in: below each chunk's first plane, and C3 + 1
     static void sweep_z_seams(const DevState<T> &S, int con, int fcur, int kch, cudaStream_t st);
+    // sweep_x_seams, sweep_z_seams (z: with the x3 sweep folded in) and the x2 sweep in one launch
+    static void sweep_y_seams(const DevState<T> &S, int con, int fcur, const XSeams &X, bool z, cudaStream_t st, int target);
     static void stress(const DevState<T> &S, int con, int bulk, cudaStream_t st);
     static void use_forces(const DevState<T> &S, int ncon, cudaStream_t st);
     // x2/x3 sweeps: lines cut into balanced segments of at most `target` faces

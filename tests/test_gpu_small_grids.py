@@ -1,4 +1,4 @@
-"""Small grids, whose sweeps are cut into chunks of a line and short segments: every interior array
+"""Small grids (and one of several waves), whose sweeps are cut into chunks of a line and short segments: every interior array
 against the oracle bit for bit (FP64), and FP32 with the separate sweeps against the folded ones."""
 import numpy as np
 import pytest
@@ -47,7 +47,7 @@ def test_fp64_small_grids_match_oracle(ark, port, C, px, pz):
 
 
 @pytest.mark.parametrize("px,pz", [(1, 1), (0, 1), (1, 0)])
-@pytest.mark.parametrize("C", [(5, 3, 2), (30, 4, 9), (48, 20, 24), (70, 33, 5), (150, 10, 31), (256, 5, 3)])
+@pytest.mark.parametrize("C", [(5, 3, 2), (30, 4, 9), (48, 20, 24), (70, 33, 5), (150, 10, 31), (256, 5, 3), (96, 64, 200)])
 def test_fp32_separate_sweeps_equal_folded_on_small_grids(ark, port, monkeypatch, C, px, pz):
     p = port.channel_params(*C, seed=23)
     st = port.channel_state(p)
