@@ -507,7 +507,7 @@ template <class T> struct EngineT : Engine {
     void mean_profile(int ncon, long long *acc) override { Launch<T>::mean_profile(S, ncon, acc, ctx->st); }
     void pack(int ncon, int fcur, const CellPack &a) override { output_pack<T>(S, ncon, fcur, a, ctx->st); }
     int alloc_nut() override { return S.nut ? ARK_OK : get(&S.nut, (size_t)S.g.ncell()); }
-    void plane_stats(int ncon, double *out) override { output_plane_stats<T>(S, ncon, out, ctx->st); }
+    void plane_stats(int ncon, double *scratch, double *out) override { output_plane_stats<T>(S, ncon, scratch, out, ctx->st); }
     void gather(int lvl, double *u0, double *u1, double *u2) override { closure_gather<T>(S, lvl, u0, u1, u2, ctx->st); }
     void average_add(int ncon) override { output_average_add<T>(S, ncon, ctx->avg, ctx->st); }
     void energy(int ncon, double *scratch, double *out) override { output_energy<T>(S, ncon, scratch, out, ctx->st); }
@@ -772,6 +772,8 @@ int ark_destroy(ark_ctx *ctx) {
         if (ctx->io_dev[b]) cudaFree(ctx->io_dev[b]);
         if (ctx->io_host[b]) cudaFreeHost(ctx->io_host[b]);
     }
+    if (ctx->stat_dev) cudaFree(ctx->stat_dev);
+    if (ctx->stat_host) cudaFreeHost(ctx->stat_host);
     if (ctx->ev0) cudaEventDestroy(ctx->ev0);
     if (ctx->ev1) cudaEventDestroy(ctx->ev1);
     if (ctx->st) cudaStreamDestroy(ctx->st);
@@ -1150,16 +1152,39 @@ int ark_set_scalars(ark_ctx *ctx, const ark_scalars *in) {
     return ARK_OK;
 }
 
+// The context's statistics scratch (allocated on first use, freed with the context).  A
+// stream-ordered allocation per call cost more than the kernels: the pool gives its memory back at
+// every synchronisation, so each call mapped it again.
+static int ensure_stat(ark_ctx *ctx) {
+    if (ctx->stat_host) return ARK_OK;
+    const size_t n = 9 * (size_t)ctx->g.C2;
+    if (!ctx->stat_dev && cudaMalloc(&ctx->stat_dev, sizeof(double) * (stat_scratch(ctx->g) + n)) != cudaSuccess) {
+        ctx->stat_dev = nullptr;
+        return fail(ARK_ERR_NOMEM, "statistics scratch");
+    }
+    if (cudaMallocHost(&ctx->stat_host, sizeof(double) * n) != cudaSuccess) {
+        ctx->stat_host = nullptr;
+        return fail(ARK_ERR_NOMEM, "statistics scratch");
+    }
+    return ARK_OK;
+}
+// Waits for n results of 8 bytes at `dev` in ctx->stat_host (after the launches that write them).
+static int stat_results(ark_ctx *ctx, const void *dev, size_t n) {
+    if (int rc = launch_status(ctx)) return rc;
+    ARK_CUDA(cudaMemcpyAsync(ctx->stat_host, dev, 8 * n, cudaMemcpyDeviceToHost, ctx->st));
+    ARK_CUDA(cudaStreamSynchronize(ctx->st));
+    return ARK_OK;
+}
+
 int ark_conservation_sums(ark_ctx *ctx, ark_sums *out) {
     if (int rc = check_ctx(ctx, true)) return rc;
     if (!out) return fail(ARK_ERR_PARAM, "out is NULL");
+    if (int rc = ensure_stat(ctx)) return rc;
     DevScalars *dsc = ctx->eng->scalars();
     ARK_CUDA(cudaMemsetAsync(&dsc->sums[0], 0, sizeof(long long) * 6, ctx->st));
     ctx->eng->sums(ctx->con ^ 1);
-    if (int rc = launch_status(ctx)) return rc;
-    long long v[6];
-    ARK_CUDA(cudaStreamSynchronize(ctx->st));
-    ARK_CUDA(cudaMemcpy(v, &dsc->sums[0], sizeof(v), cudaMemcpyDeviceToHost));
+    if (int rc = stat_results(ctx, &dsc->sums[0], 6)) return rc;
+    const long long *v = (const long long *)ctx->stat_host;
     const double q = 1.0 / 4294967296.0;
     out->mass = (double)v[0] * q;
     out->momentum1 = (double)v[1] * q;
@@ -1197,17 +1222,12 @@ int ark_selftest_division(long long n, unsigned long long seed, long long *misma
 int ark_mean_profile(ark_ctx *ctx, double *mean_u1, double *wall_shear) {
     if (int rc = check_ctx(ctx, true)) return rc;
     if (!mean_u1) return fail(ARK_ERR_PARAM, "mean_u1 is NULL");
+    if (int rc = ensure_stat(ctx)) return rc;
     const int n = ctx->g.C2;
-    long long *acc = nullptr;
-    ARK_CUDA(cudaMallocAsync((void **)&acc, sizeof(long long) * 2 * n, ctx->st));
+    long long *acc = (long long *)ctx->stat_dev;
     ctx->eng->mean_profile(ctx->con ^ 1, acc);
-    int rc = launch_status(ctx);
-    std::vector<long long> h(2 * (size_t)n);
-    if (!rc && cudaMemcpyAsync(h.data(), acc, sizeof(long long) * 2 * n, cudaMemcpyDeviceToHost, ctx->st) != cudaSuccess)
-        rc = fail(ARK_ERR_CUDA, "profile copy failed");
-    cudaFreeAsync(acc, ctx->st);
-    if (!rc) ARK_CUDA(cudaStreamSynchronize(ctx->st));
-    if (rc) return rc;
+    if (int rc = stat_results(ctx, acc, 2 * (size_t)n)) return rc;
+    const long long *h = (const long long *)ctx->stat_host;
     for (int j = 0; j < n; ++j)
         mean_u1[j] = h[2 * j + 1] > 0 ? ((double)h[2 * j] * (1.0 / 4294967296.0)) / (double)h[2 * j + 1] : 0.0;
     if (wall_shear) {
@@ -1579,17 +1599,11 @@ int ark_write_average_vtk(ark_ctx *ctx, const char *path, double start_time, int
 int ark_kinetic_energy(ark_ctx *ctx, double *energy) {
     if (int rc = check_ctx(ctx, true)) return rc;
     if (!energy) return fail(ARK_ERR_PARAM, "energy is NULL");
-    const int np = energy_scratch_count(ctx->g);
-    double *scratch = nullptr;
-    ARK_CUDA(cudaMallocAsync((void **)&scratch, sizeof(double) * (np + 1), ctx->st));
-    ctx->eng->energy(ctx->con ^ 1, scratch + 1, scratch);
-    int rc = launch_status(ctx);
-    double sum = 0.0;
-    if (!rc && cudaMemcpyAsync(&sum, scratch, sizeof(double), cudaMemcpyDeviceToHost, ctx->st) != cudaSuccess)
-        rc = fail(ARK_ERR_CUDA, "energy copy failed");
-    cudaFreeAsync(scratch, ctx->st);
-    if (!rc) ARK_CUDA(cudaStreamSynchronize(ctx->st));
-    if (rc) return rc;
+    if (int rc = ensure_stat(ctx)) return rc;
+    double *res = ctx->stat_dev + stat_scratch(ctx->g);
+    ctx->eng->energy(ctx->con ^ 1, ctx->stat_dev, res);
+    if (int rc = stat_results(ctx, res, 1)) return rc;
+    const double sum = ctx->stat_host[0];
     // allEnergy *= (x3_t - x3_b) * (x2_n - x2_s) * (x1_e - x1_w)  (main.cpp:2869-2870)
     const double volume = ctx->P.lz * ctx->P.ly * ctx->P.lx;
     *energy = sum * volume;
@@ -1613,15 +1627,12 @@ int ark_plane_stats(ark_ctx *ctx, double *out) {
     if (int rc = check_ctx(ctx, true)) return rc;
     if (!out) return fail(ARK_ERR_PARAM, "out is NULL");
     const size_t n = 9 * (size_t)ctx->g.C2;
-    double *d = nullptr;
-    ARK_CUDA(cudaMallocAsync((void **)&d, sizeof(double) * n, ctx->st));
-    ctx->eng->plane_stats(ctx->con ^ 1, d);
-    int rc = launch_status(ctx);
-    if (!rc && cudaMemcpyAsync(out, d, sizeof(double) * n, cudaMemcpyDeviceToHost, ctx->st) != cudaSuccess)
-        rc = fail(ARK_ERR_CUDA, "plane statistics copy failed");
-    cudaFreeAsync(d, ctx->st);
-    if (!rc) ARK_CUDA(cudaStreamSynchronize(ctx->st));
-    return rc;
+    if (int rc = ensure_stat(ctx)) return rc;
+    double *res = ctx->stat_dev + stat_scratch(ctx->g);
+    ctx->eng->plane_stats(ctx->con ^ 1, ctx->stat_dev, res);
+    if (int rc = stat_results(ctx, res, n)) return rc;
+    std::memcpy(out, ctx->stat_host, sizeof(double) * n);
+    return ARK_OK;
 }
 
 int ark_vorticity(ark_ctx *ctx, double *out) {

@@ -30,7 +30,7 @@ struct Engine {
     virtual void mean_profile(int ncon, long long *acc) = 0;
     virtual void pack(int ncon, int fcur, const CellPack &a) = 0;
     virtual int alloc_nut() = 0;
-    virtual void plane_stats(int ncon, double *out) = 0;
+    virtual void plane_stats(int ncon, double *scratch, double *out) = 0;
     virtual void gather(int lvl, double *u0, double *u1, double *u2) = 0;
     virtual void average_add(int ncon) = 0;
     virtual void energy(int ncon, double *scratch, double *out) = 0;
@@ -99,6 +99,9 @@ struct ark_ctx {
                     // folded into Phase1 + stress (a seam kernel finishes it), then the x2 and
                     // x3 sweeps, 5 the x1 and x3 sweeps folded in (two seam kernels), then the
                     // x2 sweep
+    // statistics: device scratch (stat_scratch doubles, then 9 n2_cells results) and page-locked room
+    // for the results, kept from the first call on
+    double *stat_dev = nullptr, *stat_host = nullptr;
     // output streaming: two device and two pinned host slab buffers of io_cap doubles
     double *io_dev[2] = {nullptr, nullptr};
     double *io_host[2] = {nullptr, nullptr};

@@ -2187,74 +2187,85 @@ __global__ void __launch_bounds__(SX *SY, 2) k_phase2_fused(const __grid_constan
 // conservation sums of one level (fixed point: identical for any grid)
 // ---------------------------------------------------------------------------------------
 
-template <class T> __global__ void __launch_bounds__(kTileX *kTileY) k_sums(DevState<T> S, int ncon) {
+// u1^2 + u2^2 + u3^2 summed left to right: FP32 values widened have exact products, which one FMA each
+// adds with the same rounding.
+template <class T> __device__ __forceinline__ double square_sum(double u1, double u2, double u3) {
+    if constexpr (std::is_same<T, float>::value) return __fma_rn(u3, u3, __fma_rn(u2, u2, u1 * u1));
+    else return u1 * u1 + u2 * u2 + u3 * u3;
+}
+// Rows over gridDim.y blocks per y plane (kStatWarps warps, lanes on i).  Bound by the FP64 pipe (7
+// operations per FP32 cell, 10 per FP64 cell); a 64 x 2 column tile per block, marching all planes,
+// left it waiting: 237 -> 73 us at 256x128x128 FP32.
+template <class T> __global__ void __launch_bounds__(32 * kStatWarps) k_sums(const __grid_constant__ DevState<T> S, int ncon) {
     constexpr bool DEV = Storage<T>::deviation;
-    __shared__ long long red[6][kTileX * kTileY / 32];
+    __shared__ long long red[6][kStatWarps];
     const Geom g = S.g;
     const Level<T> L = S.lv[ncon];
-    const int i = blockIdx.x * kTileX + threadIdx.x + 1;
-    const int j = blockIdx.y * kTileY + threadIdx.y + 1;
+    const int j = blockIdx.x + 1, lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     long long a[6] = {0, 0, 0, 0, 0, 0};
-    if (i <= g.C1 && j <= g.C2) {
-        int64_t c = g.cell(i, j, 1);
-        for (int k = 1; k <= g.C3; ++k, c += g.cs2) {
-            if (!(S.flags[c] & FL_EQ0)) continue;
-            const double ro = DEV ? S.k.ro0 + (double)L.ro[c] : (double)L.ro[c];
-            const double u1 = L.u1[c], u2 = L.u2[c], u3 = L.u3[c];
+    for (int k = (int)blockIdx.y * kStatWarps + w + 1; k <= g.C3; k += kStatWarps * gridDim.y) {
+        const int64_t row = g.cell(0, j, k);
+        for (int i = lane + 1; i <= g.C1; i += 32) {
+            const int64_t c = row + i;
+            const uint8_t fl = S.flags[c];
+            const T rv = L.ro[c], v1 = L.u1[c], v2 = L.u2[c], v3 = L.u3[c];
+            if (!(fl & FL_EQ0)) continue;
+            const double ro = DEV ? S.k.ro0 + widen(rv) : widen(rv);
+            const double u1 = widen(v1), u2 = widen(v2), u3 = widen(v3);
             a[0] += fixed32(ro);
             a[1] += fixed32(ro * u1);
             a[2] += fixed32(ro * u2);
             a[3] += fixed32(ro * u3);
-            a[4] += fixed32((u1 * u1 + u2 * u2 + u3 * u3) / 2);
+            a[4] += fixed32(dhalf(square_sum<T>(u1, u2, u3)));
             a[5] += 1;
         }
     }
     for (int q = 0; q < 6; ++q) a[q] = warp_sum_i64(a[q]);
-    const int t = threadIdx.y * kTileX + threadIdx.x, w = t >> 5;
-    if ((t & 31) == 0)
+    if (lane == 0)
         for (int q = 0; q < 6; ++q) red[q][w] = a[q];
     __syncthreads();
+    const int t = threadIdx.x;
     if (t < 6) {
         long long z = 0;
-        for (int v = 0; v < kTileX * kTileY / 32; ++v) z += red[t][v];
+        for (int v = 0; v < kStatWarps; ++v) z += red[t][v];
         if (z != 0)
             atomicAdd((unsigned long long *)(t < 5 ? &S.sc->sums[t] : &S.sc->sum_cells), (unsigned long long)z);
     }
 }
 
-// Mean of u1 over the fluid cells of each y plane (one block per plane), summed in exact
-// 2^-32 fixed point: acc[2*(j-1)] = sum, acc[2*(j-1)+1] = cells.  The plane mean profile
-// U(y) and, from its first and last entries, the wall shear 2*VIS*U/dx2 in the one-sided
-// wall form of StressTensor (main.cpp:924-927).
-template <class T> __global__ void __launch_bounds__(256) k_mean_profile(DevState<T> S, int ncon, long long *acc) {
-    __shared__ long long red[2][8];
+// Mean of u1 over the fluid cells of each y plane, summed in exact 2^-32 fixed point: acc[2*(j-1)] =
+// sum, acc[2*(j-1)+1] = cells (zeroed before; gridDim.y blocks per plane add into them).  The plane
+// mean profile U(y) and, from its first and last entries, the wall shear 2*VIS*U/dx2 in the one-sided
+// wall form of StressTensor (main.cpp:924-927).  One block per plane, dividing for every cell's
+// indices, took 134 us at 256x128x128 FP32, this 14.
+template <class T>
+__global__ void __launch_bounds__(32 * kStatWarps) k_mean_profile(const __grid_constant__ DevState<T> S, int ncon, long long *acc) {
+    __shared__ long long red[2][kStatWarps];
     const Geom g = S.g;
-    const int j = blockIdx.x + 1;
     const T *__restrict__ u1 = S.lv[ncon].u1;
+    const int j = blockIdx.x + 1, lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     long long s = 0, n = 0;
-    const int plane = g.C1 * g.C3;
-    for (int t = threadIdx.x; t < plane; t += blockDim.x) {
-        const int i = t % g.C1 + 1, k = t / g.C1 + 1;
-        const int64_t c = g.cell(i, j, k);
-        if (!(S.flags[c] & FL_EQ0)) continue;
-        s += fixed32((double)u1[c]);
-        n += 1;
+    for (int k = (int)blockIdx.y * kStatWarps + w + 1; k <= g.C3; k += kStatWarps * gridDim.y) {
+        const int64_t row = g.cell(0, j, k);
+#pragma unroll 4
+        for (int i = lane + 1; i <= g.C1; i += 32) {
+            const bool fluid = S.flags[row + i] & FL_EQ0;
+            const long long v = fixed32(u1[row + i]);
+            s += fluid ? v : 0;
+            n += fluid;
+        }
     }
     s = warp_sum_i64(s);
     n = warp_sum_i64(n);
-    if ((threadIdx.x & 31) == 0) {
-        red[0][threadIdx.x >> 5] = s;
-        red[1][threadIdx.x >> 5] = n;
+    if (lane == 0) {
+        red[0][w] = s;
+        red[1][w] = n;
     }
     __syncthreads();
-    if (threadIdx.x == 0) {
-        long long a = 0, b = 0;
-        for (int w = 0; w < 8; ++w) {
-            a += red[0][w];
-            b += red[1][w];
-        }
-        acc[2 * (j - 1)] = a;
-        acc[2 * (j - 1) + 1] = b;
+    if (threadIdx.x < 2) {
+        long long z = 0;
+        for (int v = 0; v < kStatWarps; ++v) z += red[threadIdx.x][v];
+        if (z) atomicAdd((unsigned long long *)&acc[2 * (j - 1) + threadIdx.x], (unsigned long long)z);
     }
 }
 
@@ -2679,12 +2690,12 @@ void Launch<T>::boundary_fill(const DevState<T> &S, int ncon, int axis, int peri
 }
 
 template <class T> void Launch<T>::mean_profile(const DevState<T> &S, int ncon, long long *acc, cudaStream_t st) {
-    k_mean_profile<T><<<S.g.C2, 256, 0, st>>>(S, ncon, acc);
+    cudaMemsetAsync(acc, 0, sizeof(long long) * 2 * S.g.C2, st);
+    k_mean_profile<T><<<dim3(S.g.C2, stat_splits(S.g)), 32 * kStatWarps, 0, st>>>(S, ncon, acc);
 }
 
 template <class T> void Launch<T>::sums(const DevState<T> &S, int ncon, cudaStream_t st) {
-    dim3 grid(tiles_x(S.g), tiles_y(S.g));
-    k_sums<T><<<grid, dim3(kTileX, kTileY), 0, st>>>(S, ncon);
+    k_sums<T><<<dim3(S.g.C2, stat_splits(S.g)), 32 * kStatWarps, 0, st>>>(S, ncon);
 }
 
 // Precision conversion for FP32 contexts (host arrays are always double).

@@ -75,78 +75,77 @@ template <class T> __global__ void k_average_add(const __grid_constant__ DevStat
     }
 }
 
-// Kinetic energy, pass 1: one block per kTileX x kTileY column tile, each thread summing its
-// column over k in order, then a fixed shared-memory tree.  Deterministic.
-constexpr int kEnergyThreads = kTileX * kTileY;
-template <class T> __global__ void __launch_bounds__(kEnergyThreads) k_energy_tiles(const __grid_constant__ DevState<T> S, int ncon, double *part) {
-    __shared__ double red[kEnergyThreads];
+// Moments of a level over the planes, pass 1: each block sums its rows of one y plane (stat_splits
+// blocks to a plane), per thread in order, then by a fixed shared-memory tree; pass 2 adds a plane's
+// blocks in order.  Deterministic.  ENERGY: u1^2 + u2^2 + u3^2 alone; else u1, u2, u3, u1^2, u2^2, u3^2,
+// u1 u2, u1 u3, u2 u3.  Each product goes into its sum as one FMA (the product of two widened FP32
+// values is exact, so those sums round as with a separate multiply).  Bound by the FP64 pipe: nine
+// FP64 operations per cell (three for the energy).  One block of 256 threads per plane, with separate
+// multiplies and converted values, took 187 us at 256x128x128 FP32 (energy 102), this 89 (33).
+template <class T, bool ENERGY>
+__global__ void __launch_bounds__(32 * kStatWarps) k_moments(const __grid_constant__ DevState<T> S, int ncon, double *part) {
+    constexpr int NQ = ENERGY ? 3 : 9; // the energy in three sums, one per component, added at the end
+    __shared__ double red[NQ][32 * kStatWarps];
     const Geom g = S.g;
     const Level<T> L = S.lv[ncon];
-    const int i = blockIdx.x * kTileX + threadIdx.x + 1;
-    const int j = blockIdx.y * kTileY + threadIdx.y + 1;
-    double e = 0.0;
-    if (i <= g.C1 && j <= g.C2)
-        for (int k = 1; k <= g.C3; ++k) {
-            const int64_t c = g.cell(i, j, k);
-            const double u1 = L.u1[c], u2 = L.u2[c], u3 = L.u3[c];
-            e += (u1 * u1 + u2 * u2 + u3 * u3) / 2;
+    const int j = blockIdx.x + 1, lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    double a[NQ] = {};
+    for (int k = (int)blockIdx.y * kStatWarps + w + 1; k <= g.C3; k += kStatWarps * gridDim.y) {
+        const int64_t row = g.cell(0, j, k);
+        const T *__restrict__ p1 = L.u1 + row, *__restrict__ p2 = L.u2 + row, *__restrict__ p3 = L.u3 + row;
+#pragma unroll 2
+        for (int i = lane + 1; i <= g.C1; i += 32) {
+            const double u1 = widen(p1[i]), u2 = widen(p2[i]), u3 = widen(p3[i]);
+            if constexpr (ENERGY) {
+                a[0] = __fma_rn(u1, u1, a[0]);
+                a[1] = __fma_rn(u2, u2, a[1]);
+                a[2] = __fma_rn(u3, u3, a[2]);
+            } else {
+                a[0] += u1;
+                a[1] += u2;
+                a[2] += u3;
+                a[3] = __fma_rn(u1, u1, a[3]);
+                a[4] = __fma_rn(u2, u2, a[4]);
+                a[5] = __fma_rn(u3, u3, a[5]);
+                a[6] = __fma_rn(u1, u2, a[6]);
+                a[7] = __fma_rn(u1, u3, a[7]);
+                a[8] = __fma_rn(u2, u3, a[8]);
+            }
         }
-    const int t = threadIdx.y * kTileX + threadIdx.x;
-    red[t] = e;
-    __syncthreads();
-    for (int h = kEnergyThreads / 2; h > 0; h >>= 1) {
-        if (t < h) red[t] += red[t + h];
-        __syncthreads();
     }
-    if (t == 0) part[blockIdx.y * gridDim.x + blockIdx.x] = red[0];
+#pragma unroll
+    for (int q = 0; q < NQ; ++q) red[q][threadIdx.x] = a[q];
+    __syncthreads();
+    // warp w of the tree sums value q = w (and w + 8): its 256 partials by eight per lane, then shuffles
+    for (int q = w; q < NQ; q += kStatWarps) {
+        double s = 0.0;
+        for (int v = 0; v < kStatWarps; ++v) s += red[q][32 * v + lane];
+        for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+        if (lane == 0) part[((size_t)q * g.C2 + blockIdx.x) * gridDim.y + blockIdx.y] = s;
+    }
 }
-
-// Pass 2: one block of 1024 threads, strided sums in order, then the same tree.
+// Plane statistics: out[9*(j-1) + q] = the mean over plane j of value q.
+__global__ void k_plane_totals(const double *part, int C2, int splits, double cells, double *out) {
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= 9 * C2) return;
+    const int j = t / 9, q = t - 9 * j;
+    const double *p = part + ((size_t)q * C2 + j) * splits;
+    double s = 0.0;
+    for (int v = 0; v < splits; ++v) s += p[v];
+    out[t] = s / cells;
+}
+// Half the sum of n block sums: one block, strided sums in order, then a fixed tree of shuffles.
 __global__ void __launch_bounds__(1024) k_energy_total(const double *part, int n, double *out) {
-    __shared__ double red[1024];
+    __shared__ double red[32];
     double e = 0.0;
     for (int q = threadIdx.x; q < n; q += 1024) e += part[q];
-    red[threadIdx.x] = e;
+    for (int o = 16; o > 0; o >>= 1) e += __shfl_xor_sync(0xffffffffu, e, o);
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = e;
     __syncthreads();
-    for (int h = 512; h > 0; h >>= 1) {
-        if ((int)threadIdx.x < h) red[threadIdx.x] += red[threadIdx.x + h];
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) *out = red[0];
-}
-
-// Plane statistics (one block per y plane, fixed-order sums): over the interior cells of plane
-// j of level ncon, the means of u1, u2, u3, u1^2, u2^2, u3^2, u1 u2, u1 u3, u2 u3 into
-// out[9*(j-1) + q].
-template <class T> __global__ void __launch_bounds__(256) k_plane_stats(const __grid_constant__ DevState<T> S, int ncon, double *out) {
-    __shared__ double red[9][256];
-    const Geom g = S.g;
-    const int j = blockIdx.x + 1;
-    const Level<T> L = S.lv[ncon];
-    double a[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
-    const int n = g.C1 * g.C3;
-    for (int t = threadIdx.x; t < n; t += blockDim.x) {
-        const int i = t % g.C1 + 1, k = t / g.C1 + 1;
-        const int64_t c = g.cell(i, j, k);
-        const double u1 = L.u1[c], u2 = L.u2[c], u3 = L.u3[c];
-        a[0] += u1;
-        a[1] += u2;
-        a[2] += u3;
-        a[3] += u1 * u1;
-        a[4] += u2 * u2;
-        a[5] += u3 * u3;
-        a[6] += u1 * u2;
-        a[7] += u1 * u3;
-        a[8] += u2 * u3;
-    }
-    for (int q = 0; q < 9; ++q) red[q][threadIdx.x] = a[q];
-    __syncthreads();
-    for (int h = 128; h > 0; h >>= 1) {
-        if ((int)threadIdx.x < h)
-            for (int q = 0; q < 9; ++q) red[q][threadIdx.x] += red[q][threadIdx.x + h];
-        __syncthreads();
-    }
-    if (threadIdx.x < 9) out[9 * (j - 1) + threadIdx.x] = red[threadIdx.x][0] / (double)n;
+    if (threadIdx.x >= 32) return;
+    e = red[threadIdx.x];
+    for (int o = 16; o > 0; o >>= 1) e += __shfl_xor_sync(0xffffffffu, e, o);
+    if (threadIdx.x == 0) *out = 0.5 * e;
 }
 
 int grid_for(int64_t n) {
@@ -166,19 +165,19 @@ template <class T> void output_average_add(const DevState<T> &S, int ncon, const
     k_average_add<T><<<grid_for(n), 256, 0, st>>>(S, ncon, A);
 }
 
-int energy_scratch_count(const Geom &g) { return tiles_x(g) * tiles_y(g); }
-
 template <class T> void output_energy(const DevState<T> &S, int ncon, double *scratch, double *out, cudaStream_t st) {
-    const dim3 grid(tiles_x(S.g), tiles_y(S.g));
-    k_energy_tiles<T><<<grid, dim3(kTileX, kTileY), 0, st>>>(S, ncon, scratch);
-    k_energy_total<<<1, 1024, 0, st>>>(scratch, (int)(grid.x * grid.y), out);
+    const dim3 grid(S.g.C2, stat_splits(S.g));
+    k_moments<T, true><<<grid, 32 * kStatWarps, 0, st>>>(S, ncon, scratch);
+    k_energy_total<<<1, 1024, 0, st>>>(scratch, (int)(3 * grid.x * grid.y), out);
 }
 
-template <class T> void output_plane_stats(const DevState<T> &S, int ncon, double *out, cudaStream_t st) {
-    k_plane_stats<T><<<S.g.C2, 256, 0, st>>>(S, ncon, out);
+template <class T> void output_plane_stats(const DevState<T> &S, int ncon, double *scratch, double *out, cudaStream_t st) {
+    const dim3 grid(S.g.C2, stat_splits(S.g));
+    k_moments<T, false><<<grid, 32 * kStatWarps, 0, st>>>(S, ncon, scratch);
+    k_plane_totals<<<(9 * S.g.C2 + 127) / 128, 128, 0, st>>>(scratch, S.g.C2, (int)grid.y, (double)S.g.C1 * S.g.C3, out);
 }
-template void output_plane_stats<double>(const DevState<double> &, int, double *, cudaStream_t);
-template void output_plane_stats<float>(const DevState<float> &, int, double *, cudaStream_t);
+template void output_plane_stats<double>(const DevState<double> &, int, double *, double *, cudaStream_t);
+template void output_plane_stats<float>(const DevState<float> &, int, double *, double *, cudaStream_t);
 
 template void output_pack<double>(const DevState<double> &, int, int, const CellPack &, cudaStream_t);
 template void output_pack<float>(const DevState<float> &, int, int, const CellPack &, cudaStream_t);

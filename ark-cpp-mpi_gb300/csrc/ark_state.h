@@ -386,6 +386,28 @@ int staging_plan_check(int C1, int C2, int C3, int kch, char *msg, int cap);
 int step2_plan_check(int C1, int C2, int C3, int kch, char *msg, int cap);
 
 // ---- output and statistics (ark_output.cu) ----
+#ifdef __CUDACC__
+// A stored value as a double.  A float is widened with integer instructions (the conversion runs at
+// the FP64 rate, 1/64 of FP32's): rebiased exponent and shifted significand; a zero keeps its sign;
+// subnormals, infinities and NaN take the conversion, as a call so that it is not evaluated ahead of
+// the branch for every value.
+__device__ __forceinline__ double widen(double v) { return v; }
+static __device__ __noinline__ double widen_call(float v) { return (double)v; }
+__device__ __forceinline__ double widen(float v) {
+    const unsigned b = __float_as_uint(v);
+    if (((b >> 23) & 0xFFu) - 1u < 254u)
+        return __hiloint2double((int)((b & 0x80000000u) | (((b & 0x7FFFFFFFu) >> 3) + 0x38000000u)), (int)(b << 29));
+    return (b << 1) == 0u ? __hiloint2double((int)b, 0) : widen_call(v);
+}
+// Rows of cells for a statistics kernel: block (x, y) of a grid of `planes` x gridDim.y blocks, 8
+// warps, takes the rows k = 8 y + warp + 1, + 8 gridDim.y, ... of plane j = x + 1, lanes on i.
+constexpr int kStatWarps = 8;
+#endif
+// blocks per y plane: about eight blocks of 8 warps per SM in all, every warp the same rows but one
+inline int stat_splits(const Geom &g) {
+    const int rows = (g.C3 + 7) / 8, want = (152 * 8 + g.C2 - 1) / g.C2, each = (rows + want - 1) / want;
+    return (rows + each - 1) / each;
+}
 // The reference's averageU arrays are (n1+1) x (n2+2) x (n3+1) = (C1+2) x (C2+3) x (C3+2)
 // (main.cpp:225-227): one j row more than the cell arrays.
 __host__ __device__ inline int64_t avg_index(const Geom &g, int i, int j, int k) {
@@ -409,10 +431,11 @@ struct CellPack {
 template <class T> void output_pack(const DevState<T> &S, int ncon, int fcur, const CellPack &a, cudaStream_t st);
 template <class T> void output_average_add(const DevState<T> &S, int ncon, const AvgArrays &A, cudaStream_t st);
 // sum over interior cells of (u1^2 + u2^2 + u3^2)/2 of level ncon into *out (device), in a
-// fixed order; scratch holds energy_scratch_count(g) doubles
-int energy_scratch_count(const Geom &g);
+// fixed order
+// (scratch: stat_scratch(g) doubles, also for the plane statistics)
+inline size_t stat_scratch(const Geom &g) { return 9 * (size_t)g.C2 * stat_splits(g); }
 // per y plane of level ncon: means of u1, u2, u3, u1^2, u2^2, u3^2, u1u2, u1u3, u2u3 (9 * C2, device)
-template <class T> void output_plane_stats(const DevState<T> &S, int ncon, double *out, cudaStream_t st);
+template <class T> void output_plane_stats(const DevState<T> &S, int ncon, double *scratch, double *out, cudaStream_t st);
 template <class T> void output_energy(const DevState<T> &S, int ncon, double *scratch, double *out, cudaStream_t st);
 
 // ---- learned closure (ark_closure.cu) ----
