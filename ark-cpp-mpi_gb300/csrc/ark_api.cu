@@ -508,7 +508,9 @@ template <class T> struct EngineT : Engine {
     void pack(int ncon, int fcur, const CellPack &a) override { output_pack<T>(S, ncon, fcur, a, ctx->st); }
     int alloc_nut() override { return S.nut ? ARK_OK : get(&S.nut, (size_t)S.g.ncell()); }
     void plane_stats(int ncon, double *scratch, double *out) override { output_plane_stats<T>(S, ncon, scratch, out, ctx->st); }
-    void gather(int lvl, double *u0, double *u1, double *u2) override { closure_gather<T>(S, lvl, u0, u1, u2, ctx->st); }
+    int closure_sample(int lvl, ark_closure_data *data, int sx, int sz, int ox, int oz, double u_tau) override {
+        return ark::closure_sample<T>(S, lvl, data, ctx->P.lx, ctx->P.ly, ctx->P.lz, ctx->P.vis, sx, sz, ox, oz, u_tau, ctx->st);
+    }
     void average_add(int ncon) override { output_average_add<T>(S, ncon, ctx->avg, ctx->st); }
     void energy(int ncon, double *scratch, double *out) override { output_energy<T>(S, ncon, scratch, out, ctx->st); }
     DevScalars *scalars() override { return S.sc; }
@@ -1548,13 +1550,7 @@ int ark_closure_sample(ark_ctx *ctx, ark_closure_data *data, int sx, int sz, int
     const long long count = closure_count(g.C1, g.C2, g.C3, sx, sz, ox, oz);
     if (count < 0) return fail(ARK_ERR_PARAM, "bad sampling lattice");
     if (count > closure_room(data)) return fail(ARK_ERR_PARAM, "dataset full");
-    double *u = nullptr;
-    const long long cells = (long long)g.C1 * g.C2 * g.C3;
-    if (int rc = closure_scratch(data, cells, &u)) return fail(rc, ark_closure_last_error());
-    ctx->eng->gather(ctx->con ^ 1, u, u + cells, u + 2 * cells);
-    if (int rc = closure_sample(data, g.C1, g.C2, g.C3, ctx->P.lx, ctx->P.ly, ctx->P.lz, ctx->P.vis, sx, sz, ox, oz, u_tau,
-                                ctx->st))
-        return fail(rc, ark_closure_last_error());
+    if (int rc = ctx->eng->closure_sample(ctx->con ^ 1, data, sx, sz, ox, oz, u_tau)) return fail(rc, ark_closure_last_error());
     return ARK_OK;
 }
 

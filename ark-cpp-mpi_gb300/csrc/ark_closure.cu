@@ -272,56 +272,131 @@ __device__ __forceinline__ void features_of(const R A[3][3], R y, R ly, R yplus_
     f[9] = ((R)0.5 * ly - fabs(y)) * yplus_scale;
 }
 
-// ---- dataset kernels (compact interior arrays [k][j][i], float) --------------------------
+// x^(1/2) and x^(1/3) of x >= 0 for the training data: the FP32 root of x (rounded to 24 bits by
+// integer instructions) and one Newton step in FP64, relative error near 1e-14 (the rows are stored
+// as FP32); values outside FP32's comfortable range take the library's FP64 root, as a call.
+static __device__ __noinline__ double sqrt_call(double x) { return sqrt(x); }
+static __device__ __noinline__ double cbrt_call(double x) { return cbrt(x); }
+__device__ __forceinline__ float to_float24(double x) { // x in [2^-100, 2^100)
+    return __uint_as_float((((unsigned)__double2hiint(x) - 0x38000000u) << 3) | ((unsigned)__double2loint(x) >> 29));
+}
+__device__ __forceinline__ bool float_range(double x) { return ((unsigned)__double2hiint(x) >> 20) - 923u < 200u; }
+// x rounded to FP32 (nearest, ties to even) with integer instructions; results outside FP32's normal
+// range take the conversion
+static __device__ __noinline__ float narrow_call(double x) { return (float)x; }
+__device__ __forceinline__ float narrow(double x) {
+    const unsigned h = (unsigned)__double2hiint(x), l = (unsigned)__double2loint(x);
+    if (((h >> 20) & 0x7FFu) - 897u >= 253u) return ((h << 1) | l) == 0u ? __uint_as_float(h) : narrow_call(x);
+    const unsigned m = (((h & 0x7FFFFFFFu) - 0x38000000u) << 3) | (l >> 29), rest = l << 3;
+    return __uint_as_float((h & 0x80000000u) | (m + (rest > 0x80000000u || (rest == 0x80000000u && (m & 1u)) ? 1u : 0u)));
+}
+__device__ __forceinline__ double root2(double x) {
+    if (!float_range(x)) return x > 0 ? sqrt_call(x) : 0.0;
+    const float r = sqrtf(to_float24(x));
+    const double y = widen(r);
+    return __fma_rn(__fma_rn(-y, y, x), widen(0.5f / r), y);
+}
+__device__ __forceinline__ double root3(double x) {
+    if (!float_range(x)) return x > 0 ? cbrt_call(x) : 0.0;
+    const float r = cbrtf(to_float24(x));
+    const double y = widen(r);
+    return __fma_rn(__fma_rn(-y * y, y, x), widen(1.0f / (3.0f * r * r)), y);
+}
+// features_of for the training data, in FP64 with the fewest operations: with W x = w cross x (the
+// antisymmetric part), W^2 = w w^T - |w|^2 I, so the mixed invariants are dot products of w, S w and
+// S S w (A's off-diagonal entries come halved): tr W^2 S = w.Sw - |w|^2 tr S, tr W^2 S^2 = |Sw|^2 - |w|^2 tr S^2, tr W^2 S W S^2 = Sw.(w x SSw).
+__device__ __forceinline__ void features_fp64(const double A[3][3], double y, double ly, double yplus_scale, double f[NIN]) {
+    const double s00 = A[0][0], s11 = A[1][1], s22 = A[2][2];
+    const double s01 = A[0][1] + A[1][0], s02 = A[0][2] + A[2][0], s12 = A[1][2] + A[2][1];
+    const double w[3] = {A[2][1] - A[1][2], A[0][2] - A[2][0], A[1][0] - A[0][1]};
+    auto mul = [&](const double x[3], double r[3]) { // S x
+        r[0] = s00 * x[0] + s01 * x[1] + s02 * x[2];
+        r[1] = s01 * x[0] + s11 * x[1] + s12 * x[2];
+        r[2] = s02 * x[0] + s12 * x[1] + s22 * x[2];
+    };
+    auto dot = [](const double x[3], const double z[3]) { return x[0] * z[0] + x[1] * z[1] + x[2] * z[2]; };
+    const double off = s01 * s01 + s02 * s02 + s12 * s12;
+    const double trS = s00 + s11 + s22, trS2 = s00 * s00 + s11 * s11 + s22 * s22 + 2.0 * off, ww = dot(w, w);
+    // S^2 : S from the rows of S (each off-diagonal of S^2 twice)
+    const double q00 = s00 * s00 + s01 * s01 + s02 * s02, q11 = s01 * s01 + s11 * s11 + s12 * s12,
+                 q22 = s02 * s02 + s12 * s12 + s22 * s22;
+    const double q01 = s00 * s01 + s01 * s11 + s02 * s12, q02 = s00 * s02 + s01 * s12 + s02 * s22,
+                 q12 = s01 * s02 + s11 * s12 + s12 * s22;
+    const double trS3 = q00 * s00 + q11 * s11 + q22 * s22 + 2.0 * (q01 * s01 + q02 * s02 + q12 * s12);
+    double v[3], z[3];
+    mul(w, v);
+    mul(v, z);
+    const double c[3] = {w[1] * z[2] - w[2] * z[1], w[2] * z[0] - w[0] * z[2], w[0] * z[1] - w[1] * z[0]};
+    const double i4 = dot(w, v) - ww * trS, i5 = dot(v, v) - ww * trS2, i6 = dot(v, c);
+    f[0] = trS;
+    f[1] = root2(trS2);
+    f[2] = root2(2.0 * ww);
+    f[3] = copysign(root3(fabs(trS3)), trS3);
+    f[4] = copysign(root3(fabs(i4)), i4);
+    f[5] = copysign(root2(root2(fabs(i5))), i5);
+    f[6] = copysign(root3(root2(fabs(i6))), i6);
+    const double sg = y > 0 ? -1.0 : (y < 0 ? 1.0 : 0.0);
+    f[7] = sg * s01;
+    f[8] = sg * -w[2];
+    f[9] = (0.5 * ly - fabs(y)) * yplus_scale;
+}
 
-template <class T> __global__ void k_gather(const __grid_constant__ DevState<T> S, int lvl, double *u0, double *u1, double *u2) {
+// ---- dataset kernels ----------------------------------------------------------------------
+// All bound by the FP64 pipe (1/64 of the FP32 rate): sums of widened values, one multiply by 1/27
+// per box instead of a division per pass, FP32 starting values for the roots.
+
+// The velocities of level lvl of a channel (periodic x and z, solid walls in y: a neighbour beyond a
+// wall counts as minus the cell), box-filtered 3 x 3 x 3, into three compact interior arrays
+// ub + m * cells ([k][j][i], FP64).  A block takes 32 x FY cells of a plane and marches up kch planes:
+// the sums along x of FY + 2 rows go through shared memory (two planes' buffers in turn, one barrier
+// per plane), the sums over x and y of the last three planes stay in registers.  Eight FP64
+// operations per value, against six and three divisions in three passes over memory: 700 us (and 32
+// for a gathered FP64 copy) -> 229 at 256x128x128, the FP64 pipe 73% busy (16 rows per block and three
+// blocks per SM, with spills, the same).
+constexpr int FY = 8;
+template <class T>
+__global__ void __launch_bounds__(32 * (FY + 2), 4) k_filter_velocity(const __grid_constant__ DevState<T> S, int lvl, double *ub, int kch) {
+    __shared__ double xs[2][3][FY + 2][32];
     const Geom g = S.g;
-    const int n = g.C1 * g.C2 * g.C3;
-    for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x) {
-        const int i = t % g.C1, r = t / g.C1, j = r % g.C2, k = r / g.C2;
-        const int64_t c = g.cell(i + 1, j + 1, k + 1);
-        u0[t] = (double)S.lv[lvl].u1[c];
-        u1[t] = (double)S.lv[lvl].u2[c];
-        u2[t] = (double)S.lv[lvl].u3[c];
-    }
-}
-
-__global__ void k_products(const double *u0, const double *u1, const double *u2, double *p, int n) {
-    for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x) {
-        const double a = u0[t], b = u1[t], c = u2[t];
-        p[0 * (size_t)n + t] = a * a;
-        p[1 * (size_t)n + t] = a * b;
-        p[2 * (size_t)n + t] = a * c;
-        p[3 * (size_t)n + t] = b * b;
-        p[4 * (size_t)n + t] = b * c;
-        p[5 * (size_t)n + t] = c * c;
-    }
-}
-
-// One three-point pass of the box filter along axis d (FP64); y treats j = -1 and j = C2 as
-// solid (sign * a_c).
-__global__ void k_filter_pass(const double *in, double *out, int C1, int C2, int C3, int d, double sign) {
-    const int n = C1 * C2 * C3;
-    for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x) {
-        const int i = t % C1, r = t / C1, j = r % C2, k = r / C2;
-        const double c = in[t];
-        double lo, hi;
-        if (d == 0) {
-            lo = in[t - i + (i == 0 ? C1 - 1 : i - 1)];
-            hi = in[t - i + (i == C1 - 1 ? 0 : i + 1)];
-        } else if (d == 1) {
-            lo = j == 0 ? sign * c : in[t - C1];
-            hi = j == C2 - 1 ? sign * c : in[t + C1];
-        } else {
-            const int pl = C1 * C2;
-            lo = in[t + ((k == 0 ? C3 - 1 : k - 1) - k) * pl];
-            hi = in[t + ((k == C3 - 1 ? 0 : k + 1) - k) * pl];
+    const int tx = threadIdx.x, ty = threadIdx.y;
+    const int i = (int)blockIdx.x * 32 + tx + 1, j = (int)blockIdx.y * FY + ty; // j: rows j0 - 1 .. j0 + FY
+    const int k0 = (int)blockIdx.z * kch + 1, k1 = k0 + kch - 1 < g.C3 ? k0 + kch - 1 : g.C3;
+    const bool live = i <= g.C1 && j >= 1 && j <= g.C2;  // a cell whose x sum is taken
+    const bool mine = live && ty >= 1 && ty <= FY;       // and whose box is this thread's
+    const int im = i == 1 ? g.C1 : i - 1, ip = i == g.C1 ? 1 : i + 1;
+    const T *const u[3] = {S.lv[lvl].u1, S.lv[lvl].u2, S.lv[lvl].u3};
+    const size_t cells = (size_t)g.C1 * g.C2 * g.C3;
+    double z0[3] = {0, 0, 0}, z1[3] = {0, 0, 0};
+    for (int p = k0 - 1; p <= k1 + 1; ++p) {
+        const int k = p < 1 ? g.C3 : p > g.C3 ? 1 : p, buf = (p - k0) & 1;
+        double x[3] = {0, 0, 0};
+        if (live) {
+            const int64_t row = g.cell(0, j, k);
+#pragma unroll
+            for (int m = 0; m < 3; ++m) {
+                x[m] = (widen(u[m][row + im]) + widen(u[m][row + i])) + widen(u[m][row + ip]);
+                xs[buf][m][ty][tx] = x[m];
+            }
         }
-        out[t] = (lo + c + hi) / 3.0;
+        __syncthreads();
+        if (mine) {
+            const size_t out = ((size_t)(p - 2) * g.C2 + (j - 1)) * g.C1 + (i - 1); // plane p - 1
+#pragma unroll
+            for (int m = 0; m < 3; ++m) {
+                // (the sign flipped as an integer: a negation of its own is an FP64 operation)
+                const double neg = __hiloint2double(__double2hiint(x[m]) ^ (int)0x80000000, __double2loint(x[m]));
+                const double lo = j == 1 ? neg : xs[buf][m][ty - 1][tx], hi = j == g.C2 ? neg : xs[buf][m][ty + 1][tx];
+                const double xy = (lo + x[m]) + hi;
+                if (p > k0) ub[m * cells + out] = ((z0[m] + z1[m]) + xy) * (1.0 / 27.0);
+                z0[m] = z1[m];
+                z1[m] = xy;
+            }
+        }
     }
 }
 
 // gradient of compact arrays at (i, j, k): x, z periodic, y walls (solid neighbour = -u_c)
+// (the off-diagonal entries halved: S and W are then plain sums and differences)
 __device__ __forceinline__ void grad_compact(const double *const u[3], int i, int j, int k, int C1, int C2, int C3,
                                              const double rdx2[3], double A[3][3]) {
     const int pl = C1 * C2, t = (k * C2 + j) * C1 + i;
@@ -331,58 +406,93 @@ __device__ __forceinline__ void grad_compact(const double *const u[3], int i, in
     for (int m = 0; m < 3; ++m) {
         const double c = u[m][t];
         const double jl = j == 0 ? -c : u[m][t - C1], jh = j == C2 - 1 ? -c : u[m][t + C1];
-        A[m][0] = (u[m][ip] - u[m][im]) * rdx2[0];
-        A[m][1] = (jh - jl) * rdx2[1];
-        A[m][2] = (u[m][kp] - u[m][km]) * rdx2[2];
+        A[m][0] = (u[m][ip] - u[m][im]) * (m == 0 ? rdx2[0] : 0.5 * rdx2[0]);
+        A[m][1] = (jh - jl) * (m == 1 ? rdx2[1] : 0.5 * rdx2[1]);
+        A[m][2] = (u[m][kp] - u[m][km]) * (m == 2 ? rdx2[2] : 0.5 * rdx2[2]);
     }
 }
 
 struct SampleArgs {
     const double *ub[3]; // filtered velocities
-    const double *pb;    // filtered products (6 fields: 11 12 13 22 23 33)
     float *feat, *targ;  // dataset rows written from `at`
     long long at;
-    int C1, C2, C3, sx, sz, ox, oz, nx, nz;
+    int sx, sz, ox, oz, nx, nz, jc;
     double rdx2[3], ly, dy, yplus_scale, rnu;
 };
 
 // Features of the filtered field and the least-squares target at the sampled cells (i = ox +
-// sx*a, k = oz + sz*b, every j); sample (a, j, b) goes to row at + (b*C2 + j)*nx + a.
-__global__ void k_samples(SampleArgs s) {
-    const int n = s.nx * s.C2 * s.nz;
-    for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x) {
-        const int a = t % s.nx, r = t / s.nx, j = r % s.C2, b = r / s.C2;
-        const int i = s.ox + s.sx * a, k = s.oz + s.sz * b;
+// sx*a, k = oz + sz*b, every j); sample (a, j, b) goes to row at + (b*C2 + j)*nx + a.  The filtered
+// products u_m u_n are needed at the samples only: a thread marches along jc rows of one (a, b), with
+// the nine cells' products of a row summed in x and z, and the sums of three rows in registers
+// (a row beyond a wall counts as the row itself).  Every product filtered everywhere took 18 passes
+// (1400 us) and 55 us of products; the samples of a 4 x 4 lattice 180 -> 165 with the products in them,
+// the FP64 pipe 83% busy.
+template <class T> __global__ void __launch_bounds__(128) k_samples(const __grid_constant__ DevState<T> S, int lvl, SampleArgs s) {
+    const Geom g = S.g;
+    const int C1 = g.C1, C2 = g.C2, C3 = g.C3;
+    const int t = (int)(blockIdx.x * blockDim.x + threadIdx.x), njc = (C2 + s.jc - 1) / s.jc;
+    const int a = t % s.nx, r = t / s.nx, b = r / njc, j0 = (r - b * njc) * s.jc;
+    if (b >= s.nz) return;
+    const int i = s.ox + s.sx * a, k = s.oz + s.sz * b; // zero-based
+    const int j1 = j0 + s.jc < C2 ? j0 + s.jc : C2;
+    const int ci[3] = {(i == 0 ? C1 - 1 : i - 1) + 1, i + 1, (i == C1 - 1 ? 0 : i + 1) + 1};
+    const int ck[3] = {(k == 0 ? C3 - 1 : k - 1) + 1, k + 1, (k == C3 - 1 ? 0 : k + 1) + 1};
+    const T *const u[3] = {S.lv[lvl].u1, S.lv[lvl].u2, S.lv[lvl].u3};
+    // the products 11 12 13 22 23 33 of row j (zero-based), summed over the nine cells
+    auto row_sum = [&](int j, double q[6]) {
+#pragma unroll
+        for (int n = 0; n < 6; ++n) q[n] = 0.0;
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            const int64_t row = g.cell(0, j + 1, ck[c]);
+#pragma unroll
+            for (int d = 0; d < 3; ++d) {
+                const double x = widen(u[0][row + ci[d]]), y = widen(u[1][row + ci[d]]), z = widen(u[2][row + ci[d]]);
+                q[0] = __fma_rn(x, x, q[0]);
+                q[1] = __fma_rn(x, y, q[1]);
+                q[2] = __fma_rn(x, z, q[2]);
+                q[3] = __fma_rn(y, y, q[3]);
+                q[4] = __fma_rn(y, z, q[4]);
+                q[5] = __fma_rn(z, z, q[5]);
+            }
+        }
+    };
+    double lo[6], mid[6], hi[6];
+    row_sum(j0, mid);
+    if (j0 > 0) row_sum(j0 - 1, lo);
+    else
+        for (int n = 0; n < 6; ++n) lo[n] = mid[n];
+    for (int j = j0; j < j1; ++j) {
+        if (j < C2 - 1) row_sum(j + 1, hi);
+        else
+            for (int n = 0; n < 6; ++n) hi[n] = mid[n];
         double A[3][3];
-        grad_compact(s.ub, i, j, k, s.C1, s.C2, s.C3, s.rdx2, A);
+        grad_compact(s.ub, i, j, k, C1, C2, C3, s.rdx2, A);
         const double y = -0.5 * s.ly + ((double)j + 0.5) * s.dy;
         double f[NIN];
-        features_of<double>(A, y, s.ly, s.yplus_scale, f);
-        const size_t cn = (size_t)s.C1 * s.C2 * s.C3, c = ((size_t)k * s.C2 + j) * s.C1 + i;
-        const double u[3] = {s.ub[0][c], s.ub[1][c], s.ub[2][c]};
-        double tau[3][3];
-        const int pidx[3][3] = {{0, 1, 2}, {1, 3, 4}, {2, 4, 5}};
+        features_fp64(A, y, s.ly, s.yplus_scale, f);
+        const size_t c = ((size_t)k * C2 + j) * C1 + i;
+        const double v[3] = {s.ub[0][c], s.ub[1][c], s.ub[2][c]};
+        double tau[6];
 #pragma unroll
-        for (int p = 0; p < 3; ++p)
-#pragma unroll
-            for (int q = 0; q < 3; ++q) tau[p][q] = s.pb[pidx[p][q] * cn + c] - u[p] * u[q];
-        const double trS = A[0][0] + A[1][1] + A[2][2];
-        const double trT = tau[0][0] + tau[1][1] + tau[2][2];
-        double num = 0.0, den = 0.0;
-#pragma unroll
-        for (int p = 0; p < 3; ++p)
-#pragma unroll
-            for (int q = 0; q < 3; ++q) {
-                const double sd = 0.5 * (A[p][q] + A[q][p]) - (p == q ? trS / 3.0 : 0.0);
-                const double td = tau[p][q] - (p == q ? trT / 3.0 : 0.0);
-                num -= td * sd;
-                den += 2.0 * sd * sd;
-            }
+        for (int n = 0; n < 6; ++n) {
+            constexpr int p[6] = {0, 0, 0, 1, 1, 2}, q[6] = {0, 1, 2, 1, 2, 2};
+            tau[n] = ((lo[n] + mid[n]) + hi[n]) * (1.0 / 27.0) - v[p[n]] * v[q[n]];
+            lo[n] = mid[n];
+            mid[n] = hi[n];
+        }
+        // -tau^d : S^d / (2 S^d : S^d), the off-diagonals twice
+        const double ts = (A[0][0] + A[1][1] + A[2][2]) * (1.0 / 3.0), tt = (tau[0] + tau[3] + tau[5]) * (1.0 / 3.0);
+        const double s00 = A[0][0] - ts, s11 = A[1][1] - ts, s22 = A[2][2] - ts;
+        const double s01 = A[0][1] + A[1][0], s02 = A[0][2] + A[2][0], s12 = A[1][2] + A[2][1];
+        const double num = -((tau[0] - tt) * s00 + (tau[3] - tt) * s11 + (tau[5] - tt) * s22 +
+                             2.0 * (tau[1] * s01 + tau[2] * s02 + tau[4] * s12));
+        const double den = 2.0 * (s00 * s00 + s11 * s11 + s22 * s22 + 2.0 * (s01 * s01 + s02 * s02 + s12 * s12));
         const double nut = den > 1e-30 ? fmax(num / den, 0.0) : 0.0;
-        const long long row = s.at + t;
+        const long long row = s.at + ((long long)b * C2 + j) * s.nx + a;
 #pragma unroll
-        for (int q = 0; q < NIN; ++q) s.feat[row * NIN + q] = (float)f[q];
-        s.targ[row] = (float)(nut * s.rnu);
+        for (int q = 0; q < NIN; ++q) s.feat[row * NIN + q] = narrow(f[q]);
+        s.targ[row] = narrow(nut * s.rnu);
     }
 }
 
@@ -871,12 +981,6 @@ template <class T> void closure_nut(const DevState<T> &S, int lvl, const void *n
 template void closure_nut<float>(const DevState<float> &, int, const void *, float, cudaStream_t);
 template void closure_nut<double>(const DevState<double> &, int, const void *, float, cudaStream_t);
 
-template <class T> void closure_gather(const DevState<T> &S, int lvl, double *u0, double *u1, double *u2, cudaStream_t st) {
-    cl::k_gather<T><<<cl::grid_for((long long)S.g.C1 * S.g.C2 * S.g.C3), 256, 0, st>>>(S, lvl, u0, u1, u2);
-}
-template void closure_gather<float>(const DevState<float> &, int, double *, double *, double *, cudaStream_t);
-template void closure_gather<double>(const DevState<double> &, int, double *, double *, double *, cudaStream_t);
-
 } // namespace ark
 
 // ---- C ABI --------------------------------------------------------------------------------
@@ -901,7 +1005,7 @@ struct ark_closure_data {
     cudaStream_t st = nullptr;
     long long cap = 0, n = 0;
     float *feat = nullptr, *targ = nullptr;
-    // FP64 filter scratch for the grid last sampled: 3 velocities, 6 products, 9 filtered, 1 temp
+    // the filtered velocities of the grid last sampled (3 compact FP64 arrays)
     double *scratch = nullptr;
     long long scratch_cells = 0;
     int last[3] = {0, 0, 0}; // grid of the last filtered field (in the scratch)
@@ -977,7 +1081,7 @@ int ark_closure_data_filtered_stats(ark_closure_data *d, double *out) {
     const int C1 = d->last[0], C2 = d->last[1], C3 = d->last[2];
     if (C1 < 1) return cfail(ARK_ERR_STATE, "no field has been sampled");
     const long long cells = (long long)C1 * C2 * C3;
-    const double *ub = d->scratch + 9 * cells;
+    const double *ub = d->scratch;
     double *o = nullptr;
     CL_CUDA(cudaMalloc(&o, sizeof(double) * 9 * C2));
     cl::k_plane_stats_compact<<<C2, 256, 0, d->st>>>(ub, ub + cells, ub + 2 * cells, C1, C2, C3, o);
@@ -1001,22 +1105,8 @@ int ark_closure_data_append(ark_closure_data *d, long long count, const float *f
 
 } // extern "C"
 
-// Used by ark_api.cu (needs the context's internals): the gather buffers for a grid's velocities
-// (3 compact interior arrays), then the samples of what was gathered into them on ctx_st.
+// Used by ark_api.cu (needs the context's internals).
 namespace ark {
-int closure_scratch(ark_closure_data *d, long long cells, double **u) {
-    if (d->scratch_cells != cells) {
-        cudaFree(d->scratch);
-        d->scratch = nullptr;
-        d->scratch_cells = 0;
-        if (cudaMalloc(&d->scratch, sizeof(double) * 19 * (size_t)cells) != cudaSuccess)
-            return cfail(ARK_ERR_NOMEM, "filter scratch allocation failed");
-        d->scratch_cells = cells;
-    }
-    *u = d->scratch;
-    return ARK_OK;
-}
-
 long long closure_count(int C1, int C2, int C3, int sx, int sz, int ox, int oz) {
     if (sx < 1 || sz < 1 || ox < 0 || oz < 0 || ox >= sx || oz >= sz || ox >= C1 || oz >= C3) return -1;
     return (long long)((C1 - ox + sx - 1) / sx) * C2 * ((C3 - oz + sz - 1) / sz);
@@ -1024,58 +1114,71 @@ long long closure_count(int C1, int C2, int C3, int sx, int sz, int ox, int oz) 
 
 long long closure_room(const ark_closure_data *d) { return d->cap - d->n; }
 
-int closure_sample(ark_closure_data *d, int C1, int C2, int C3, double lx, double ly, double lz, double vis, int sx,
-                   int sz, int ox, int oz, double u_tau, cudaStream_t ctx_st) {
+// The samples of level lvl of a context, on its stream (waited for).
+template <class T>
+int closure_sample(const DevState<T> &S, int lvl, ark_closure_data *d, double lx, double ly, double lz, double vis, int sx,
+                   int sz, int ox, int oz, double u_tau, cudaStream_t st) {
+    const int C1 = S.g.C1, C2 = S.g.C2, C3 = S.g.C3;
     const int nx = (C1 - ox + sx - 1) / sx, nz = (C3 - oz + sz - 1) / sz;
-    const long long count = (long long)nx * C2 * nz;
     const long long cells = (long long)C1 * C2 * C3;
-    double *u = d->scratch;           // 3 gathered velocities
-    double *p = u + 3 * cells;        // 6 products
-    double *ub = p + 6 * cells;       // 3 filtered velocities
-    double *pb = ub + 3 * cells;      // 6 filtered products
-    double *tmp = pb + 6 * cells;     // 1
-    CL_CUDA(cudaGetLastError());
-    CL_CUDA(cudaStreamSynchronize(ctx_st));
-    const int gb = cl::grid_for(cells);
-    cl::k_products<<<gb, 256, 0, d->st>>>(u, u + cells, u + 2 * cells, p, (int)cells);
-    for (int f = 0; f < 9; ++f) {
-        const double *src = f < 3 ? u + f * cells : p + (f - 3) * cells;
-        double *dst = f < 3 ? ub + f * cells : pb + (f - 3) * cells;
-        const double sign = f < 3 ? -1.0 : 1.0;
-        cl::k_filter_pass<<<gb, 256, 0, d->st>>>(src, dst, C1, C2, C3, 0, sign);
-        cl::k_filter_pass<<<gb, 256, 0, d->st>>>(dst, tmp, C1, C2, C3, 1, sign);
-        cl::k_filter_pass<<<gb, 256, 0, d->st>>>(tmp, dst, C1, C2, C3, 2, sign);
+    if (d->scratch_cells != cells) {
+        cudaFree(d->scratch);
+        d->scratch = nullptr;
+        d->scratch_cells = 0;
+        d->last[0] = 0;
+        if (cudaMalloc(&d->scratch, sizeof(double) * 3 * (size_t)cells) != cudaSuccess)
+            return cfail(ARK_ERR_NOMEM, "filter scratch allocation failed");
+        d->scratch_cells = cells;
     }
+    CL_CUDA(cudaStreamSynchronize(d->st));
+    // planes per block, two more starting each chunk: the least planes on the SM with the most blocks
+    // (256x128x128: 19 planes)
+    const int bx = (C1 + 31) / 32, by = (C2 + cl::FY - 1) / cl::FY;
+    int kch = C3;
+    long long least = 1ll << 60;
+    for (int n = 1; n <= C3; ++n) {
+        const int c = (C3 + n - 1) / n;
+        const long long per = ((long long)bx * by * ((C3 + c - 1) / c) + 151) / 152, load = std::max(2ll, per) * (c + 2);
+        if (load < least) {
+            least = load;
+            kch = c;
+        }
+    }
+    cl::k_filter_velocity<T><<<dim3(bx, by, (C3 + kch - 1) / kch), dim3(32, cl::FY + 2), 0, st>>>(S, lvl, d->scratch, kch);
     cl::SampleArgs s;
-    for (int m = 0; m < 3; ++m) s.ub[m] = ub + m * cells;
-    s.pb = pb;
+    for (int m = 0; m < 3; ++m) s.ub[m] = d->scratch + m * cells;
     s.feat = d->feat;
     s.targ = d->targ;
     s.at = d->n;
-    s.C1 = C1;
-    s.C2 = C2;
-    s.C3 = C3;
     s.sx = sx;
     s.sz = sz;
     s.ox = ox;
     s.oz = oz;
     s.nx = nx;
     s.nz = nz;
+    // rows per thread: two more start each march; two warps per sub-partition first
+    s.jc = 16;
+    while (s.jc > 2 && (long long)nx * nz * ((C2 + s.jc - 1) / s.jc) < 152 * 4 * 2 * 32) s.jc /= 2;
     const double dx[3] = {lx / C1, ly / C2, lz / C3};
     for (int q = 0; q < 3; ++q) s.rdx2[q] = 0.5 / dx[q];
     s.ly = ly;
     s.dy = dx[1];
     s.yplus_scale = u_tau / vis;
     s.rnu = 1.0 / vis;
-    cl::k_samples<<<cl::grid_for(count), 256, 0, d->st>>>(s);
+    const long long threads = (long long)nx * nz * ((C2 + s.jc - 1) / s.jc);
+    cl::k_samples<T><<<(unsigned)((threads + 127) / 128), 128, 0, st>>>(S, lvl, s);
     CL_CUDA(cudaGetLastError());
-    CL_CUDA(cudaStreamSynchronize(d->st));
-    d->n += count;
+    CL_CUDA(cudaStreamSynchronize(st));
+    d->n += (long long)nx * C2 * nz;
     d->last[0] = C1;
     d->last[1] = C2;
     d->last[2] = C3;
     return ARK_OK;
 }
+template int closure_sample<float>(const DevState<float> &, int, ark_closure_data *, double, double, double, double, int, int, int,
+                                   int, double, cudaStream_t);
+template int closure_sample<double>(const DevState<double> &, int, ark_closure_data *, double, double, double, double, int, int, int,
+                                    int, double, cudaStream_t);
 } // namespace ark
 
 extern "C" {

@@ -31,7 +31,7 @@ struct Engine {
     virtual void pack(int ncon, int fcur, const CellPack &a) = 0;
     virtual int alloc_nut() = 0;
     virtual void plane_stats(int ncon, double *scratch, double *out) = 0;
-    virtual void gather(int lvl, double *u0, double *u1, double *u2) = 0;
+    virtual int closure_sample(int lvl, ark_closure_data *data, int sx, int sz, int ox, int oz, double u_tau) = 0;
     virtual void average_add(int ncon) = 0;
     virtual void energy(int ncon, double *scratch, double *out) = 0;
     virtual DevScalars *scalars() = 0;

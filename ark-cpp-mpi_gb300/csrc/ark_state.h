@@ -449,8 +449,6 @@ template <class T> void closure_nut(const DevState<T> &S, int lvl, const void *n
 // bytes, which closure_nut reads
 size_t mlp_bytes();
 int mlp_snapshot_device(const ark_mlp *M, void *dev_out);
-// the interior velocities of level lvl into three compact FP64 arrays
-template <class T> void closure_gather(const DevState<T> &S, int lvl, double *u0, double *u1, double *u2, cudaStream_t st);
 // samples of a C1 x C2 x C3 grid on the lattice (sx, sz, ox, oz), or -1 for a bad lattice
 long long closure_count(int C1, int C2, int C3, int sx, int sz, int ox, int oz);
 
@@ -496,8 +494,8 @@ struct ark_closure_data;
 struct ark_mlp;
 namespace ark {
 long long closure_room(const ark_closure_data *d);
-int closure_scratch(ark_closure_data *d, long long cells, double **u);
-int closure_sample(ark_closure_data *d, int C1, int C2, int C3, double lx, double ly, double lz, double vis, int sx,
-                   int sz, int ox, int oz, double u_tau, cudaStream_t ctx_st);
+template <class T>
+int closure_sample(const DevState<T> &S, int lvl, ark_closure_data *d, double lx, double ly, double lz, double vis, int sx, int sz,
+                   int ox, int oz, double u_tau, cudaStream_t st);
 const void *mlp_device_net(const ark_mlp *M);
 } // namespace ark
