@@ -528,10 +528,6 @@ __global__ void __launch_bounds__(256) k_plane_stats_compact(const double *u0, c
     if (threadIdx.x < 9) out[9 * j + threadIdx.x] = red[threadIdx.x][0] / (double)n;
 }
 
-// ---- training kernels ---------------------------------------------------------------------
-
-constexpr int TS = 128; // samples per tile (one per thread in the elementwise phases)
-
 // ---- training on the tensor cores ---------------------------------------------------------
 // The layers' products over a tile of TS samples are warp-level BF16 matrix multiply-accumulates
 // (m16n8k16, FP32 accumulation): the forward layers Z1 = X W1^T, Z2 = H1 W2^T, the backward
@@ -543,9 +539,18 @@ constexpr int TS = 128; // samples per tile (one per thread in the elementwise p
 // keeps 8.  The elementwise parts (normalisation, GELU and its derivative, the softplus output,
 // the loss) stay in FP32 per sample.  All sums run in a fixed order, so the gradient is
 // deterministic.
-
-constexpr int LDX = 20;      // floats per staged input row (10 inputs padded to 16, + 4 against bank conflicts)
-constexpr int LDH = NH + 4;  // floats per staged hidden row
+//
+// A warp takes 16 of the tile's samples through the whole network in registers: the accumulator
+// fragment of a product (row = sample, column = unit) is the A fragment of the next one, tanh is taken
+// once per unit for GELU and its derivative, the weights' fragments are packed once per block.  Only
+// the sums over samples meet in shared memory (X, H1, H2, D2, D1 as FP32; one barrier before and
+// after): eight warps take an m16n8 tile of D2^T H1 each, four of them one of D1^T X, the other four
+// the bias sums.  With every layer's operands staged and split again for each product, a barrier
+// after each phase and tanh taken four times per unit pair, 65536 samples took 45.8 us, this 19.
+constexpr int TS = 128, GW = TS / 16;  // samples per tile, warps per block
+constexpr int LDX = 20;                // floats per staged input row (10 inputs padded to 16, + 4 against bank conflicts)
+constexpr int LDH = NH + 4;            // floats per staged hidden row
+constexpr int FR1 = 8, FR2 = 16;       // B fragments of W1^T (4 n-tiles x 2), of W2^T and of W2 (4 x 2 x 2)
 
 // a two-term BF16 expansion of a pair of values, packed as the pair registers of a fragment
 struct Pair2 {
@@ -561,243 +566,326 @@ __device__ __forceinline__ Pair2 split_pair(float a, float b) {
     r.lo = pack_bf16(a - __bfloat162float(ah), b - __bfloat162float(bh));
     return r;
 }
-
-// C[16 x 8] += A[16 x 16k] B[16k x 8] for an operand A given by element reads a(row, col) (split
-// into two BF16 terms) and B by b(row, col): exact BF16 (wexact, one term) or split (three
-// products).  Thread lane = 4 g + t holds C[g][2t], C[g][2t+1], C[g+8][2t], C[g+8][2t+1].
-template <int KSTEPS, bool B_EXACT, class FA, class FB>
-__device__ __forceinline__ void mma_tile(float c[4], int lane, FA a, FB b) {
-    const int g = lane >> 2, t = lane & 3;
+// C[16 x 8] += A[16 x TS] B[TS x 8] for operands given by element reads a(row, sample), b(sample,
+// column), both split.  Thread lane = 4 g + t holds C[g][2t], C[g][2t+1], C[g+8][2t], C[g+8][2t+1].
+template <class FA, class FB> __device__ __forceinline__ void mma_samples(float c[4], int g, int t, FA a, FB b) {
 #pragma unroll
-    for (int ks = 0; ks < KSTEPS; ++ks) {
-        const int k0 = 16 * ks;
+    for (int k0 = 0; k0 < TS; k0 += 16) {
         const Pair2 a0 = split_pair(a(g, k0 + 2 * t), a(g, k0 + 2 * t + 1));
         const Pair2 a1 = split_pair(a(g + 8, k0 + 2 * t), a(g + 8, k0 + 2 * t + 1));
         const Pair2 a2 = split_pair(a(g, k0 + 2 * t + 8), a(g, k0 + 2 * t + 9));
         const Pair2 a3 = split_pair(a(g + 8, k0 + 2 * t + 8), a(g + 8, k0 + 2 * t + 9));
         const unsigned ahi[4] = {a0.hi, a1.hi, a2.hi, a3.hi}, alo[4] = {a0.lo, a1.lo, a2.lo, a3.lo};
-        if (B_EXACT) {
-            const unsigned b0 = pack_bf16(b(k0 + 2 * t, g), b(k0 + 2 * t + 1, g));
-            const unsigned b1 = pack_bf16(b(k0 + 2 * t + 8, g), b(k0 + 2 * t + 9, g));
-            mma_bf16(c, ahi, b0, b1);
-            mma_bf16(c, alo, b0, b1);
-        } else {
-            const Pair2 b0 = split_pair(b(k0 + 2 * t, g), b(k0 + 2 * t + 1, g));
-            const Pair2 b1 = split_pair(b(k0 + 2 * t + 8, g), b(k0 + 2 * t + 9, g));
-            mma_bf16(c, ahi, b0.hi, b1.hi);
-            mma_bf16(c, ahi, b0.lo, b1.lo);
-            mma_bf16(c, alo, b0.hi, b1.hi);
-        }
+        const Pair2 b0 = split_pair(b(k0 + 2 * t, g), b(k0 + 2 * t + 1, g));
+        const Pair2 b1 = split_pair(b(k0 + 2 * t + 8, g), b(k0 + 2 * t + 9, g));
+        mma_bf16(c, ahi, b0.hi, b1.hi);
+        mma_bf16(c, ahi, b0.lo, b1.lo);
+        mma_bf16(c, alo, b0.hi, b1.hi);
     }
 }
+// GELU and its derivative (gelu, gelu_grad) from one tanh
+__device__ __forceinline__ void gelu_both(float z, float &h, float &d) {
+    const float th = tanhf(GK0 * (z + GK1 * z * z * z));
+    h = 0.5f * z * (1.0f + th);
+    d = 0.5f * (1.0f + th) + 0.5f * z * (1.0f - th * th) * GK0 * (1.0f + 3.0f * GK1 * z * z);
+}
+
+// Training alternates two short kernels, each launched while the one before still runs (programmatic
+// stream serialization): grid_release lets the next grid start, grid_wait waits for the one before to
+// have ended with its writes visible.  Before grid_wait a kernel reads only what the other does not
+// write (the samples; the moments and masters, which k_mlp_update alone writes).
+__device__ __forceinline__ void grid_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+constexpr int kMaxRows = 608; // rows of block partials: at most four blocks per SM
+
+struct GradSmem {
+    unsigned f1[FR1][32], f2[FR2][32], f2t[FR2][32]; // the weights' B fragments, per lane
+    float b1[NH], b2[NH], w3[NH], mu[16], rsd[16];
+    float D3[TS], R2[TS];                            // dL/dz3, squared errors
+    float X[TS * LDX], H1[TS * LDH], H2[TS * LDH], D2[TS * LDH], D1[TS * LDH];
+};
 
 // Gradient of the mean squared error over samples [first, first + count) of the batch map
 // (sample index = (first + q) * stride + offset), into block partials part[block][NPARAM + 1]
 // (the last entry: the block's sum of squared errors).  scale = 2 / (samples of the batch).
-__global__ void __launch_bounds__(TS, 2) k_mlp_grad(const float *__restrict__ feat, const float *__restrict__ targ,
-                                                    long long first, long long count, long long stride, long long offset,
-                                                    const Net *__restrict__ net, float scale, float *part) {
-    extern __shared__ float smem[];
-    float *w = smem;                  // NPARAM (BF16-exact working weights)
-    float *acc = w + NPARAM;          // NPARAM + 1 (this block's sums)
-    float *X = acc + NPARAM + 1;      // TS x LDX: normalised inputs, zero past NIN
-    float *Z1 = X + TS * LDX;         // TS x LDH: z1, then dL/dz1
-    float *H1 = Z1 + TS * LDH;        // TS x LDH: gelu(z1)
-    float *Z2 = H1 + TS * LDH;        // TS x LDH: z2, then dL/dz2
-    float *H2 = Z2 + TS * LDH;        // TS x LDH: gelu(z2)
-    float *D3 = H2 + TS * LDH;        // TS: dL/dz3
-    float *R2 = D3 + TS;              // TS: squared errors
-    const int t = threadIdx.x, lane = t & 31, wid = t >> 5, g = lane >> 2, tq = lane & 3;
-    for (int q = t; q < NPARAM; q += TS) {
-        w[q] = net->w[q];
-        acc[q] = 0.f;
-    }
-    if (t == 0) acc[NPARAM] = 0.f;
-    __shared__ float mu[NIN], rsd[NIN];
-    if (t < NIN) {
-        mu[t] = net->mu[t];
-        rsd[t] = net->rsd[t];
+__global__ void __launch_bounds__(32 * GW, 2) k_mlp_grad(const float *__restrict__ feat, const float *__restrict__ targ,
+                                                         long long first, long long count, long long stride, long long offset,
+                                                         const Net *__restrict__ net, float scale, float *part) {
+    extern __shared__ __align__(16) unsigned char grad_raw[];
+    GradSmem &sm = *reinterpret_cast<GradSmem *>(grad_raw);
+    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, g = lane >> 2, t = lane & 3;
+    static_assert(NPARAM <= TS * LDH, "the weights pass through H1's rows");
+    float *const w = sm.H1;
+    const int s0 = 16 * wid; // this warp's rows of a tile
+    // a tile's inputs: this lane's columns of samples g and g + 8 of the warp's, and (lanes 0 .. 15) the
+    // target of sample `lane`
+    float2 xlo[2], xhi[2];
+    float target = 0.f;
+    auto fetch = [&](long long tile) {
+#pragma unroll
+        for (int r = 0; r < 2; ++r) {
+            const long long q = tile * TS + s0 + g + 8 * r, smp = q < count ? (first + q) * stride + offset : 0;
+            xlo[r] = *reinterpret_cast<const float2 *>(feat + smp * NIN + 2 * t);
+            xhi[r] = t == 0 ? *reinterpret_cast<const float2 *>(feat + smp * NIN + 8) : make_float2(0.f, 0.f);
+        }
+        const long long q = tile * TS + s0 + lane;
+        target = lane < 16 && q < count ? targ[(first + q) * stride + offset] : 0.f;
+    };
+    fetch(blockIdx.x);
+    grid_wait();
+#pragma unroll
+    for (int q = 0; q < (NPARAM + 32 * GW - 1) / (32 * GW); ++q)
+        if (tid + q * 32 * GW < NPARAM) w[tid + q * 32 * GW] = net->w[tid + q * 32 * GW];
+    if (tid < 16) {
+        sm.mu[tid] = tid < NIN ? net->mu[tid] : 0.f;
+        sm.rsd[tid] = tid < NIN ? net->rsd[tid] : 0.f;
     }
     __syncthreads();
+    for (int f = wid; f < FR1 + 2 * FR2; f += GW) {
+        if (f < FR1) { // n-tile f / 2, register f % 2: W1 rows 8 nt + g, inputs 2t (+ 8)
+            const int n = 8 * (f >> 1) + g, k = 2 * t + 8 * (f & 1);
+            sm.f1[f][lane] = pack_bf16(k < NIN ? w[O_W1 + n * NIN + k] : 0.f, k + 1 < NIN ? w[O_W1 + n * NIN + k + 1] : 0.f);
+        } else { // n-tile q / 4, k-step (q / 2) % 2, register q % 2
+            const int q = (f - FR1) % FR2, n = 8 * (q >> 2) + g, k = 16 * ((q >> 1) & 1) + 2 * t + 8 * (q & 1);
+            if (f - FR1 < FR2) sm.f2[q][lane] = pack_bf16(w[O_W2 + n * NH + k], w[O_W2 + n * NH + k + 1]);
+            else sm.f2t[q][lane] = pack_bf16(w[O_W2 + k * NH + n], w[O_W2 + (k + 1) * NH + n]);
+        }
+    }
+    if (tid < NH) {
+        sm.b1[tid] = w[O_B1 + tid];
+        sm.b2[tid] = w[O_B2 + tid];
+        sm.w3[tid] = w[O_W3 + tid];
+    }
+    const float b3 = w[O_B3];
+    __syncthreads();
+
+    // the block's sums: this warp's fragment of D2^T H1, D1^T X, and (warps 4 ..) a lane's bias sum
+    float gw2[4] = {0.f, 0.f, 0.f, 0.f}, gw1[4] = {0.f, 0.f, 0.f, 0.f}, gb = 0.f;
     const long long ntiles = (count + TS - 1) / TS;
     for (long long tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
-        const long long q = tile * TS + t;
-        const bool live = q < count;
-        const long long smp = live ? (first + q) * stride + offset : 0;
-        // inputs (a sample past the end enters as zeros; its error and derivatives are zero)
+        // this lane's rows: samples g and g + 8 of the warp's (a sample past the end enters as zeros;
+        // its error and derivatives are zero)
+        unsigned ahi[2][4], alo[2][4]; // A fragments (two k-steps of 16)
 #pragma unroll
-        for (int i = 0; i < 16; ++i) X[t * LDX + i] = (live && i < NIN) ? (feat[smp * NIN + i] - mu[i]) * rsd[i] : 0.f;
-        __syncthreads();
-        // Z1 = X W1^T + b1: warp w takes sample rows 32w .. 32w+31 (two m-tiles), all four n-tiles
+        for (int r = 0; r < 2; ++r) {
+            const long long q = tile * TS + s0 + g + 8 * r;
+            const bool live = q < count;
+            const float2 lo = xlo[r], hi = xhi[r];
+            const float x[4] = {live ? (lo.x - sm.mu[2 * t]) * sm.rsd[2 * t] : 0.f,
+                                live ? (lo.y - sm.mu[2 * t + 1]) * sm.rsd[2 * t + 1] : 0.f,
+                                live ? (hi.x - sm.mu[2 * t + 8]) * sm.rsd[2 * t + 8] : 0.f,
+                                live ? (hi.y - sm.mu[2 * t + 9]) * sm.rsd[2 * t + 9] : 0.f};
 #pragma unroll
-        for (int mt = 0; mt < 2; ++mt)
-#pragma unroll
-            for (int nt = 0; nt < 4; ++nt) {
-                const int s0 = 32 * wid + 16 * mt, n0 = 8 * nt;
-                float c[4] = {0.f, 0.f, 0.f, 0.f};
-                mma_tile<1, true>(c, lane, [&](int r, int k) { return X[(s0 + r) * LDX + k]; },
-                                  [&](int k, int n) { return k < NIN ? w[O_W1 + (n0 + n) * NIN + k] : 0.f; });
-                const int n = n0 + 2 * tq;
-                Z1[(s0 + g) * LDH + n] = c[0] + w[O_B1 + n];
-                Z1[(s0 + g) * LDH + n + 1] = c[1] + w[O_B1 + n + 1];
-                Z1[(s0 + g + 8) * LDH + n] = c[2] + w[O_B1 + n];
-                Z1[(s0 + g + 8) * LDH + n + 1] = c[3] + w[O_B1 + n + 1];
+            for (int c = 0; c < 2; ++c) {
+                const Pair2 p = split_pair(x[2 * c], x[2 * c + 1]);
+                ahi[0][r + 2 * c] = p.hi;
+                alo[0][r + 2 * c] = p.lo;
+                *reinterpret_cast<float2 *>(&sm.X[(s0 + g + 8 * r) * LDX + 2 * t + 8 * c]) = make_float2(x[2 * c], x[2 * c + 1]);
             }
-        __syncthreads();
-        for (int k = 0; k < NH; ++k) H1[t * LDH + k] = gelu(Z1[t * LDH + k]);
-        __syncthreads();
-        // Z2 = H1 W2^T + b2
+        }
+        const long long mine = tile * TS + s0 + lane; // lanes 0 .. 15: the sample whose output they take
+        const bool live = lane < 16 && mine < count;
+        // Z1 = X W1^T + b1; H1 = gelu(Z1) (the next A fragments), d1 = gelu'(Z1)
+        float d1[4][4];
+        unsigned hhi[2][4], hlo[2][4];
+        auto put = [&](float *m, int r, int n, float a, float b) { // columns n, n + 1 of row g + 8 r
+            *reinterpret_cast<float2 *>(&m[(s0 + g + 8 * r) * LDH + n]) = make_float2(a, b);
+        };
 #pragma unroll
-        for (int mt = 0; mt < 2; ++mt)
+        for (int nt = 0; nt < 4; ++nt) {
+            float c[4] = {0.f, 0.f, 0.f, 0.f}, h[4];
+            const unsigned w0 = sm.f1[2 * nt][lane], w1 = sm.f1[2 * nt + 1][lane];
+            mma_bf16(c, ahi[0], w0, w1);
+            mma_bf16(c, alo[0], w0, w1);
+            const int n = 8 * nt + 2 * t;
+            const float2 bias = *reinterpret_cast<const float2 *>(&sm.b1[n]);
+            gelu_both(c[0] + bias.x, h[0], d1[nt][0]);
+            gelu_both(c[1] + bias.y, h[1], d1[nt][1]);
+            gelu_both(c[2] + bias.x, h[2], d1[nt][2]);
+            gelu_both(c[3] + bias.y, h[3], d1[nt][3]);
 #pragma unroll
-            for (int nt = 0; nt < 4; ++nt) {
-                const int s0 = 32 * wid + 16 * mt, n0 = 8 * nt;
-                float c[4] = {0.f, 0.f, 0.f, 0.f};
-                mma_tile<2, true>(c, lane, [&](int r, int k) { return H1[(s0 + r) * LDH + k]; },
-                                  [&](int k, int n) { return w[O_W2 + (n0 + n) * NH + k]; });
-                const int n = n0 + 2 * tq;
-                Z2[(s0 + g) * LDH + n] = c[0] + w[O_B2 + n];
-                Z2[(s0 + g) * LDH + n + 1] = c[1] + w[O_B2 + n + 1];
-                Z2[(s0 + g + 8) * LDH + n] = c[2] + w[O_B2 + n];
-                Z2[(s0 + g + 8) * LDH + n + 1] = c[3] + w[O_B2 + n + 1];
+            for (int r = 0; r < 2; ++r) {
+                const Pair2 p = split_pair(h[2 * r], h[2 * r + 1]);
+                hhi[nt >> 1][r + 2 * (nt & 1)] = p.hi;
+                hlo[nt >> 1][r + 2 * (nt & 1)] = p.lo;
+                put(sm.H1, r, n, h[2 * r], h[2 * r + 1]);
             }
-        __syncthreads();
-        // per sample: the second activation, the output, the error and dL/dz3, then dL/dz2
-        {
-            float z3 = w[O_B3];
-            for (int k = 0; k < NH; ++k) {
-                const float h2 = gelu(Z2[t * LDH + k]);
-                H2[t * LDH + k] = h2;
-                z3 += w[O_W3 + k] * h2;
+        }
+        // Z2 = H1 W2^T + b2, H2 = gelu(Z2), d2 = gelu'(Z2)
+        float d2[4][4];
+#pragma unroll
+        for (int nt = 0; nt < 4; ++nt) {
+            float c[4] = {0.f, 0.f, 0.f, 0.f}, h[4];
+#pragma unroll
+            for (int ks = 0; ks < 2; ++ks) {
+                const unsigned w0 = sm.f2[4 * nt + 2 * ks][lane], w1 = sm.f2[4 * nt + 2 * ks + 1][lane];
+                mma_bf16(c, hhi[ks], w0, w1);
+                mma_bf16(c, hlo[ks], w0, w1);
             }
-            float d3 = 0.f, r2 = 0.f;
+            const int n = 8 * nt + 2 * t;
+            const float2 bias = *reinterpret_cast<const float2 *>(&sm.b2[n]);
+            gelu_both(c[0] + bias.x, h[0], d2[nt][0]);
+            gelu_both(c[1] + bias.y, h[1], d2[nt][1]);
+            gelu_both(c[2] + bias.x, h[2], d2[nt][2]);
+            gelu_both(c[3] + bias.y, h[3], d2[nt][3]);
+            put(sm.H2, 0, n, h[0], h[1]);
+            put(sm.H2, 1, n, h[2], h[3]);
+        }
+        __syncwarp();
+        // per sample (lanes 0 .. 15): the output z3 = w3 . H2 + b3 summed in order, the error and dL/dz3
+        float d3 = 0.f, r2 = 0.f;
+        if (lane < 16) {
+            float z3 = b3;
+            const float *h = &sm.H2[(s0 + lane) * LDH];
+#pragma unroll
+            for (int k = 0; k < NH; k += 4) {
+                const float4 v = *reinterpret_cast<const float4 *>(h + k), q = *reinterpret_cast<const float4 *>(&sm.w3[k]);
+                z3 += q.x * v.x;
+                z3 += q.y * v.y;
+                z3 += q.z * v.z;
+                z3 += q.w * v.w;
+            }
             if (live) {
-                const float y = softplus(z3), r = y - targ[smp];
+                const float y = softplus(z3), r = y - target;
                 r2 = r * r;
                 d3 = scale * r * sigmoid(z3);
             }
-            D3[t] = d3;
-            R2[t] = r2;
-            for (int k = 0; k < NH; ++k) Z2[t * LDH + k] = d3 * w[O_W3 + k] * gelu_grad(Z2[t * LDH + k]);
+            sm.D3[s0 + lane] = d3;
+            sm.R2[s0 + lane] = r2;
         }
-        __syncthreads();
-        // dL/dz1 = (D2 W2) * gelu'(z1), in place of z1
-        {
-            float d1[2][4][4];
+        const float d3r[2] = {__shfl_sync(0xffffffffu, d3, g), __shfl_sync(0xffffffffu, d3, g + 8)};
+        // D2 = d3 w3 gelu'(Z2)
 #pragma unroll
-            for (int mt = 0; mt < 2; ++mt)
+        for (int nt = 0; nt < 4; ++nt) {
+            const int n = 8 * nt + 2 * t;
+            const float2 w3 = *reinterpret_cast<const float2 *>(&sm.w3[n]);
 #pragma unroll
-                for (int nt = 0; nt < 4; ++nt) {
-                    const int s0 = 32 * wid + 16 * mt, n0 = 8 * nt;
-                    float *c = d1[mt][nt];
-                    c[0] = c[1] = c[2] = c[3] = 0.f;
-                    mma_tile<2, true>(c, lane, [&](int r, int k) { return Z2[(s0 + r) * LDH + k]; },
-                                      [&](int k, int n) { return w[O_W2 + k * NH + n0 + n]; });
-                }
-            // every warp reads only its own sample rows of Z1: no barrier between
-#pragma unroll
-            for (int mt = 0; mt < 2; ++mt)
-#pragma unroll
-                for (int nt = 0; nt < 4; ++nt) {
-                    const int s0 = 32 * wid + 16 * mt, n = 8 * nt + 2 * tq;
-                    const float *c = d1[mt][nt];
-                    float *z = &Z1[(s0 + g) * LDH + n];
-                    z[0] = c[0] * gelu_grad(z[0]);
-                    z[1] = c[1] * gelu_grad(z[1]);
-                    z = &Z1[(s0 + g + 8) * LDH + n];
-                    z[0] = c[2] * gelu_grad(z[0]);
-                    z[1] = c[3] * gelu_grad(z[1]);
-                }
-        }
-        __syncthreads();
-        // weight gradients over the tile: gW2 = D2^T H1 (warp w: unit rows 16 (w & 1) .. +15,
-        // n-tiles 2 (w >> 1), +1), gW1 = D1^T X (warp w: unit rows 16 (w & 1), input n-tile w >> 1)
-        {
-            const int k0 = 16 * (wid & 1);
-#pragma unroll
-            for (int j = 0; j < 2; ++j) {
-                const int n0 = 8 * (2 * (wid >> 1) + j);
-                float c[4] = {0.f, 0.f, 0.f, 0.f};
-                mma_tile<TS / 16, false>(c, lane, [&](int r, int s) { return Z2[s * LDH + k0 + r]; },
-                                         [&](int s, int n) { return H1[s * LDH + n0 + n]; });
-                const int n = n0 + 2 * tq;
-                acc[O_W2 + (k0 + g) * NH + n] += c[0];
-                acc[O_W2 + (k0 + g) * NH + n + 1] += c[1];
-                acc[O_W2 + (k0 + g + 8) * NH + n] += c[2];
-                acc[O_W2 + (k0 + g + 8) * NH + n + 1] += c[3];
+            for (int r = 0; r < 2; ++r) {
+                const float a = d3r[r] * w3.x * d2[nt][2 * r], b = d3r[r] * w3.y * d2[nt][2 * r + 1];
+                const Pair2 p = split_pair(a, b);
+                ahi[nt >> 1][r + 2 * (nt & 1)] = p.hi;
+                alo[nt >> 1][r + 2 * (nt & 1)] = p.lo;
+                put(sm.D2, r, n, a, b);
             }
-            const int i0 = 8 * (wid >> 1);
+        }
+        // D1 = (D2 W2) gelu'(Z1)
+#pragma unroll
+        for (int nt = 0; nt < 4; ++nt) {
             float c[4] = {0.f, 0.f, 0.f, 0.f};
-            mma_tile<TS / 16, false>(c, lane, [&](int r, int s) { return Z1[s * LDH + k0 + r]; },
-                                     [&](int s, int n) { return X[s * LDX + i0 + n]; });
-            const int i = i0 + 2 * tq;
-            if (i < NIN) {
-                acc[O_W1 + (k0 + g) * NIN + i] += c[0];
-                acc[O_W1 + (k0 + g + 8) * NIN + i] += c[2];
+#pragma unroll
+            for (int ks = 0; ks < 2; ++ks) {
+                const unsigned w0 = sm.f2t[4 * nt + 2 * ks][lane], w1 = sm.f2t[4 * nt + 2 * ks + 1][lane];
+                mma_bf16(c, ahi[ks], w0, w1);
+                mma_bf16(c, alo[ks], w0, w1);
             }
-            if (i + 1 < NIN) {
-                acc[O_W1 + (k0 + g) * NIN + i + 1] += c[1];
-                acc[O_W1 + (k0 + g + 8) * NIN + i + 1] += c[3];
+            put(sm.D1, 0, 8 * nt + 2 * t, c[0] * d1[nt][0], c[1] * d1[nt][1]);
+            put(sm.D1, 1, 8 * nt + 2 * t, c[2] * d1[nt][2], c[3] * d1[nt][3]);
+        }
+        __syncthreads();
+        // weight gradients over the tile: gW2 = D2^T H1, warp w units 16 (w & 1) .. +15 by columns
+        // 8 (w >> 1) .. +7; gW1 = D1^T X, warps 0 .. 3 units 16 (w & 1) by inputs 8 (w >> 1)
+        {
+            const int k0 = 16 * (wid & 1), n0 = 8 * (wid >> 1);
+            float c[4] = {0.f, 0.f, 0.f, 0.f};
+            mma_samples(c, g, t, [&](int r, int s) { return sm.D2[s * LDH + k0 + r]; },
+                        [&](int s, int n) { return sm.H1[s * LDH + n0 + n]; });
+#pragma unroll
+            for (int q = 0; q < 4; ++q) gw2[q] += c[q];
+            if (wid < 4) {
+                float e[4] = {0.f, 0.f, 0.f, 0.f};
+                mma_samples(e, g, t, [&](int r, int s) { return sm.D1[s * LDH + k0 + r]; },
+                            [&](int s, int n) { return sm.X[s * LDX + n0 + n]; });
+#pragma unroll
+                for (int q = 0; q < 4; ++q) gw1[q] += e[q];
+            } else { // the bias gradients, the last layer's and the squared errors: sums over the tile in order
+                float sum = 0.f;
+                if (wid == 4) {
+#pragma unroll 16
+                    for (int s = 0; s < TS; ++s) sum += sm.D1[s * LDH + lane];
+                } else if (wid == 5) {
+#pragma unroll 16
+                    for (int s = 0; s < TS; ++s) sum += sm.D2[s * LDH + lane];
+                } else if (wid == 6) {
+#pragma unroll 16
+                    for (int s = 0; s < TS; ++s) sum += sm.D3[s] * sm.H2[s * LDH + lane];
+                } else if (lane < 2) {
+                    const float *v = lane ? sm.R2 : sm.D3;
+#pragma unroll 16
+                    for (int s = 0; s < TS; ++s) sum += v[s];
+                }
+                gb += sum;
             }
         }
-        // the bias gradients, the last layer's and the squared errors: sums over the tile in order
-        for (int p = t; p <= NPARAM; p += TS) {
-            float gsum = 0.f;
-            if (p >= O_B1 && p < O_W2) {
-                const int k = p - O_B1;
-                for (int s2 = 0; s2 < TS; ++s2) gsum += Z1[s2 * LDH + k];
-            } else if (p >= O_B2 && p < O_W3) {
-                const int k = p - O_B2;
-                for (int s2 = 0; s2 < TS; ++s2) gsum += Z2[s2 * LDH + k];
-            } else if (p >= O_W3 && p < O_B3) {
-                const int k = p - O_W3;
-                for (int s2 = 0; s2 < TS; ++s2) gsum += D3[s2] * H2[s2 * LDH + k];
-            } else if (p == O_B3) {
-                for (int s2 = 0; s2 < TS; ++s2) gsum += D3[s2];
-            } else if (p == NPARAM) {
-                for (int s2 = 0; s2 < TS; ++s2) gsum += R2[s2];
-            } else {
-                continue; // W1 and W2: taken by the multiplies above
-            }
-            acc[p] += gsum;
-        }
+        if (tile + gridDim.x < ntiles) fetch(tile + gridDim.x);
         __syncthreads();
     }
-    for (int p = t; p <= NPARAM; p += TS) part[(size_t)blockIdx.x * (NPARAM + 1) + p] = acc[p];
+    grid_release();
+    float *const out = part + (size_t)blockIdx.x * (NPARAM + 1);
+    const int k0 = 16 * (wid & 1) + g, n0 = 8 * (wid >> 1) + 2 * t;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        const int k = k0 + 8 * (q >> 1), n = n0 + (q & 1);
+        out[O_W2 + k * NH + n] = gw2[q];
+        if (wid < 4 && n < NIN) out[O_W1 + k * NIN + n] = gw1[q];
+    }
+    if (wid == 4) out[O_B1 + lane] = gb;
+    else if (wid == 5) out[O_B2 + lane] = gb;
+    else if (wid == 6) out[O_W3 + lane] = gb;
+    else if (wid == 7 && lane < 2) out[lane ? NPARAM : O_B3] = gb;
 }
 
-// Sum of the block partials in block order (deterministic): out[p] for p <= NPARAM.
-__global__ void k_mlp_reduce(const float *part, int nblocks, float *out) {
-    const int p = blockIdx.x * blockDim.x + threadIdx.x;
-    if (p > NPARAM) return;
-    float s = 0.f;
-    for (int b = 0; b < nblocks; ++b) s += part[(size_t)b * (NPARAM + 1) + p];
-    out[p] = s;
-}
-
+// One Adam step: the FP32 master weights and moments, and the step's constants.
 struct Adam {
-    float lr, beta1, beta2, eps;
+    float *master, *m, *v, *loss;
+    Net *net;
+    float lr, beta1, beta2, eps, loss_scale;
+    int step; // 1-based count for the bias corrections
 };
 
-// One Adam step on the FP32 master weights; the network's working weights are their BF16
-// roundings.  step: 1-based count for the bias corrections.
-__global__ void k_adam(float *master, float *m, float *v, const float *grad, Net *net, Adam a, int step) {
-    const int p = blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= NPARAM) return;
-    const float g = grad[p];
-    const float mm = a.beta1 * m[p] + (1.f - a.beta1) * g;
-    const float vv = a.beta2 * v[p] + (1.f - a.beta2) * g * g;
-    m[p] = mm;
-    v[p] = vv;
-    const float mh = mm / (1.f - powf(a.beta1, (float)step));
-    const float vh = vv / (1.f - powf(a.beta2, (float)step));
-    const float x = master[p] - a.lr * mh / (sqrtf(vh) + a.eps);
-    master[p] = x;
-    net->w[p] = __bfloat162float(__float2bfloat16_rn(x));
-}
-
-__global__ void k_add_loss(const float *grad, float *acc, float scale) {
-    if (threadIdx.x == 0) *acc += grad[NPARAM] * scale;
+// The block partials summed in block order (deterministic) into grad[p], p <= NPARAM, 32 parameters
+// per block: all threads bring the partials in, their loads in flight together (at most kMaxRows rows
+// of 32), one warp adds them from shared memory.  Then, with A.master set, the Adam step of each parameter
+// (the network's working weights are the BF16 roundings of its masters) and the batch's error added
+// to *A.loss.  One thread per parameter loading as it added 512 partials, and two more launches for
+// the step and the loss, took 22.7 + 3.7 + 2.8 us, this 7 (a batch of 65536: 68 -> 26.6 us in all).
+__global__ void __launch_bounds__(512) k_mlp_update(const float *__restrict__ part, int nblocks, float *grad, const Adam A) {
+    extern __shared__ float rows[]; // [nblocks][32]
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, p = blockIdx.x * 32 + lane;
+    const bool step = wid == 0 && p < NPARAM && A.master;
+    const float m0 = step ? __ldcg(A.m + p) : 0.f, v0 = step ? __ldcg(A.v + p) : 0.f, x0 = step ? __ldcg(A.master + p) : 0.f;
+    const float c1 = 1.f - powf(A.beta1, (float)A.step), c2 = 1.f - powf(A.beta2, (float)A.step);
+    grid_wait();
+    if (p <= NPARAM) {
+#pragma unroll
+        for (int q = 0; q < kMaxRows / 16; ++q) {
+            const int b = wid + 16 * q;
+            if (b < nblocks) rows[32 * b + lane] = part[(size_t)b * (NPARAM + 1) + p];
+        }
+    }
+    grid_release();
+    __syncthreads();
+    float s = 0.f;
+    if (wid == 0) {
+#pragma unroll 16
+        for (int b = 0; b < nblocks; ++b) s += rows[32 * b + lane];
+    }
+    if (wid || p > NPARAM) return;
+    grad[p] = s;
+    if (!A.master) return;
+    if (p == NPARAM) {
+        *A.loss += s * A.loss_scale;
+        return;
+    }
+    const float g = s;
+    const float mm = A.beta1 * m0 + (1.f - A.beta1) * g;
+    const float vv = A.beta2 * v0 + (1.f - A.beta2) * g * g;
+    A.m[p] = mm;
+    A.v[p] = vv;
+    const float mh = mm / c1;
+    const float vh = vv / c2;
+    const float x = x0 - A.lr * mh / (sqrtf(vh) + A.eps);
+    A.master[p] = x;
+    A.net->w[p] = __bfloat162float(__float2bfloat16_rn(x));
 }
 
 __global__ void k_set_working(const float *master, Net *net) {
@@ -1015,7 +1103,8 @@ struct ark_mlp {
     int device = 0;
     cudaStream_t st = nullptr;
     cl::Net *net = nullptr; // device: working weights and normalisation
-    float *master = nullptr, *m = nullptr, *v = nullptr, *grad = nullptr, *part = nullptr;
+    // masters and Adam moments; the gradient and squared error, the block partials, an epoch's error
+    float *master = nullptr, *m = nullptr, *v = nullptr, *grad = nullptr, *part = nullptr, *loss = nullptr;
     int nblocks = 0;
     int step = 0;
 };
@@ -1192,13 +1281,14 @@ ark_mlp *ark_mlp_create(unsigned long long seed, int device, int *status) {
     }
     ark_mlp *M = new ark_mlp();
     M->device = device;
-    M->nblocks = 152 * 4;
+    M->nblocks = cl::kMaxRows;
     bool ok = cudaStreamCreateWithFlags(&M->st, cudaStreamNonBlocking) == cudaSuccess &&
               cudaMalloc(&M->net, sizeof(cl::Net)) == cudaSuccess &&
               cudaMalloc(&M->master, sizeof(float) * cl::NPARAM) == cudaSuccess &&
               cudaMalloc(&M->m, sizeof(float) * cl::NPARAM) == cudaSuccess &&
               cudaMalloc(&M->v, sizeof(float) * cl::NPARAM) == cudaSuccess &&
               cudaMalloc(&M->grad, sizeof(float) * (cl::NPARAM + 1)) == cudaSuccess &&
+              cudaMalloc(&M->loss, sizeof(float)) == cudaSuccess &&
               cudaMalloc(&M->part, sizeof(float) * (cl::NPARAM + 1) * M->nblocks) == cudaSuccess;
     if (!ok) {
         *status = cfail(ARK_ERR_NOMEM, "network allocation failed");
@@ -1238,6 +1328,7 @@ int ark_mlp_destroy(ark_mlp *M) {
     cudaFree(M->v);
     cudaFree(M->grad);
     cudaFree(M->part);
+    cudaFree(M->loss);
     if (M->st) cudaStreamDestroy(M->st);
     delete M;
     return ARK_OK;
@@ -1315,26 +1406,36 @@ int ark_mlp_fit_normalization(ark_mlp *M, ark_closure_data *d) {
 
 namespace {
 
-size_t grad_smem() {
-    return sizeof(float) * (2 * cl::NPARAM + 1 + cl::TS * cl::LDX + 4 * cl::TS * cl::LDH + 2 * cl::TS);
-}
-
 // gradient (and summed squared error) of samples (first + q) * stride + offset, q < count,
-// with scale 2 / count, into M->grad on M->st
+// with scale 2 / count, into M->grad on M->st; with A.master set, then one Adam step
 void launch_grad(ark_mlp *M, const ark_closure_data *d, long long first, long long count, long long stride,
-                 long long offset) {
-    const long long tiles = (count + cl::TS - 1) / cl::TS;
-    const int nb = (int)std::min<long long>(tiles, M->nblocks);
-    cl::k_mlp_grad<<<nb, cl::TS, grad_smem(), M->st>>>(d->feat, d->targ, first, count, stride, offset, M->net,
-                                                       (float)(2.0 / (double)count), M->part);
-    cl::k_mlp_reduce<<<(cl::NPARAM + 1 + 255) / 256, 256, 0, M->st>>>(M->part, nb, M->grad);
+                 long long offset, const cl::Adam &A) {
+    const int nb = (int)std::min<long long>(M->nblocks, (count + cl::TS - 1) / cl::TS);
+    cudaLaunchAttribute early;
+    early.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    early.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t c = {};
+    c.stream = M->st;
+    c.attrs = &early;
+    c.numAttrs = 1;
+    c.gridDim = dim3(nb);
+    c.blockDim = dim3(32 * cl::GW);
+    c.dynamicSmemBytes = sizeof(cl::GradSmem);
+    cudaLaunchKernelEx(&c, cl::k_mlp_grad, (const float *)d->feat, (const float *)d->targ, first, count, stride, offset,
+                       (const cl::Net *)M->net, (float)(2.0 / (double)count), M->part);
+    c.gridDim = dim3((cl::NPARAM + 1 + 31) / 32);
+    c.blockDim = dim3(512);
+    c.dynamicSmemBytes = sizeof(float) * 32 * nb;
+    cudaLaunchKernelEx(&c, cl::k_mlp_update, (const float *)M->part, nb, M->grad, A);
 }
 
 int prepare_grad() {
     static std::once_flag once;
     static cudaError_t err = cudaSuccess;
     std::call_once(once, [] {
-        err = cudaFuncSetAttribute(cl::k_mlp_grad, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)grad_smem());
+        err = cudaFuncSetAttribute(cl::k_mlp_grad, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(cl::GradSmem));
+        if (err == cudaSuccess)
+            err = cudaFuncSetAttribute(cl::k_mlp_update, cudaFuncAttributeMaxDynamicSharedMemorySize, 4 * 32 * cl::kMaxRows);
     });
     return err == cudaSuccess ? ARK_OK : cfail(ARK_ERR_CUDA, "k_mlp_grad shared memory attribute");
 }
@@ -1347,7 +1448,7 @@ int ark_mlp_gradient(ark_mlp *M, ark_closure_data *d, long long first, long long
     if (!M || !d || first < 0 || count < 1 || first + count > d->n) return cfail(ARK_ERR_PARAM, "bad range");
     if (int rc = prepare_grad()) return rc;
     CL_CUDA(cudaStreamSynchronize(d->st));
-    launch_grad(M, d, first, count, 1, 0);
+    launch_grad(M, d, first, count, 1, 0, cl::Adam{});
     CL_CUDA(cudaGetLastError());
     std::vector<float> h(cl::NPARAM + 1);
     CL_CUDA(cudaStreamSynchronize(M->st));
@@ -1367,17 +1468,15 @@ int ark_mlp_train(ark_mlp *M, ark_closure_data *d, int epochs, long long batch, 
     if (nb < 1) return cfail(ARK_ERR_PARAM, "fewer samples than one batch");
     if (int rc = prepare_grad()) return rc;
     CL_CUDA(cudaStreamSynchronize(d->st));
-    float *lossacc = nullptr;
-    CL_CUDA(cudaMalloc(&lossacc, sizeof(float)));
-    const cl::Adam a = {(float)lr, 0.9f, 0.999f, 1e-8f};
+    cl::Adam a = {M->master, M->m, M->v, M->loss, M->net, (float)lr, 0.9f, 0.999f, 1e-8f,
+                  (float)(1.0 / ((double)batch * (double)nb)), 0};
     int rc = ARK_OK;
     for (int ep = 0; ep < epochs && rc == ARK_OK; ++ep) {
-        cudaMemsetAsync(lossacc, 0, sizeof(float), M->st);
+        cudaMemsetAsync(M->loss, 0, sizeof(float), M->st);
         for (long long b = 0; b < nb; ++b) {
-            launch_grad(M, d, 0, batch, nb, b);
             M->step += 1;
-            cl::k_adam<<<(cl::NPARAM + 255) / 256, 256, 0, M->st>>>(M->master, M->m, M->v, M->grad, M->net, a, M->step);
-            cl::k_add_loss<<<1, 32, 0, M->st>>>(M->grad, lossacc, (float)(1.0 / ((double)batch * (double)nb)));
+            a.step = M->step;
+            launch_grad(M, d, 0, batch, nb, b, a);
             if (cudaGetLastError() != cudaSuccess) {
                 rc = cfail(ARK_ERR_CUDA, "training launch failed");
                 break;
@@ -1387,10 +1486,9 @@ int ark_mlp_train(ark_mlp *M, ark_closure_data *d, int epochs, long long batch, 
     float h = 0.f;
     if (rc == ARK_OK) {
         cudaError_t e = cudaStreamSynchronize(M->st);
-        if (e == cudaSuccess) e = cudaMemcpy(&h, lossacc, sizeof(float), cudaMemcpyDeviceToHost);
+        if (e == cudaSuccess) e = cudaMemcpy(&h, M->loss, sizeof(float), cudaMemcpyDeviceToHost);
         if (e != cudaSuccess) rc = cfail(ARK_ERR_CUDA, std::string("training: ") + cudaGetErrorString(e));
     }
-    cudaFree(lossacc);
     if (rc) return rc;
     if (loss) *loss = epochs > 0 ? (double)h : 0.0;
     return ARK_OK;
