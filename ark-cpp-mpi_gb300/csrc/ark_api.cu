@@ -483,7 +483,8 @@ template <class T> struct EngineT : Engine {
             // captured, the seam faces of the folded sweeps go with the x2 sweep in one launch
             const bool merged = xs && !ev;
             if (merged) Launch<T>::sweep_y_seams(S, y, fcur, seams, zs, st, ctx->seg_target);
-            for (int ax = 0; ax < 3; ++ax) {
+            const bool all = !fold && !ev && ctx->x1_lines <= 0 && Launch<T>::sweeps(S, y, fcur, st, ctx->seg_target);
+            for (int ax = 0; ax < 3 && !all; ++ax) {
                 if (ax == 0 && xs) {
                     if (!merged) Launch<T>::sweep_x_seams(S, y, fcur, seams, st);
                 } else if (ax == 2 && zs) {

@@ -20,6 +20,7 @@
 //   k_sweep_x, k_sweep_col<AX>       Phase2 sweeps (main.cpp:1726-2011, 2023-2255, 2261-2494)
 //   k_boundary_fill                  BoundaryConditions (source/BoundaryConditions.cpp:22-83)
 #pragma once
+#include <algorithm>
 #include <cstdint>
 #include <cstring>
 #include <cuda.h> // CUtensorMap and its enums (types only: the encoder comes through the runtime)
@@ -2058,6 +2059,29 @@ __global__ void __launch_bounds__(128, 9) k_sweep_y_seams(const __grid_constant_
     }
 }
 
+// The three sweeps in one launch of independent blocks: x1 (n1 blocks), x2 (n2, c2 to a segment), x3 (c3 to
+// a segment).  One after the other, each ends in a wave that leaves most SMs idle: FP64 64x32x32 96 -> 90
+// us per step, 200x60x1 56 -> 47, 128x96x96 1082 -> 1021, 256x128x128 3383 -> 3358; FP32 with the closure
+// 64x48x48 43 -> 40.  The registers are the x1 sweep's for all (FP64 three blocks per SM, where the
+// column sweeps alone have four; FP32 six instead of nine, so only for grids of a few waves).
+template <class T>
+__global__ void __launch_bounds__(128, sizeof(T) == 4 ? 6 : 3) k_sweeps(const __grid_constant__ DevState<T> S, int con, int fcur, int gl,
+                                                                       int nch, int n1, int seg2, int n2, int c2, int seg3, int c3) {
+    BIx bx = {(int)blockIdx.x, 0, 0, 0, 0};
+    if (bx.x < n1) {
+        sweep_x_body<T>(S, con, fcur, gl, bx, nch);
+    } else if ((bx.x -= n1) < n2) {
+        bx.z = bx.x / c2;
+        bx.x -= bx.z * c2;
+        sweep_col_body<T, 1>(S, con, fcur, seg2, bx);
+    } else {
+        bx.x -= n2;
+        bx.z = bx.x / c3;
+        bx.x -= bx.z * c3;
+        sweep_col_body<T, 2>(S, con, fcur, seg3, bx);
+    }
+}
+
 // ---------------------------------------------------------------------------------------
 // Phase2 with the three sweeps fused.  The sweeps are independent (each reads its own face
 // set and the two cell levels, and writes its own new face generation), so one kernel can do
@@ -2329,6 +2353,45 @@ inline int sweep_segment(int nd, int target, int blocks, bool fp64, int *nseg) {
     return seg;
 }
 
+// How the three sweeps in one launch are cut: chunks (nch) or lines (gl) of x1, segments of x2 and x3, and
+// their blocks.
+struct SweepCut {
+    int gl, nch, seg2, seg3, n1, n2, n3, c2, c3;
+};
+inline SweepCut sweep_cut(const Geom &g, int target, bool fp64) {
+    SweepCut c;
+    const int lines = g.C2 * g.C3, nd2 = g.C2 + 1, nd3 = g.C3 + 1;
+    c.gl = x_lines_per_warp(g, fp64);
+    c.nch = x_chunks_per_warp(g, c.gl, fp64);
+    c.n1 = c.nch ? x_chunk_blocks(g, c.nch) : (lines + 4 * c.gl - 1) / (4 * c.gl);
+    c.c2 = col_sweep_blocks(g, 1);
+    c.c3 = col_sweep_blocks(g, 2);
+    int m2, m3;
+    c.seg2 = sweep_segment(nd2, target, c.c2, fp64, &m2);
+    c.seg3 = sweep_segment(nd3, target, c.c3, fp64, &m3);
+    c.n2 = c.c2 * m2;
+    c.n3 = c.c3 * m3;
+    if (!fp64 || c.n1 + c.n2 + c.n3 > 4 * 3 * 152) return c;
+    // FP64 grids of a few waves: segments of the x2 and x3 sweeps that fill whole waves of three blocks
+    // per SM (96x64x64: 384 blocks of 18 cells 403 us per step, 576 of 12 cells 430; 128x64x64: 896 of 11
+    // cells 469, 512 of 18 cells 499, 1408 of 7 cells 489)
+    int least = 1 << 30;
+    for (int most = 1; most <= target; ++most) {
+        const int k2 = (nd2 + most - 1) / most, k3 = (nd3 + most - 1) / most;
+        const int s2 = (nd2 + k2 - 1) / k2, s3 = (nd3 + k3 - 1) / k3;
+        const int n2 = c.c2 * ((nd2 + s2 - 1) / s2), n3 = c.c3 * ((nd3 + s3 - 1) / s3);
+        const int cost = (n2 + n3 + 3 * 152 - 1) / (3 * 152) * (std::max(s2, s3) + 1);
+        if (cost <= least) {
+            least = cost;
+            c.seg2 = s2;
+            c.seg3 = s3;
+            c.n2 = n2;
+            c.n3 = n3;
+        }
+    }
+    return c;
+}
+
 inline int grid_for(int64_t n, int block, int cap) {
     int64_t b = (n + block - 1) / block;
     if (b > cap) b = cap;
@@ -2577,6 +2640,14 @@ template <class T> void Launch<T>::sweep_z_seams(const DevState<T> &S, int con, 
     k_sweep_z_seams<T><<<dim3(col_sweep_blocks(S.g, 2), 1, nch + 1), 128, 0, st>>>(S, con, fcur, kch);
 }
 
+
+template <class T> bool Launch<T>::sweeps(const DevState<T> &S, int con, int fcur, cudaStream_t st, int target) {
+    constexpr bool fp64 = sizeof(T) == 8;
+    const SweepCut c = sweep_cut(S.g, target, fp64);
+    if (!fp64 && c.n1 + c.n2 + c.n3 > 3 * 6 * 152) return false;
+    k_sweeps<T><<<c.n1 + c.n2 + c.n3, 128, 0, st>>>(S, con, fcur, c.gl, c.nch, c.n1, c.seg2, c.n2, c.c2, c.seg3, c.c3);
+    return true;
+}
 
 template <class T>
 void Launch<T>::sweep_y_seams(const DevState<T> &S, int con, int fcur, const XSeams &X, bool z, cudaStream_t st, int target) {

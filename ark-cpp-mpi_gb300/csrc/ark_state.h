@@ -354,6 +354,8 @@ template <class T> struct Launch {
     // x2/x3 sweeps: lines cut into balanced segments of at most `target` faces
     // x1 sweep: xlines lines per warp (0: x_lines_per_warp's choice)
     static void sweep(const DevState<T> &S, int con, int fcur, int axis, cudaStream_t st, int target = 32, int xlines = 0);
+    // the three sweeps' blocks in one launch, where the grid is small enough for it (else false)
+    static bool sweeps(const DevState<T> &S, int con, int fcur, cudaStream_t st, int target);
     // the three sweeps in one kernel (same results)
     static void phase2_fused(const DevState<T> &S, int con, int fcur, cudaStream_t st);
     // FP32: the three sweeps and the second Phase1 (UseForces, bulk-flow partials) in one kernel,
