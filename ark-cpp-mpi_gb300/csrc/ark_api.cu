@@ -416,7 +416,8 @@ template <class T> struct EngineT : Engine {
     // One full step of main.cpp:82-91 with "Con" = level x at entry and exit, reading the
     // dt / bulk-flow partials of the current state and leaving those of the next one.  With
     // ev given, an event is recorded after each of the step_launches() launches.
-    void step(int x, int fcur, cudaEvent_t *ev) override {
+    bool rotates() override { return use_step2(); }
+    void step(int x, int fcur, cudaEvent_t *ev, bool chained) override {
         const int y = x ^ 1;
         cudaStream_t st = ctx->st;
         int nmark = 0;
@@ -442,7 +443,7 @@ template <class T> struct EngineT : Engine {
         const bool nofill = skip_phase2_fill();
         if (!ev) {
             // captured: dt and the ghost fill of the "Con" level in one launch
-            Launch<T>::step_begin(S, y, xg ? 2 : nofill ? 0 : 1, st);
+            Launch<T>::step_begin(S, y, xg ? 2 : nofill ? 0 : 1, st, chained);
         } else { // timed one launch after the other
             Launch<T>::finalize_dt(S, 1, st);
             mark();
@@ -480,20 +481,29 @@ template <class T> struct EngineT : Engine {
             Launch<T>::phase2_fused(S, y, fcur, st);
             for (int ax = 0; ax < 3; ++ax) mark();
         } else {
-            // captured, the seam faces of the folded sweeps go with the x2 sweep in one launch
-            const bool merged = xs && !ev;
-            if (merged) Launch<T>::sweep_y_seams(S, y, fcur, seams, zs, st, ctx->seg_target);
+            // captured, the seam faces of the folded sweeps (only the second Phase1 reads the x and z
+            // faces) are written in one launch with the x2 sweep, or beside it on the second stream
+            const bool merged = xs && !ev && Launch<T>::sweep_y_seams(S, y, fcur, seams, zs, st, ctx->seg_target);
+            const bool beside = xs && !ev && !merged;
+            if (beside) {
+                cudaEventRecord(ctx->seam_fork, st);
+                cudaStreamWaitEvent(ctx->fill, ctx->seam_fork, 0);
+                Launch<T>::sweep_x_seams(S, y, fcur, seams, ctx->fill);
+                if (zs) Launch<T>::sweep_z_seams(S, y, fcur, seams.kch, ctx->fill);
+                cudaEventRecord(ctx->seam_join, ctx->fill);
+            }
             const bool all = !fold && !ev && ctx->x1_lines <= 0 && Launch<T>::sweeps(S, y, fcur, st, ctx->seg_target);
             for (int ax = 0; ax < 3 && !all; ++ax) {
                 if (ax == 0 && xs) {
-                    if (!merged) Launch<T>::sweep_x_seams(S, y, fcur, seams, st);
+                    if (!merged && !beside) Launch<T>::sweep_x_seams(S, y, fcur, seams, st);
                 } else if (ax == 2 && zs) {
-                    if (!merged) Launch<T>::sweep_z_seams(S, y, fcur, seams.kch, st);
+                    if (!merged && !beside) Launch<T>::sweep_z_seams(S, y, fcur, seams.kch, st);
                 } else if (ax == 1 ? !merged : ax > 0 || !fold) {
                     Launch<T>::sweep(S, y, fcur, ax, st, ctx->seg_target, ctx->x1_lines);
                 }
                 mark();
             }
+            if (beside) cudaStreamWaitEvent(st, ctx->seam_join, 0);
         }
         Launch<T>::phase1(S, x, y, fcur ^ 1, P1_FORCES | P1_RSUM, ctx->march[1], st, ctx->p1_chunk);
         mark();
@@ -697,7 +707,10 @@ ark_ctx *ark_create(const ark_params *params, int *status) {
     // learned closure's inference) only takes SMs the step's kernels leave idle
     int prio_low = 0, prio_high = 0;
     cudaDeviceGetStreamPriorityRange(&prio_low, &prio_high);
-    if (cudaStreamCreateWithPriority(&ctx->st, cudaStreamNonBlocking, prio_high) != cudaSuccess) {
+    if (cudaStreamCreateWithPriority(&ctx->st, cudaStreamNonBlocking, prio_high) != cudaSuccess ||
+        cudaStreamCreateWithPriority(&ctx->fill, cudaStreamNonBlocking, prio_high) != cudaSuccess ||
+        cudaEventCreateWithFlags(&ctx->seam_fork, cudaEventDisableTiming) != cudaSuccess ||
+        cudaEventCreateWithFlags(&ctx->seam_join, cudaEventDisableTiming) != cudaSuccess) {
         *status = fail(ARK_ERR_CUDA, "cudaStreamCreate failed");
         return nullptr;
     }
@@ -758,7 +771,8 @@ int ark_destroy(ark_ctx *ctx) {
     cudaStreamSynchronize(ctx->st);
     for (int a = 0; a < 2; ++a)
         for (int b = 0; b < 2; ++b)
-            if (ctx->graph[a][b]) cudaGraphExecDestroy(ctx->graph[a][b]);
+            for (cudaGraphExec_t g : {ctx->graph[a][b], ctx->chain[a][b]})
+                if (g) cudaGraphExecDestroy(g);
     ctx->eng.reset();
     if (ctx->stage) cudaFree(ctx->stage);
     if (ctx->cond_dev) cudaFree(ctx->cond_dev);
@@ -771,6 +785,12 @@ int ark_destroy(ark_ctx *ctx) {
     }
     if (ctx->fork) cudaEventDestroy(ctx->fork);
     if (ctx->join) cudaEventDestroy(ctx->join);
+    if (ctx->fill) {
+        cudaStreamSynchronize(ctx->fill);
+        cudaStreamDestroy(ctx->fill);
+    }
+    if (ctx->seam_fork) cudaEventDestroy(ctx->seam_fork);
+    if (ctx->seam_join) cudaEventDestroy(ctx->seam_join);
     for (int b = 0; b < 2; ++b) {
         if (ctx->io_dev[b]) cudaFree(ctx->io_dev[b]);
         if (ctx->io_host[b]) cudaFreeHost(ctx->io_host[b]);
@@ -970,6 +990,26 @@ int ark_set_dt(ark_ctx *ctx, double dt) {
     return ARK_OK;
 }
 
+// `n` fused steps captured from the current roles of the cell levels and face generations.
+static int capture_steps(ark_ctx *ctx, int n, cudaGraphExec_t *exec) {
+    cudaGraph_t graph = nullptr;
+    ARK_CUDA(cudaStreamBeginCapture(ctx->st, cudaStreamCaptureModeThreadLocal));
+    for (int s = 0; s < n; ++s) ctx->eng->step(ctx->con, ctx->fcur ^ (s & 1), nullptr, s > 0);
+    cudaError_t le = cudaGetLastError();
+    cudaError_t ce = cudaStreamEndCapture(ctx->st, &graph);
+    if (le != cudaSuccess || ce != cudaSuccess) {
+        if (graph) cudaGraphDestroy(graph);
+        return fail(ARK_ERR_CUDA, std::string("step capture: ") + cudaGetErrorString(le != cudaSuccess ? le : ce));
+    }
+    cudaError_t ie = cudaGraphInstantiate(exec, graph, 0);
+    cudaGraphDestroy(graph);
+    if (ie != cudaSuccess) {
+        *exec = nullptr;
+        return fail(ARK_ERR_CUDA, std::string("graph instantiate: ") + cudaGetErrorString(ie));
+    }
+    return ARK_OK;
+}
+
 // Captures the fused step for the current role of the two cell levels (once per role).  A graph
 // holds the level buffers it was captured with; when the one-kernel Phase2 + second Phase1
 // rotates them through the spare, each face generation meets its own buffers again every
@@ -981,26 +1021,25 @@ static int ensure_graph(ark_ctx *ctx) {
         cudaGraphExecDestroy(ctx->graph[x][fc]);
         ctx->graph[x][fc] = nullptr;
     }
-    if (!ctx->graph[x][fc]) {
-        std::memcpy(ctx->graph_levels[x][fc], lv, sizeof lv);
-        cudaGraph_t graph = nullptr;
-        ARK_CUDA(cudaStreamBeginCapture(ctx->st, cudaStreamCaptureModeThreadLocal));
-        ctx->eng->step(x, fc, nullptr);
-        cudaError_t le = cudaGetLastError();
-        cudaError_t ce = cudaStreamEndCapture(ctx->st, &graph);
-        if (le != cudaSuccess || ce != cudaSuccess) {
-            if (graph) cudaGraphDestroy(graph);
-            return fail(ARK_ERR_CUDA, std::string("step capture: ") +
-                                          cudaGetErrorString(le != cudaSuccess ? le : ce));
-        }
-        cudaError_t ie = cudaGraphInstantiate(&ctx->graph[x][fc], graph, 0);
-        cudaGraphDestroy(graph);
-        if (ie != cudaSuccess) {
-            ctx->graph[x][fc] = nullptr;
-            return fail(ARK_ERR_CUDA, std::string("graph instantiate: ") + cudaGetErrorString(ie));
-        }
-    }
-    return ARK_OK;
+    if (ctx->graph[x][fc]) return ARK_OK;
+    std::memcpy(ctx->graph_levels[x][fc], lv, sizeof lv);
+    return capture_steps(ctx, 1, &ctx->graph[x][fc]);
+}
+
+// A run of many steps launches graphs of kChain steps: a graph's end and the next one's start cost
+// about 3 us, which a step of a small grid is not much longer than (us per step, one step to a graph and
+// eight: FP32 32x32x32 20.5 -> 17.3, 64x48x48 27.3 -> 24.2, with the closure 39.2 -> 34.4, 128x64x64 53.1 ->
+// 49.5; FP64 64x32x32 91.3 -> 88.6, 200x60x1 47.2 -> 44.2).  An even count, so that a graph begins and
+// ends with the same face generation; long runs only (the capture takes as long as the gaps of about a
+// hundred steps), on grids whose step takes up to about a hundred of those gaps.
+constexpr int kChain = 8, kChainFrom = 64;
+static bool chains(ark_ctx *ctx, int nsteps) {
+    return (nsteps >= kChainFrom || (nsteps >= kChain && ctx->chain[ctx->con][ctx->fcur])) && !ctx->eng->rotates() &&
+           (int64_t)ctx->g.C1 * ctx->g.C2 * ctx->g.C3 <= (1 << 23);
+}
+static int ensure_chain(ark_ctx *ctx) {
+    cudaGraphExec_t *exec = &ctx->chain[ctx->con][ctx->fcur];
+    return *exec ? ARK_OK : capture_steps(ctx, kChain, exec);
 }
 
 int ark_step(ark_ctx *ctx, int nsteps) {
@@ -1011,8 +1050,13 @@ int ark_step(ark_ctx *ctx, int nsteps) {
         ctx->eng->reduce(ctx->con);
         ctx->parts_valid = true;
     }
+    int s = 0;
+    if (chains(ctx, nsteps)) {
+        if (int rc = ensure_chain(ctx)) return rc;
+        for (; nsteps - s >= kChain; s += kChain) ARK_CUDA(cudaGraphLaunch(ctx->chain[ctx->con][ctx->fcur], ctx->st));
+    }
     // each step flips the face generation; the graph of each parity is captured once
-    for (int s = 0; s < nsteps; ++s) {
+    for (; s < nsteps; ++s) {
         if (int rc = ensure_graph(ctx)) return rc;
         ARK_CUDA(cudaGraphLaunch(ctx->graph[ctx->con][ctx->fcur], ctx->st));
         ctx->fcur ^= 1;
@@ -1043,6 +1087,8 @@ int ark_time_steps(ark_ctx *ctx, int nsteps, double *ms) {
     ctx->fcur ^= 1;
     ctx->eng->after_step(ctx->con);
     if (rc2) return rc2;
+    if (chains(ctx, nsteps))
+        if (int rc = ensure_chain(ctx)) return rc;
     ARK_CUDA(cudaStreamSynchronize(ctx->st));
     ARK_CUDA(cudaEventRecord(ctx->ev0, ctx->st));
     if (int rc = ark_step(ctx, nsteps)) return rc;
@@ -1250,10 +1296,11 @@ namespace {
 void drop_graphs(ark_ctx *ctx) {
     for (int a = 0; a < 2; ++a)
         for (int b = 0; b < 2; ++b)
-            if (ctx->graph[a][b]) {
-                cudaGraphExecDestroy(ctx->graph[a][b]);
-                ctx->graph[a][b] = nullptr;
-            }
+            for (cudaGraphExec_t *g : {&ctx->graph[a][b], &ctx->chain[a][b]})
+                if (*g) {
+                    cudaGraphExecDestroy(*g);
+                    *g = nullptr;
+                }
 }
 
 // The two slab buffers (device and pinned host) of at least n doubles each.

@@ -590,12 +590,9 @@ __device__ __forceinline__ void gelu_both(float z, float &h, float &d) {
     d = 0.5f * (1.0f + th) + 0.5f * z * (1.0f - th * th) * GK0 * (1.0f + 3.0f * GK1 * z * z);
 }
 
-// Training alternates two short kernels, each launched while the one before still runs (programmatic
-// stream serialization): grid_release lets the next grid start, grid_wait waits for the one before to
-// have ended with its writes visible.  Before grid_wait a kernel reads only what the other does not
-// write (the samples; the moments and masters, which k_mlp_update alone writes).
-__device__ __forceinline__ void grid_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-__device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// Training alternates two short kernels, each launched while the one before still runs (launch_early).
+// Before grid_wait a kernel reads only what the other does not write (the samples; the moments and
+// masters, which k_mlp_update alone writes).
 constexpr int kMaxRows = 608; // rows of block partials: at most four blocks per SM
 
 struct GradSmem {
@@ -1411,22 +1408,9 @@ namespace {
 void launch_grad(ark_mlp *M, const ark_closure_data *d, long long first, long long count, long long stride,
                  long long offset, const cl::Adam &A) {
     const int nb = (int)std::min<long long>(M->nblocks, (count + cl::TS - 1) / cl::TS);
-    cudaLaunchAttribute early;
-    early.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    early.val.programmaticStreamSerializationAllowed = 1;
-    cudaLaunchConfig_t c = {};
-    c.stream = M->st;
-    c.attrs = &early;
-    c.numAttrs = 1;
-    c.gridDim = dim3(nb);
-    c.blockDim = dim3(32 * cl::GW);
-    c.dynamicSmemBytes = sizeof(cl::GradSmem);
-    cudaLaunchKernelEx(&c, cl::k_mlp_grad, (const float *)d->feat, (const float *)d->targ, first, count, stride, offset,
-                       (const cl::Net *)M->net, (float)(2.0 / (double)count), M->part);
-    c.gridDim = dim3((cl::NPARAM + 1 + 31) / 32);
-    c.blockDim = dim3(512);
-    c.dynamicSmemBytes = sizeof(float) * 32 * nb;
-    cudaLaunchKernelEx(&c, cl::k_mlp_update, (const float *)M->part, nb, M->grad, A);
+    launch_early(true, cl::k_mlp_grad, dim3(nb), dim3(32 * cl::GW), sizeof(cl::GradSmem), M->st, d->feat, d->targ, first, count, stride,
+                 offset, M->net, (float)(2.0 / (double)count), M->part);
+    launch_early(true, cl::k_mlp_update, dim3((cl::NPARAM + 1 + 31) / 32), dim3(512), sizeof(float) * 32 * nb, M->st, M->part, nb, M->grad, A);
 }
 
 int prepare_grad() {

@@ -24,7 +24,10 @@ struct Engine {
     virtual void stress(int con, int bulk) = 0;
     virtual void use_forces(int ncon) = 0;
     virtual void phase2(int con, int fcur) = 0;
-    virtual void step(int con, int fcur, cudaEvent_t *ev) = 0;
+    // chained: captured behind another step
+    virtual void step(int con, int fcur, cudaEvent_t *ev, bool chained = false) = 0;
+    // whether steps pass their levels on through the spare (the graph of a step then holds others each time)
+    virtual bool rotates() = 0;
     virtual void boundary_fill(int ncon, int axis, int periodic) = 0;
     virtual void sums(int ncon) = 0;
     virtual void mean_profile(int ncon, long long *acc) = 0;
@@ -81,6 +84,7 @@ struct ark_ctx {
     bool parts_valid = false; // the dt / bulk-flow partials describe the current state
     int march[2] = {1, 0};    // Phase1 kernel shape of the two Phase1 launches of a step
     cudaGraphExec_t graph[2][2] = {{nullptr, nullptr}, {nullptr, nullptr}}; // [con][fcur]
+    cudaGraphExec_t chain[2][2] = {{nullptr, nullptr}, {nullptr, nullptr}}; // the same of kChain steps
     const void *graph_levels[2][2][3] = {};  // the level buffers each graph was captured with
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     double *stage = nullptr; // contiguous double staging for host transfers
@@ -89,6 +93,8 @@ struct ark_ctx {
     void *closure_net = nullptr;          // learned closure: the network's constants (device copy)
     cudaStream_t side = nullptr;          // the closure's branch of the step
     cudaEvent_t fork = nullptr, join = nullptr;
+    cudaStream_t fill = nullptr;          // the captured step's second stream
+    cudaEvent_t seam_fork = nullptr, seam_join = nullptr; // the seam kernels on `fill`, beside the x2 sweep
     float closure_scale = 0.f;            // u_tau / vis for the y+ feature
     int seg_target = 32;                  // x2/x3 sweep segment length (faces)
     int x1_lines = 0;                     // x1 sweep lines per warp (0: x_lines_per_warp's choice)

@@ -600,6 +600,8 @@ template <class T> __global__ void k_wrap(Geom g, const __grid_constant__ WrapJo
 template <class T>
 __global__ void __launch_bounds__(256) k_step_begin(const __grid_constant__ DevState<T> S, const __grid_constant__ WrapJob J, int nb) {
     static_assert(kBuckets == 256, "one thread per slot");
+    grid_release();
+    grid_wait();
     if (blockIdx.x == 0) {
         finalize_dt_body(S, 1);
         return;
@@ -1125,6 +1127,8 @@ __device__ __forceinline__ FaceQ<T> face_q(const FaceVal<T> &V, int d, uint8_t f
 template <class T, int MODE>
 __global__ void __launch_bounds__(SX *SY, 3) k_phase1_faces(const __grid_constant__ DevState<T> S, int src, int dst, int fcur, int kch) {
     static_assert(!Storage<T>::deviation, "face-centric Phase1: FP64 storage form");
+    grid_release();
+    grid_wait();
     constexpr bool STRESS = (MODE & P1_STRESS) != 0;
     // two generations of a plane's x and y face quantities (face_smem bytes), alternating by
     // plane: a thread may write plane k+1's while others still read plane k's, and the barrier
@@ -2029,16 +2033,20 @@ __global__ void __launch_bounds__(128) k_sweep_z_seams(const __grid_constant__ D
     sweep_col_body<T, 2>(S, con, fcur, 1, bx);
 }
 
-// What is left of Phase2 after Phase1 + stress with the x1 (and x3) sweeps folded in, in one launch of
-// independent blocks: the x2 sweep (ny blocks, yc to a segment), the z seams (nz, zc to a seam plane)
-// and the x seams (nx).  The seam faces are 2-3% of the faces, scattered and bound by latency.  As
-// two launches on a second stream they were the longer branch of a small grid's step (64x48x48: 12
-// us beside an x2 sweep of 13.6; 32.5 -> 28.7 us per step in one launch).  A grid that fits the SMs
-// at once (first = 1) has them first, beside everything; a larger one last, where they fill the x2
-// sweep's last wave (512x256x256 with them first 2.4 us slower per step than last).
+// What is left of a small grid's Phase2 after Phase1 + stress with the x1 (and x3) sweeps folded in, in one
+// launch of independent blocks: the x seams (nx blocks), the z seams (nz, zc to a seam plane) and the x2
+// sweep (yc to a segment).  As launches on two streams the seam kernels were the longer branch
+// (64x48x48: 12 us beside an x2 sweep of 13.6; 32.5 -> 28.7 us per step in one launch).  The seam faces
+// are scattered, latency-bound work: first in the grid where it fits the SMs at once (`first`), last where
+// it does not, filling the x2 sweep's last wave (150x67x93 90.4 us per step, 93.0 with them first).  From
+// two waves on they do better beside the x2 sweep on a stream of their own (256x128x128: 298.7 us in one
+// launch, 297.2 on two streams).
 template <class T>
 __global__ void __launch_bounds__(128, 9) k_sweep_y_seams(const __grid_constant__ DevState<T> S, int con, int fcur, int seg, int ny,
-                                                          int yc, const __grid_constant__ XSeams X, int nx, int nz, int zc, int first) {
+                                                          int yc, const __grid_constant__ XSeams X, int nx, int nz, int zc,
+                                                          int first) {
+    grid_release();
+    grid_wait();
     int b = (int)blockIdx.x - (first ? nx + nz : 0);
     BIx bx = {0, 0, 0, 0, 0};
     if (b >= 0 && b < ny) {
@@ -2067,6 +2075,8 @@ __global__ void __launch_bounds__(128, 9) k_sweep_y_seams(const __grid_constant_
 template <class T>
 __global__ void __launch_bounds__(128, sizeof(T) == 4 ? 6 : 3) k_sweeps(const __grid_constant__ DevState<T> S, int con, int fcur, int gl,
                                                                        int nch, int n1, int seg2, int n2, int c2, int seg3, int c3) {
+    grid_release();
+    grid_wait();
     BIx bx = {(int)blockIdx.x, 0, 0, 0, 0};
     if (bx.x < n1) {
         sweep_x_body<T>(S, con, fcur, gl, bx, nch);
@@ -2447,10 +2457,10 @@ template <class T> inline WrapJob wrap_con_job(const DevState<T> &S, int con, in
 template <class T> void Launch<T>::wrap_con(const DevState<T> &S, int con, int with_ro, cudaStream_t st) {
     wrap_launch(S, wrap_con_job(S, con, with_ro), st);
 }
-template <class T> void Launch<T>::step_begin(const DevState<T> &S, int con, int with_ro, cudaStream_t st) {
+template <class T> void Launch<T>::step_begin(const DevState<T> &S, int con, int with_ro, cudaStream_t st, bool chained) {
     const WrapJob J = wrap_con_job(S, con, with_ro);
     const int nb = (wrap_lines(S.g) + 255) / 256;
-    k_step_begin<T><<<1 + nb * J.n, 256, 0, st>>>(S, J, nb);
+    launch_early(chained && sizeof(T) == 4 && early_grid(S.g), k_step_begin<T>, dim3(1 + nb * J.n), dim3(256), 0, st, S, J, nb);
 }
 
 // The halo exchange before Phase2 (main.cpp:1049-1698): u?nCon and ronCon wrap or copy on
@@ -2558,17 +2568,12 @@ void Launch<T>::phase1(const DevState<T> &S, int src, int dst, int fcur, int mod
             const int kch = kch_in > 0 ? std::min(kch_in, S.g.C3) : kdef;
             const dim3 grid((S.g.C1 + fcs::SX - 1) / fcs::SX, (S.g.C2 + fcs::SY - 1) / fcs::SY, (S.g.C3 + kch - 1) / kch);
             const dim3 block(fcs::SX, fcs::SY);
+            constexpr int A = P1_STRESS | P1_FORCES | P1_RMAX, B = A | P1_BULK, C = P1_FORCES | P1_RSUM;
+            auto go = [&](auto kernel) { launch_early(false, kernel, grid, block, fcs::face_smem<T>(), st, S, src, dst, fcur, kch); };
             switch (mode) {
-            case P1_STRESS | P1_FORCES | P1_RMAX:
-                fcs::k_phase1_faces<T, P1_STRESS | P1_FORCES | P1_RMAX><<<grid, block, fcs::face_smem<T>(), st>>>(S, src, dst, fcur, kch);
-                return;
-            case P1_STRESS | P1_FORCES | P1_BULK | P1_RMAX:
-                fcs::k_phase1_faces<T, P1_STRESS | P1_FORCES | P1_BULK | P1_RMAX><<<grid, block, fcs::face_smem<T>(), st>>>(S, src, dst, fcur,
-                                                                                                      kch);
-                return;
-            case P1_FORCES | P1_RSUM:
-                fcs::k_phase1_faces<T, P1_FORCES | P1_RSUM><<<grid, block, fcs::face_smem<T>(), st>>>(S, src, dst, fcur, kch);
-                return;
+            case A: go(fcs::k_phase1_faces<T, A>); return;
+            case B: go(fcs::k_phase1_faces<T, B>); return;
+            case C: go(fcs::k_phase1_faces<T, C>); return;
             default: march = 0; break;
             }
         }
@@ -2645,21 +2650,25 @@ template <class T> bool Launch<T>::sweeps(const DevState<T> &S, int con, int fcu
     constexpr bool fp64 = sizeof(T) == 8;
     const SweepCut c = sweep_cut(S.g, target, fp64);
     if (!fp64 && c.n1 + c.n2 + c.n3 > 3 * 6 * 152) return false;
-    k_sweeps<T><<<c.n1 + c.n2 + c.n3, 128, 0, st>>>(S, con, fcur, c.gl, c.nch, c.n1, c.seg2, c.n2, c.c2, c.seg3, c.c3);
+    launch_early(!fp64 && early_grid(S.g), k_sweeps<T>, dim3(c.n1 + c.n2 + c.n3), dim3(128), 0, st, S, con, fcur, c.gl, c.nch, c.n1, c.seg2, c.n2, c.c2, c.seg3,
+                 c.c3);
     return true;
 }
 
 template <class T>
-void Launch<T>::sweep_y_seams(const DevState<T> &S, int con, int fcur, const XSeams &X, bool z, cudaStream_t st, int target) {
+bool Launch<T>::sweep_y_seams(const DevState<T> &S, int con, int fcur, const XSeams &X, bool z, cudaStream_t st, int target) {
     if constexpr (std::is_same<T, float>::value) {
         const int yc = col_sweep_blocks(S.g, 1), zc = col_sweep_blocks(S.g, 2);
         int nseg;
         const int seg = sweep_segment(S.g.C2 + 1, target, yc, false, &nseg);
         const int nx = (int)((seam_slots(S.g, X.tw) + 127) / 128);
-        const int nz = z ? zc * ((S.g.C3 + X.kch - 1) / X.kch + 1) : 0;
-        const int ny = yc * nseg, blocks = nx + nz + ny;
-        k_sweep_y_seams<T><<<blocks, 128, 0, st>>>(S, con, fcur, seg, ny, yc, X, nx, nz, zc, blocks <= 9 * 152);
+        const int nz = z ? zc * ((S.g.C3 + X.kch - 1) / X.kch + 1) : 0, blocks = nx + nz + yc * nseg;
+        if (blocks > 2 * 9 * 152) return false;
+        launch_early(early_grid(S.g), k_sweep_y_seams<T>, dim3(blocks), dim3(128), 0, st, S, con, fcur, seg, yc * nseg, yc, X, nx, nz, zc,
+                     (int)(blocks <= 9 * 152));
+        return true;
     }
+    return false;
 }
 
 template <class T> void Launch<T>::prepare() {

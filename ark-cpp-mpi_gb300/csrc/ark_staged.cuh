@@ -708,6 +708,7 @@ __device__ __forceinline__ void phase1_tma_body(const DevState<float> &S, const 
     auto empty_of = [&](int p) { return smem_u32(&bar[NS + (p - pfirst) % NS]); }; // empty
     auto parity_of = [&](int p) { return (unsigned)(((p - pfirst) / NS) & 1); };
     volatile unsigned long long *const abort_flag = bar + 2 * NS;
+    grid_release();
     if (t == NT) {
         if (fence_maps)
             for (int q = 0; q < A.n; ++q) fence_tensormap(map(q));
@@ -724,6 +725,7 @@ __device__ __forceinline__ void phase1_tma_body(const DevState<float> &S, const 
         fence_proxy_async();
     }
     __syncthreads();
+    grid_wait();
 
     bool failed = false;
     int issued = pfirst - 1; // the producer: the last plane issued
@@ -1016,8 +1018,8 @@ inline void launch_staged_tma(const DevState<float> &S, int src, int dst, int fc
         return;
     }
     const int kch = kch_in > 0 ? (kch_in < S.g.C3 ? kch_in : S.g.C3) : tile_chunk<TSX, TSY>(S.g, TLayout<MODE, TSX, TSY>::STRESS);
-    k_phase1_tma<MODE, TSX, TSY><<<tile_grid<TSX, TSY>(S.g, kch), dim3(TSX * TSY + 32), TLayout<MODE, TSX, TSY>::SMEM + 128, st>>>(
-        S, A, src, dst, kch, fcur, XSeams{});
+    launch_early(early_grid(S.g), k_phase1_tma<MODE, TSX, TSY>, tile_grid<TSX, TSY>(S.g, kch), dim3(TSX * TSY + 32), TLayout<MODE, TSX, TSY>::SMEM + 128,
+                 st, S, A, src, dst, kch, fcur, XSeams{});
 }
 // Phase1 + stress with the x1 sweep (XS = 1) or the x1 and x3 sweeps (XS = 3) folded in (X.tw
 // and X.kch set to the tile width and the planes per block); false, launching nothing, when the
@@ -1029,9 +1031,8 @@ inline bool launch_staged_tma_xs(const DevState<float> &S, int src, int dst, int
     const int kch = kch_in > 0 ? (kch_in < S.g.C3 ? kch_in : S.g.C3) : tile_chunk<TSX, TSY>(S.g, TLayout<MODE, TSX, TSY>::STRESS);
     X.tw = TSX;
     X.kch = kch;
-    k_phase1_tma<MODE, TSX, TSY, XS>
-        <<<tile_grid<TSX, TSY>(S.g, kch), dim3(TSX * TSY + 32), TLayout<MODE, TSX, TSY>::SMEM + 128, st>>>(S, A, src, dst, kch,
-                                                                                                      fcur, X);
+    launch_early(early_grid(S.g), k_phase1_tma<MODE, TSX, TSY, XS>, tile_grid<TSX, TSY>(S.g, kch), dim3(TSX * TSY + 32),
+                 TLayout<MODE, TSX, TSY>::SMEM + 128, st, S, A, src, dst, kch, fcur, X);
     return true;
 }
 // The bounded-wait check: the same launch with every plane expecting `extra` bytes more than its
