@@ -194,6 +194,61 @@ __device__ __forceinline__ double dhalf(double x) {
     return halve_call(x);
 }
 __device__ __forceinline__ float dhalf(float x) { return x / 2.f; }
+// RN(a * b) on the integer pipes: the 106-bit product of the significands, normalised and rounded to
+// nearest even.  Other than normal operands with a normal product take the multiply, zeros a zero.
+// GB300's FP64 pipe takes 16 cycles of an SM for a warp's instruction, about 32 instructions' worth of
+// its four schedulers, and the FP64 kernels left those three quarters idle; with part of their products
+// here the two run side by side (256x128x128: x2 sweep 498 -> 404 us, x3 494 -> 406, x1 459 -> 447, with
+// 12 of a cell's 51 FP64 instructions; Phase1 + stress 1199 -> 1035, with 21 of 132, the products with
+// face areas; second Phase1 752 -> 561, with 30 of 75; the step 3350 -> 2856.  More of them in Phase1 +
+// stress is slower again: 1047 with 7 more, 1324 with all.)
+static __device__ __noinline__ double mul_call(double a, double b) { return a * b; }
+__device__ __forceinline__ double mulq(double a, double b) {
+    const unsigned ha = (unsigned)__double2hiint(a), a0 = (unsigned)__double2loint(a);
+    const unsigned hb = (unsigned)__double2hiint(b), lb = (unsigned)__double2loint(b);
+    constexpr unsigned EXP = 0x7FF00000u, ONE = 1u << 20;
+    // a's significand (53 bits) and b's shifted to the top of 64: w3:w2 has 52 or 53 bits
+    const unsigned a1 = (ha & 0xFFFFFu) | ONE, b1 = __funnelshift_l(lb, hb, 11) | 0x80000000u, b0 = lb << 11;
+    unsigned w0, w1, w2, w3;
+    asm("mul.lo.u32 %0, %4, %6;\n\t"
+        "mul.hi.u32 %1, %4, %6;\n\t"
+        "mad.lo.cc.u32 %1, %4, %7, %1;\n\t"
+        "madc.hi.u32 %2, %4, %7, 0;\n\t"
+        "mad.lo.cc.u32 %1, %5, %6, %1;\n\t"
+        "madc.hi.cc.u32 %2, %5, %6, %2;\n\t"
+        "addc.u32 %3, 0, 0;\n\t"
+        "mad.lo.cc.u32 %2, %5, %7, %2;\n\t"
+        "madc.hi.u32 %3, %5, %7, %3;"
+        : "=&r"(w0), "=&r"(w1), "=&r"(w2), "=&r"(w3)
+        : "r"(a0), "r"(a1), "r"(b0), "r"(b1));
+    const unsigned s = 1u - (w3 >> 20); // 1: 52 bits
+    const unsigned hi = __funnelshift_l(w2, w3, s), lo = __funnelshift_l(w1, w2, s);
+    const unsigned r1 = __funnelshift_l(w0, w1, s), r0 = w0 << s; // below the last bit
+    // the product's exponent less one, in place; the hidden bit of hi adds the one
+    const unsigned e = (ha & EXP) + (hb & EXP) - 1023u * ONE - s * ONE;
+    // rounded: half a unit less one, and one more where the last bit is odd, carries into it
+    unsigned top, low;
+    asm("{\n\t.reg .u32 t;\n\t"
+        "add.cc.u32 t, %2, 0xFFFFFFFF;\n\t"
+        "addc.cc.u32 t, %3, 0xFFFFFFFF;\n\t"
+        "addc.cc.u32 t, %4, 0x7FFFFFFF;\n\t"
+        "addc.cc.u32 %0, %5, 0;\n\t"
+        "addc.u32 %1, %6, %7;\n\t}"
+        : "=&r"(low), "=&r"(top)
+        : "r"(lo & 1u), "r"(r0), "r"(r1), "r"(lo), "r"(hi), "r"(e));
+    // both exponents in 2^-511 .. 2^512 (their top bits differ), and the product's below the largest
+    if (((ha ^ (ha << 1)) & (hb ^ (hb << 1)) & 0x40000000u) && e < 2044u * ONE)
+        return __hiloint2double((int)(top | ((ha ^ hb) & 0x80000000u)), (int)low);
+    const bool za = ((ha << 1) | a0) == 0u, zb = ((hb << 1) | lb) == 0u;
+    if ((za || zb) && (ha & EXP) != EXP && (hb & EXP) != EXP) return __hiloint2double((int)((ha ^ hb) & 0x80000000u), 0);
+    return mul_call(a, b);
+}
+__device__ __forceinline__ float mulq(float a, float b) { return a * b; }
+// INT: mulq, else the multiply
+template <bool INT, class T> __device__ __forceinline__ T product(T a, T b) {
+    if constexpr (INT) return mulq(a, b);
+    else return a * b;
+}
 // b that changes from cell to cell (Q from qrecip_var): the other path is the IEEE division
 __device__ __forceinline__ double qdiv_v(double a, double b, const QRecip &Q) {
     bool ok;
@@ -1134,20 +1189,25 @@ template <class T> constexpr int face_smem() { return 2 * (SY * (SX + 1) + (SY +
 // The quantities of the face normal to d with values V: the mass flux ro u_d, the momentum
 // fluxes (ro u_m) u_d (+ p when m == d) of half_step, and StressTensor's sigma_md between the
 // cell below (flags flo, velocity ulo) and the cell above (fhi, uhi).
-template <class T, bool STRESS>
+template <class T, bool STRESS, bool INT>
 __device__ __forceinline__ FaceQ<T> face_q(const FaceVal<T> &V, int d, uint8_t flo, uint8_t fhi, const T ulo[3],
                                            const T uhi[3], const K<T> &kk) {
+    constexpr bool I = INT && !STRESS;
     FaceQ<T> q;
-    q.mf = V.ro * V.u[d];
+    T ru[3];
+#pragma unroll
+    for (int m = 0; m < 3; ++m) ru[m] = product<I>(V.ro, V.u[m]);
+    q.mf = ru[d];
 #pragma unroll
     for (int m = 0; m < 3; ++m) {
-        q.mom[m] = (m == d) ? V.ro * V.u[m] * V.u[d] + V.p : V.ro * V.u[m] * V.u[d];
+        const T f = product<I>(ru[m], V.u[d]);
+        q.mom[m] = (m == d) ? f + V.p : f;
         q.sig[m] = STRESS ? sigma(flo, fhi, ulo[m], uhi[m], kk, d) : (T)0;
     }
     return q;
 }
 
-template <class T, int MODE>
+template <class T, int MODE, bool INT>
 __global__ void __launch_bounds__(SX *SY, 3) k_phase1_faces(const __grid_constant__ DevState<T> S, int src, int dst, int fcur, int kch) {
     static_assert(!Storage<T>::deviation, "face-centric Phase1: FP64 storage form");
     grid_release();
@@ -1193,7 +1253,7 @@ __global__ void __launch_bounds__(SX *SY, 3) k_phase1_faces(const __grid_constan
         cellu(c, uc);
         T ud[3];
         if (STRESS) cellu(c - cs2, ud);
-        zlo = face_q<T, STRESS>(load_face(S.fc[fcur][2], f, kk), 2, STRESS ? flags[c - cs2] : 0, fl, STRESS ? ud : zero3,
+        zlo = face_q<T, STRESS, INT>(load_face(S.fc[fcur][2], f, kk), 2, STRESS ? flags[c - cs2] : 0, fl, STRESS ? ud : zero3,
                                 uc, kk);
     }
     for (int k = k0; k <= k1; ++k) {
@@ -1210,29 +1270,29 @@ __global__ void __launch_bounds__(SX *SY, 3) k_phase1_faces(const __grid_constan
                 fn = flags[c - 1];
                 cellu(c - 1, un);
             }
-            Fx[ty][tx] = face_q<T, STRESS>(load_face(S.fc[fcur][0], f, kk), 0, fn, fl, un, uc, kk);
+            Fx[ty][tx] = face_q<T, STRESS, INT>(load_face(S.fc[fcur][0], f, kk), 0, fn, fl, un, uc, kk);
             if (i == ilast) {
                 if (STRESS) {
                     fn = flags[c + 1];
                     cellu(c + 1, un);
                 }
-                Fx[ty][tx + 1] = face_q<T, STRESS>(load_face(S.fc[fcur][0], f + 1, kk), 0, fl, fn, uc, un, kk);
+                Fx[ty][tx + 1] = face_q<T, STRESS, INT>(load_face(S.fc[fcur][0], f + 1, kk), 0, fl, fn, uc, un, kk);
             }
             if (STRESS) {
                 fn = flags[c - cs1];
                 cellu(c - cs1, un);
             }
-            Fy[ty][tx] = face_q<T, STRESS>(load_face(S.fc[fcur][1], f, kk), 1, fn, fl, un, uc, kk);
+            Fy[ty][tx] = face_q<T, STRESS, INT>(load_face(S.fc[fcur][1], f, kk), 1, fn, fl, un, uc, kk);
             if (j == jlast) {
                 if (STRESS) {
                     fn = flags[c + cs1];
                     cellu(c + cs1, un);
                 }
-                Fy[ty + 1][tx] = face_q<T, STRESS>(load_face(S.fc[fcur][1], f + fs1, kk), 1, fl, fn, uc, un, kk);
+                Fy[ty + 1][tx] = face_q<T, STRESS, INT>(load_face(S.fc[fcur][1], f + fs1, kk), 1, fl, fn, uc, un, kk);
             }
             flu = flags[c + cs2];
             cellu(c + cs2, uu);
-            zhi = face_q<T, STRESS>(load_face(S.fc[fcur][2], f + fs2, kk), 2, fl, flu, uc, uu, kk);
+            zhi = face_q<T, STRESS, INT>(load_face(S.fc[fcur][2], f + fs2, kk), 2, fl, flu, uc, uu, kk);
         }
         __syncthreads();
         if (valid) {
@@ -1252,7 +1312,7 @@ __global__ void __launch_bounds__(SX *SY, 3) k_phase1_faces(const __grid_constan
 #pragma unroll
                 for (int m = 0; m < 3; ++m) {
                     const T fx0 = Hx.mom[m] - Lx.mom[m], fx1 = Hy.mom[m] - Ly.mom[m], fx2 = zhi.mom[m] - zlo.mom[m];
-                    ucn[m] = qdiv_v(ro_c * uc[m] * kk.dvc - (T)0.5 * dt * (fx0 * kk.ds[0] + fx1 * kk.ds[1] + fx2 * kk.ds[2]),
+                    ucn[m] = qdiv_v(ro_c * uc[m] * kk.dvc - product<INT>((T)0.5 * dt, product<INT>(fx0, kk.ds[0]) + product<INT>(fx1, kk.ds[1]) + product<INT>(fx2, kk.ds[2])),
                                     den, qden);
                 }
             } else {
@@ -1264,9 +1324,9 @@ __global__ void __launch_bounds__(SX *SY, 3) k_phase1_faces(const __grid_constan
                 if (fl & FL_EQ0) {
 #pragma unroll
                     for (int m = 0; m < 3; ++m)
-                        fv[m] = ((Hx.sig[m] - Lx.sig[m]) * kk.ds[0] + (Hy.sig[m] - Ly.sig[m]) * kk.ds[1] +
-                                 (zhi.sig[m] - zlo.sig[m]) * kk.ds[2]) *
-                                ro_c;
+                        fv[m] = product<INT>(product<INT>(Hx.sig[m] - Lx.sig[m], kk.ds[0]) + product<INT>(Hy.sig[m] - Ly.sig[m], kk.ds[1]) +
+                                         product<INT>(zhi.sig[m] - zlo.sig[m], kk.ds[2]),
+                                     ro_c);
                     if (MODE & P1_BULK) fv[0] = bulk_force(fv[0], ro_c, kk, G);
                 }
                 S.f[0][c] = fv[0];
@@ -1427,6 +1487,12 @@ __device__ __forceinline__ float grad_sum(float d, float b, const SweepK<float> 
 __device__ __forceinline__ double twice_minus(double x, double y) { return __fma_rn(2.0, x, -y); }
 __device__ __forceinline__ float twice_minus(float x, float y) { return __fmaf_rn(2.f, x, -y); }
 
+// The limiter's bound max + dt * g (or min + dt * g), the product (bound_term) given in FP64.
+template <bool INT> __device__ __forceinline__ double bound_term(double dt, double g) { return product<INT>(dt, g); }
+template <bool INT> __device__ __forceinline__ float bound_term(float, float) { return 0.f; }
+__device__ __forceinline__ double bound(double, double, double t, double m) { return t + m; }
+__device__ __forceinline__ float bound(float dt, float g, float, float m) { return mad(dt, g, m); }
+
 // The Riemann invariants of a face, R = u_n + p/(ro0 c) and Q = u_n - p/(ro0 c)
 // (main.cpp:1790-1797).  The sweeps compute them once per face and hand them to the cell ahead.
 template <class T> struct RQ { T r, q; };
@@ -1438,13 +1504,14 @@ template <class T> __device__ __forceinline__ RQ<T> face_rq(T u_n, T p, const Sw
     return v;
 }
 
-// The extrapolation with the invariants of the forward (f) and backward (b) face given.
-template <class T, bool Q_USES_R>
+// The extrapolation with the invariants of the forward (f) and backward (b) face given.  INT: FP64 products on the integer
+// pipes (mulq).
+template <class T, bool Q_USES_R, bool INT = true>
 __device__ __forceinline__ Ext<T> extrapolate_rq(RQ<T> f, RQ<T> b, T u1_cn, T u1_c, T u2_f, T u2_b, T u2_cn, T u2_c,
                                                  T u3_f, T u3_b, T u3_cn, T u3_c, T ro_cn, T ro_c, const SweepK<T> &q) {
     constexpr bool DEV = Storage<T>::deviation;
-    const T p_cn = DEV ? q.c2 * ro_cn : q.c2 * (ro_cn - q.ro0);
-    const T p_c = DEV ? q.c2 * ro_c : q.c2 * (ro_c - q.ro0);
+    const T p_cn = product<INT>(q.c2, DEV ? ro_cn : ro_cn - q.ro0);
+    const T p_c = product<INT>(q.c2, DEV ? ro_c : ro_c - q.ro0);
     const T pcn = divq(p_cn, q.roc, q.rroc, q.qroc), pc = divq(p_c, q.roc, q.rroc, q.qroc);
 
     // max + dt*g: mad rounds it exactly as written in FP64, fused in FP32
@@ -1458,19 +1525,21 @@ __device__ __forceinline__ Ext<T> extrapolate_rq(RQ<T> f, RQ<T> b, T u1_cn, T u1
     T u3_fn = twice_minus(u3_cn, u3_b);
     T u3_bn = twice_minus(u3_cn, u3_f);
 
-    const T gr = grad_sum(r_cn - r_c, (u1_cn + q.sound) * (r_f - r_b), q);
-    const T gq = grad_sum(Q_USES_R ? (r_cn - r_c) : (q_cn - q_c), (u1_cn - q.sound) * (q_f - q_b), q);
-    const T gu2 = grad_sum(u2_cn - u2_c, u1_cn * (u2_f - u2_b), q);
-    const T gu3 = grad_sum(u3_cn - u3_c, u1_cn * (u3_f - u3_b), q);
+    const T gr = grad_sum(r_cn - r_c, product<INT>(u1_cn + q.sound, r_f - r_b), q);
+    const T gq = grad_sum(Q_USES_R ? (r_cn - r_c) : (q_cn - q_c), product<INT>(u1_cn - q.sound, q_f - q_b), q);
+    const T gu2 = grad_sum(u2_cn - u2_c, product<INT>(u1_cn, u2_f - u2_b), q);
+    const T gu3 = grad_sum(u3_cn - u3_c, product<INT>(u1_cn, u3_f - u3_b), q);
 
-    const T rmax = mad(q.dt, gr, max3d(r_f, r_c, r_b));
-    const T rmin = mad(q.dt, gr, min3d(r_f, r_c, r_b));
-    const T qmax = mad(q.dt, gq, max3d(q_f, q_c, q_b));
-    const T qmin = mad(q.dt, gq, min3d(q_f, q_c, q_b));
-    const T u2_max = mad(q.dt, gu2, max3d(u2_f, u2_c, u2_b));
-    const T u2_min = mad(q.dt, gu2, min3d(u2_f, u2_c, u2_b));
-    const T u3_max = mad(q.dt, gu3, max3d(u3_f, u3_c, u3_b));
-    const T u3_min = mad(q.dt, gu3, min3d(u3_f, u3_c, u3_b));
+    // dt * g: once for both bounds (FP64; FP32 fuses it with each)
+    const T tgr = bound_term<INT>(q.dt, gr), tgq = bound_term<INT>(q.dt, gq), tgu2 = bound_term<INT>(q.dt, gu2), tgu3 = bound_term<INT>(q.dt, gu3);
+    const T rmax = bound(q.dt, gr, tgr, max3d(r_f, r_c, r_b));
+    const T rmin = bound(q.dt, gr, tgr, min3d(r_f, r_c, r_b));
+    const T qmax = bound(q.dt, gq, tgq, max3d(q_f, q_c, q_b));
+    const T qmin = bound(q.dt, gq, tgq, min3d(q_f, q_c, q_b));
+    const T u2_max = bound(q.dt, gu2, tgu2, max3d(u2_f, u2_c, u2_b));
+    const T u2_min = bound(q.dt, gu2, tgu2, min3d(u2_f, u2_c, u2_b));
+    const T u3_max = bound(q.dt, gu3, tgu3, max3d(u3_f, u3_c, u3_b));
+    const T u3_min = bound(q.dt, gu3, tgu3, min3d(u3_f, u3_c, u3_b));
 
     limit(r_fn, rmax, rmin);
     limit(q_bn, qmax, qmin);
@@ -1541,7 +1610,7 @@ template <class T> struct NVals {
 // their flags and ucb/ucf their half-step normal velocities.  uA_old/uB_old: the face's
 // previous tangential velocities.  WALL_A_FROM_N: the x2 sweep takes the tangential u1 from
 // u2nCon in its wall branches (main.cpp:2219, 2238).
-template <class T, bool WALL_A_FROM_N, class NV>
+template <class T, bool WALL_A_FROM_N, bool INT = true, class NV>
 __device__ __forceinline__ FaceNew<T> face_values_v(const NV &V, uint8_t flb, uint8_t flf, T ucb, T ucf, const Ext<T> &prev,
                                                     const Ext<T> &cur, T uA_old, T uB_old, const SweepK<T> &q) {
     constexpr bool DEV = Storage<T>::deviation;
@@ -1549,7 +1618,7 @@ __device__ __forceinline__ FaceNew<T> face_values_v(const NV &V, uint8_t flb, ui
     if ((flb & FL_LT) && (flf & FL_LT)) {
         const T rn = prev.rf, qn = cur.qb;
         un = dhalf(rn + qn);
-        pn = dhalf((rn - qn) * q.sound * q.ro0);
+        pn = dhalf(product<INT>(product<INT>(rn - qn, q.sound), q.ro0));
         ro_n = q.ro0 + divq(pn, q.c2, q.rc2, q.qc2);
         if constexpr (DEV) {
             // the branches below as two conditions (a branch for the rare one only)
@@ -1623,11 +1692,11 @@ __device__ __forceinline__ FaceNew<T> face_values_v(const NV &V, uint8_t flb, ui
     return v;
 }
 // cb / cf index the cells behind and ahead in the half-step level N
-template <class T, bool WALL_A_FROM_N>
+template <class T, bool WALL_A_FROM_N, bool INT = true>
 __device__ __forceinline__ FaceNew<T> face_values(const NCell<T> &N, int cb, int cf, uint8_t flb, uint8_t flf, T ucb,
                                                   T ucf, const Ext<T> &prev, const Ext<T> &cur, T uA_old, T uB_old,
                                                   const SweepK<T> &q) {
-    return face_values_v<T, WALL_A_FROM_N>(NAt<T>{N, cb, cf}, flb, flf, ucb, ucf, prev, cur, uA_old, uB_old, q);
+    return face_values_v<T, WALL_A_FROM_N, INT>(NAt<T>{N, cb, cf}, flb, flf, ucb, ucf, prev, cur, uA_old, uB_old, q);
 }
 
 template <class T> __device__ __forceinline__ void face_store(const FaceOut<T> &W, int fc, const FaceNew<T> &v) {
@@ -1639,14 +1708,14 @@ template <class T> __device__ __forceinline__ void face_store(const FaceOut<T> &
 }
 
 // face_values stored into the new face generation at face fc
-template <class T, bool WALL_A_FROM_N>
+template <class T, bool WALL_A_FROM_N, bool INT = true>
 __device__ __forceinline__ void face_update(const NCell<T> &N, const FaceOut<T> &W, int cb, int cf, int fc,
                                             uint8_t flb, uint8_t flf, T ucb, T ucf, const Ext<T> &prev,
                                             const Ext<T> &cur, T uA_old, T uB_old, const SweepK<T> &q) {
     cb = ARK_CK(cb, N.nc);
     cf = ARK_CK(cf, N.nc);
     fc = ARK_CK(fc, W.nf);
-    face_store(W, fc, face_values<T, WALL_A_FROM_N>(N, cb, cf, flb, flf, ucb, ucf, prev, cur, uA_old, uB_old, q));
+    face_store(W, fc, face_values<T, WALL_A_FROM_N, INT>(N, cb, cf, flb, flf, ucb, ucf, prev, cur, uA_old, uB_old, q));
 }
 
 template <class T>
@@ -1761,7 +1830,7 @@ __device__ __forceinline__ int zface(int s, int C3, bool periodic) {
 // neighbouring lane, or the carry from the previous chunk's last lane.  Old faces come from
 // generation fcur, new faces go to fcur^1.
 
-template <class T>
+template <class T, bool INT = true>
 __device__ __forceinline__ void sweep_x_body(const DevState<T> &S, int con, int fcur, int glines, const BIx &bx, int nch = 0) {
     const Geom g = S.g;
     const int lane = threadIdx.x & 31;
@@ -1856,7 +1925,7 @@ __device__ __forceinline__ void sweep_x_body(const DevState<T> &S, int con, int 
         carry_rq.q = __shfl_sync(0xffffffffu, rqf.q, 31);
         Ext<T> e = {};
         if (act)
-            e = extrapolate_rq<T, true>(rqf, rqb, cur.nN, cur.cN, cur.uA_f, uA_b, cur.nA, cur.cA, cur.uB_f, uB_b, cur.nB,
+            e = extrapolate_rq<T, true, INT>(rqf, rqb, cur.nN, cur.cN, cur.uA_f, uA_b, cur.nA, cur.cA, cur.uB_f, uB_b, cur.nB,
                                         cur.cB, cur.nR, cur.cR, q);
         if (bounded && act) {
             // a bounded x axis sweeps cells 1..C1 only; the edge faces take the reference's
@@ -1892,7 +1961,7 @@ __device__ __forceinline__ void sweep_x_body(const DevState<T> &S, int con, int 
         carry_u = __shfl_sync(0xffffffffu, cur.nN, 31);
         carry_fl = (uint8_t)__shfl_sync(0xffffffffu, (int)cur.fl, 31);
         if (act && s >= 1 && !lead)
-            face_update<T, false>(N, W, c0 + s - 1 + dp, c0 + s + dc, f0 + s, flb, cur.fl, ucb, cur.nN, prev, e, uA_b,
+            face_update<T, false, INT>(N, W, c0 + s - 1 + dp, c0 + s + dc, f0 + s, flb, cur.fl, ucb, cur.nN, prev, e, uA_b,
                                   uB_b, q);
         cur = nxt;
         uA_b = nuA_b;
@@ -1992,7 +2061,7 @@ __global__ void __launch_bounds__(256) k_sweep_x_seams(const __grid_constant__ D
 __host__ __device__ inline int col_sweep_blocks(const Geom &g, int axis) {
     return (((g.C1 + 31) >> 5) * (axis == 1 ? g.C3 : g.C2) + 3) >> 2;
 }
-template <class T, int AX>
+template <class T, int AX, bool INT = true>
 __device__ __forceinline__ void sweep_col_body(const DevState<T> &S, int con, int fcur, int seg, const BIx &bx) {
     const Geom g = S.g;
     const int nic = (g.C1 + 31) >> 5;
@@ -2028,10 +2097,10 @@ __device__ __forceinline__ void sweep_col_body(const DevState<T> &S, int con, in
         const bool last = s + 1 == nd; // the next position is the ghost C3+1, its forward face C3+2
         if (s < s1) sweep_load(R, c + cst + (last ? c1 : 0), fb + 2 * fst + (last ? f1 : 0), nxt, c + cst);
         const RQ<T> rqf = face_rq(cur.uN_f, cur.p_f, q);
-        const Ext<T> e = extrapolate_rq<T, AX == 2>(rqf, rqb, cur.nN, cur.cN, cur.uA_f, uA_b, cur.nA, cur.cA, cur.uB_f,
+        const Ext<T> e = extrapolate_rq<T, AX == 2, INT>(rqf, rqb, cur.nN, cur.cN, cur.uA_f, uA_b, cur.nA, cur.cA, cur.uB_f,
                                                     uB_b, cur.nB, cur.cB, cur.nR, cur.cR, q);
         if (s > s0)
-            face_update<T, AX == 1>(N, W, c - cst + (s == 1 ? c0 : 0), c + (s == nd ? c1 : 0), fb, flprev, cur.fl, uprev,
+            face_update<T, AX == 1, INT>(N, W, c - cst + (s == 1 ? c0 : 0), c + (s == nd ? c1 : 0), fb, flprev, cur.fl, uprev,
                                     cur.nN, prev, e, uA_b, uB_b, q);
         prev = e;
         uprev = cur.nN;
@@ -2099,23 +2168,23 @@ __global__ void __launch_bounds__(128, 9) k_sweep_y_seams(const __grid_constant_
 // us per step, 200x60x1 56 -> 47, 128x96x96 1082 -> 1021, 256x128x128 3383 -> 3358; FP32 with the closure
 // 64x48x48 43 -> 40.  The registers are the x1 sweep's for all (FP64 three blocks per SM, where the
 // column sweeps alone have four; FP32 six instead of nine, so only for grids of a few waves).
-template <class T>
+template <class T, bool INT>
 __global__ void __launch_bounds__(128, sizeof(T) == 4 ? 6 : 3) k_sweeps(const __grid_constant__ DevState<T> S, int con, int fcur, int gl,
                                                                        int nch, int n1, int seg2, int n2, int c2, int seg3, int c3) {
     grid_release();
     grid_wait();
     BIx bx = {(int)blockIdx.x, 0, 0, 0, 0};
     if (bx.x < n1) {
-        sweep_x_body<T>(S, con, fcur, gl, bx, nch);
+        sweep_x_body<T, INT>(S, con, fcur, gl, bx, nch);
     } else if ((bx.x -= n1) < n2) {
         bx.z = bx.x / c2;
         bx.x -= bx.z * c2;
-        sweep_col_body<T, 1>(S, con, fcur, seg2, bx);
+        sweep_col_body<T, 1, INT>(S, con, fcur, seg2, bx);
     } else {
         bx.x -= n2;
         bx.z = bx.x / c3;
         bx.x -= bx.z * c3;
-        sweep_col_body<T, 2>(S, con, fcur, seg3, bx);
+        sweep_col_body<T, 2, INT>(S, con, fcur, seg3, bx);
     }
 }
 
@@ -2533,6 +2602,12 @@ template <class T> void Launch<T>::halo_exchange(const Geom &g, const HaloJob *j
     k_halo<T><<<dim3((g.C1 * g.C2 + 255) / 256, njobs), 256, 0, st>>>(g, jobs);
 }
 
+// Whether a grid's FP64 kernels take products on the integer pipes (mulq): from about eight warps of
+// cells per SM on, where the FP64 pipe is the bound.  Below that a step waits for its chain of dependent
+// operations, which mulq makes longer (32x24x20: 52.5 us per step with multiplies, 60.6 with mulq;
+// 200x60x1 43.9 and 44.7; 64x32x19, at the line, 77.0 and 74.9; 48x40x32 120.5 and 105.2).
+inline bool int_products(const Geom &g) { return (long long)g.C1 * g.C2 * g.C3 >= 152 * 256; }
+
 template <class T, template <class, int> class KERNEL>
 void launch_phase1(const DevState<T> &S, int src, int dst, int fcur, int mode, dim3 grid, cudaStream_t st) {
     const dim3 block(kTileX, kTileY);
@@ -2597,10 +2672,15 @@ void Launch<T>::phase1(const DevState<T> &S, int src, int dst, int fcur, int mod
             const dim3 block(fcs::SX, fcs::SY);
             constexpr int A = P1_STRESS | P1_FORCES | P1_RMAX, B = A | P1_BULK, C = P1_FORCES | P1_RSUM;
             auto go = [&](auto kernel) { launch_early(false, kernel, grid, block, fcs::face_smem<T>(), st, S, src, dst, fcur, kch); };
+            auto pick = [&](auto m) {
+                constexpr int M = decltype(m)::value;
+                if (int_products(S.g)) go(fcs::k_phase1_faces<T, M, true>);
+                else go(fcs::k_phase1_faces<T, M, false>);
+            };
             switch (mode) {
-            case A: go(fcs::k_phase1_faces<T, A>); return;
-            case B: go(fcs::k_phase1_faces<T, B>); return;
-            case C: go(fcs::k_phase1_faces<T, C>); return;
+            case A: pick(std::integral_constant<int, A>()); return;
+            case B: pick(std::integral_constant<int, B>()); return;
+            case C: pick(std::integral_constant<int, C>()); return;
             default: march = 0; break;
             }
         }
@@ -2677,8 +2757,12 @@ template <class T> bool Launch<T>::sweeps(const DevState<T> &S, int con, int fcu
     constexpr bool fp64 = sizeof(T) == 8;
     const SweepCut c = sweep_cut(S.g, target, fp64);
     if (!fp64 && c.n1 + c.n2 + c.n3 > 3 * 6 * 152) return false;
-    launch_early(!fp64 && early_grid(S.g), k_sweeps<T>, dim3(c.n1 + c.n2 + c.n3), dim3(128), 0, st, S, con, fcur, c.gl, c.nch, c.n1, c.seg2, c.n2, c.c2, c.seg3,
-                 c.c3);
+    auto go = [&](auto kernel) {
+        launch_early(!fp64 && early_grid(S.g), kernel, dim3(c.n1 + c.n2 + c.n3), dim3(128), 0, st, S, con, fcur, c.gl, c.nch, c.n1,
+                     c.seg2, c.n2, c.c2, c.seg3, c.c3);
+    };
+    if (fp64 && int_products(S.g)) go(k_sweeps<T, fp64>);
+    else go(k_sweeps<T, false>);
     return true;
 }
 
@@ -2701,11 +2785,14 @@ bool Launch<T>::sweep_y_seams(const DevState<T> &S, int con, int fcur, const XSe
 template <class T> void Launch<T>::prepare() {
     if constexpr (std::is_same<T, double>::value) {
         constexpr int fb = fcs::face_smem<double>();
-        cudaFuncSetAttribute(fcs::k_phase1_faces<double, P1_STRESS | P1_FORCES | P1_RMAX>,
-                             cudaFuncAttributeMaxDynamicSharedMemorySize, fb);
-        cudaFuncSetAttribute(fcs::k_phase1_faces<double, P1_STRESS | P1_FORCES | P1_BULK | P1_RMAX>,
-                             cudaFuncAttributeMaxDynamicSharedMemorySize, fb);
-        cudaFuncSetAttribute(fcs::k_phase1_faces<double, P1_FORCES | P1_RSUM>, cudaFuncAttributeMaxDynamicSharedMemorySize, fb);
+        constexpr int A = P1_STRESS | P1_FORCES | P1_RMAX, B = A | P1_BULK, C = P1_FORCES | P1_RSUM;
+        auto attr = [&](auto kernel) { cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, fb); };
+        attr(fcs::k_phase1_faces<double, A, true>);
+        attr(fcs::k_phase1_faces<double, B, true>);
+        attr(fcs::k_phase1_faces<double, C, true>);
+        attr(fcs::k_phase1_faces<double, A, false>);
+        attr(fcs::k_phase1_faces<double, B, false>);
+        attr(fcs::k_phase1_faces<double, C, false>);
     }
     if constexpr (std::is_same<T, float>::value) {
         stg::prepare_staged<P1_STRESS | P1_FORCES | P1_RMAX>();
