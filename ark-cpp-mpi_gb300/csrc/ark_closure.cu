@@ -349,10 +349,10 @@ __device__ __forceinline__ void features_fp64(const double A[3][3], double y, do
 // wall counts as minus the cell), box-filtered 3 x 3 x 3, into three compact interior arrays
 // ub + m * cells ([k][j][i], FP64).  A block takes 32 x FY cells of a plane and marches up kch planes:
 // the sums along x of FY + 2 rows go through shared memory (two planes' buffers in turn, one barrier
-// per plane), the sums over x and y of the last three planes stay in registers.  Eight FP64
-// operations per value, against six and three divisions in three passes over memory: 700 us (and 32
-// for a gathered FP64 copy) -> 229 at 256x128x128, the FP64 pipe 73% busy (16 rows per block and three
-// blocks per SM, with spills, the same).
+// per plane), the sums over x and y of the last three planes stay in registers.  Seven FP64 sums
+// per value and a product on the integer pipes (mulq), against six and three divisions in three passes
+// over memory: 700 us (and 32 for a gathered FP64 copy) -> 229 at 256x128x128, 215 with mulq (16 rows per
+// block and three blocks per SM, with spills, the same).
 constexpr int FY = 8;
 template <class T>
 __global__ void __launch_bounds__(32 * (FY + 2), 4) k_filter_velocity(const __grid_constant__ DevState<T> S, int lvl, double *ub, int kch) {
@@ -387,7 +387,7 @@ __global__ void __launch_bounds__(32 * (FY + 2), 4) k_filter_velocity(const __gr
                 const double neg = __hiloint2double(__double2hiint(x[m]) ^ (int)0x80000000, __double2loint(x[m]));
                 const double lo = j == 1 ? neg : xs[buf][m][ty - 1][tx], hi = j == g.C2 ? neg : xs[buf][m][ty + 1][tx];
                 const double xy = (lo + x[m]) + hi;
-                if (p > k0) ub[m * cells + out] = ((z0[m] + z1[m]) + xy) * (1.0 / 27.0);
+                if (p > k0) ub[m * cells + out] = mulq((z0[m] + z1[m]) + xy, 1.0 / 27.0);
                 z0[m] = z1[m];
                 z1[m] = xy;
             }
@@ -406,9 +406,9 @@ __device__ __forceinline__ void grad_compact(const double *const u[3], int i, in
     for (int m = 0; m < 3; ++m) {
         const double c = u[m][t];
         const double jl = j == 0 ? -c : u[m][t - C1], jh = j == C2 - 1 ? -c : u[m][t + C1];
-        A[m][0] = (u[m][ip] - u[m][im]) * (m == 0 ? rdx2[0] : 0.5 * rdx2[0]);
-        A[m][1] = (jh - jl) * (m == 1 ? rdx2[1] : 0.5 * rdx2[1]);
-        A[m][2] = (u[m][kp] - u[m][km]) * (m == 2 ? rdx2[2] : 0.5 * rdx2[2]);
+        A[m][0] = mulq(u[m][ip] - u[m][im], m == 0 ? rdx2[0] : 0.5 * rdx2[0]);
+        A[m][1] = mulq(jh - jl, m == 1 ? rdx2[1] : 0.5 * rdx2[1]);
+        A[m][2] = mulq(u[m][kp] - u[m][km], m == 2 ? rdx2[2] : 0.5 * rdx2[2]);
     }
 }
 
@@ -426,7 +426,7 @@ struct SampleArgs {
 // the nine cells' products of a row summed in x and z, and the sums of three rows in registers
 // (a row beyond a wall counts as the row itself).  Every product filtered everywhere took 18 passes
 // (1400 us) and 55 us of products; the samples of a 4 x 4 lattice 180 -> 165 with the products in them,
-// the FP64 pipe 83% busy.
+// the FP64 pipe 83% busy (161 with the gradients' products on the integer pipes).
 template <class T> __global__ void __launch_bounds__(128) k_samples(const __grid_constant__ DevState<T> S, int lvl, SampleArgs s) {
     const Geom g = S.g;
     const int C1 = g.C1, C2 = g.C2, C3 = g.C3;

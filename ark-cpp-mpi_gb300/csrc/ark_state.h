@@ -403,6 +403,61 @@ __device__ __forceinline__ double widen(float v) {
         return __hiloint2double((int)((b & 0x80000000u) | (((b & 0x7FFFFFFFu) >> 3) + 0x38000000u)), (int)(b << 29));
     return (b << 1) == 0u ? __hiloint2double((int)b, 0) : widen_call(v);
 }
+// RN(a * b) on the integer pipes: the 106-bit product of the significands, normalised and rounded to
+// nearest even.  Other than normal operands with a normal product take the multiply, zeros a zero.
+// GB300's FP64 pipe takes 16 cycles of an SM for a warp's instruction, about 32 instructions' worth of
+// its four schedulers, and the FP64 kernels left those three quarters idle; with part of their products
+// here the two run side by side (256x128x128: x2 sweep 498 -> 404 us, x3 494 -> 406, x1 459 -> 447, with
+// 12 of a cell's 51 FP64 instructions; Phase1 + stress 1199 -> 1035, with 21 of 132, the products with
+// face areas; second Phase1 752 -> 561, with 30 of 75; the step 3350 -> 2856.  More of them in Phase1 +
+// stress is slower again: 1047 with 7 more, 1324 with all.)
+static __device__ __noinline__ double mul_call(double a, double b) { return a * b; }
+__device__ __forceinline__ double mulq(double a, double b) {
+    const unsigned ha = (unsigned)__double2hiint(a), a0 = (unsigned)__double2loint(a);
+    const unsigned hb = (unsigned)__double2hiint(b), lb = (unsigned)__double2loint(b);
+    constexpr unsigned EXP = 0x7FF00000u, ONE = 1u << 20;
+    // a's significand (53 bits) and b's shifted to the top of 64: w3:w2 has 52 or 53 bits
+    const unsigned a1 = (ha & 0xFFFFFu) | ONE, b1 = __funnelshift_l(lb, hb, 11) | 0x80000000u, b0 = lb << 11;
+    unsigned w0, w1, w2, w3;
+    asm("mul.lo.u32 %0, %4, %6;\n\t"
+        "mul.hi.u32 %1, %4, %6;\n\t"
+        "mad.lo.cc.u32 %1, %4, %7, %1;\n\t"
+        "madc.hi.u32 %2, %4, %7, 0;\n\t"
+        "mad.lo.cc.u32 %1, %5, %6, %1;\n\t"
+        "madc.hi.cc.u32 %2, %5, %6, %2;\n\t"
+        "addc.u32 %3, 0, 0;\n\t"
+        "mad.lo.cc.u32 %2, %5, %7, %2;\n\t"
+        "madc.hi.u32 %3, %5, %7, %3;"
+        : "=&r"(w0), "=&r"(w1), "=&r"(w2), "=&r"(w3)
+        : "r"(a0), "r"(a1), "r"(b0), "r"(b1));
+    const unsigned s = 1u - (w3 >> 20); // 1: 52 bits
+    const unsigned hi = __funnelshift_l(w2, w3, s), lo = __funnelshift_l(w1, w2, s);
+    const unsigned r1 = __funnelshift_l(w0, w1, s), r0 = w0 << s; // below the last bit
+    // the product's exponent less one, in place; the hidden bit of hi adds the one
+    const unsigned e = (ha & EXP) + (hb & EXP) - 1023u * ONE - s * ONE;
+    // rounded: half a unit less one, and one more where the last bit is odd, carries into it
+    unsigned top, low;
+    asm("{\n\t.reg .u32 t;\n\t"
+        "add.cc.u32 t, %2, 0xFFFFFFFF;\n\t"
+        "addc.cc.u32 t, %3, 0xFFFFFFFF;\n\t"
+        "addc.cc.u32 t, %4, 0x7FFFFFFF;\n\t"
+        "addc.cc.u32 %0, %5, 0;\n\t"
+        "addc.u32 %1, %6, %7;\n\t}"
+        : "=&r"(low), "=&r"(top)
+        : "r"(lo & 1u), "r"(r0), "r"(r1), "r"(lo), "r"(hi), "r"(e));
+    // both exponents in 2^-511 .. 2^512 (their top bits differ), and the product's below the largest
+    if (((ha ^ (ha << 1)) & (hb ^ (hb << 1)) & 0x40000000u) && e < 2044u * ONE)
+        return __hiloint2double((int)(top | ((ha ^ hb) & 0x80000000u)), (int)low);
+    const bool za = ((ha << 1) | a0) == 0u, zb = ((hb << 1) | lb) == 0u;
+    if ((za || zb) && (ha & EXP) != EXP && (hb & EXP) != EXP) return __hiloint2double((int)((ha ^ hb) & 0x80000000u), 0);
+    return mul_call(a, b);
+}
+__device__ __forceinline__ float mulq(float a, float b) { return a * b; }
+// INT: mulq, else the multiply
+template <bool INT, class T> __device__ __forceinline__ T product(T a, T b) {
+    if constexpr (INT) return mulq(a, b);
+    else return a * b;
+}
 // Rows of cells for a statistics kernel: block (x, y) of a grid of `planes` x gridDim.y blocks, 8
 // warps, takes the rows k = 8 y + warp + 1, + 8 gridDim.y, ... of plane j = x + 1, lanes on i.
 constexpr int kStatWarps = 8;
