@@ -163,7 +163,8 @@ static __device__ __noinline__ double div_rn_call(double a, double b, double rb)
 // A zero numerator is the one case of the other path that whole fields meet (a component at rest,
 // a still region): its quotient by a normal divisor is the zero of the signs' product, without the
 // call.  In the 200x60x1 flow over a step (u3 = 0 everywhere) the calls took most of the sweeps'
-// time: x1 20 -> 10 us, x2 31 -> 12, x3 37 -> 14, Phase1 + stress 30 -> 20, the step 123 -> 62.
+// time: x1 20 -> 10 us, x2 31 -> 12, x3 37 -> 14, Phase1 + stress 30 -> 20, the step 123 -> 62 (44 with
+// the sweeps in one launch and graphs of several steps).
 __device__ __forceinline__ bool zero_over_normal(double a, const QRecip &Q) {
     return (((unsigned)__double2hiint(a) << 1) | (unsigned)__double2loint(a)) == 0u && Q.k != -100000;
 }
@@ -2112,7 +2113,8 @@ __global__ void __launch_bounds__(128, 9) k_sweep_y_seams(const __grid_constant_
 // a segment).  One after the other, each ends in a wave that leaves most SMs idle: FP64 64x32x32 96 -> 90
 // us per step, 200x60x1 56 -> 47, 128x96x96 1082 -> 1021, 256x128x128 3383 -> 3358; FP32 with the closure
 // 64x48x48 43 -> 40.  The registers are the x1 sweep's for all (FP64 three blocks per SM, where the
-// column sweeps alone have four; FP32 six instead of nine, so only for grids of a few waves).
+// column sweeps alone have four; FP32 six instead of nine, so only for grids of a few waves).  (FP64
+// figures before mulq.)
 template <class T, bool INT>
 __global__ void __launch_bounds__(128, sizeof(T) == 4 ? 6 : 3) k_sweeps(const __grid_constant__ DevState<T> S, int con, int fcur, int gl,
                                                                        int nch, int n1, int seg2, int n2, int c2, int seg3, int c3) {
@@ -2383,7 +2385,7 @@ inline int x_chunks_per_warp(const Geom &g, int gl, bool fp64) {
 }
 // Segments of the x2 / x3 sweeps: of at most `target` faces, balanced so no thread gets a short
 // tail; where those are fewer than two waves of four blocks per SM (FP32: one wave of nine), the
-// count with the least load instead, if it is larger.  FP64, us: 64x32x32 66 / 56 -> 23 / 16 (2 faces; 1 face 27 /
+// count with the least load instead, if it is larger.  FP64 (before mulq), us: 64x32x32 66 / 56 -> 23 / 16 (2 faces; 1 face 27 /
 // 19, 4 faces 26 / 18), 200x60x1 x2 153 -> 28 (1 face), 96x64x64 89 / 77 -> 69 / 61.  FP32: 64x48x48
 // x2 13.6 -> 5.5 (2 faces instead of 13), 150x67x93 17.7 -> 15 (8 instead of 14).
 inline int sweep_segment(int nd, int target, int blocks, bool fp64, int *nseg) {
@@ -2423,7 +2425,7 @@ inline SweepCut sweep_cut(const Geom &g, int target, bool fp64) {
     c.n2 = c.c2 * m2;
     c.n3 = c.c3 * m3;
     if (!fp64 || c.n1 + c.n2 + c.n3 > 4 * 3 * 152) return c;
-    // FP64 grids of a few waves: segments of the x2 and x3 sweeps that fill whole waves of three blocks
+    // FP64 grids of a few waves (figures before mulq): segments of the x2 and x3 sweeps that fill whole waves of three blocks
     // per SM (96x64x64: 384 blocks of 18 cells 403 us per step, 576 of 12 cells 430; 128x64x64: 896 of 11
     // cells 469, 512 of 18 cells 499, 1408 of 7 cells 489)
     int least = 1 << 30;
