@@ -19,6 +19,7 @@
 #include <cstdio>
 #include <cstring>
 #include <memory>
+#include <queue>
 #include <string>
 #include <vector>
 
@@ -399,6 +400,30 @@ int seam_width(const Shape &s, const Geom &g) {
     return t && narrow_tiles(g.C1) ? 32 : 64;
 }
 
+// The time until the last of E's staged blocks is done, in planes, when they take the members' chunks of
+// up to kens planes in turn, an item taking two planes' time to start (and 0.8 of its time where at most
+// one block runs per SM).
+double staged_end(const ark_ensemble *E, int kens) {
+    std::vector<int> planes;
+    for (int q = 0; q < E->n; ++q) {
+        const Geom &g = E->S[q].g;
+        const int nch = (g.C3 + kens - 1) / kens, kch = (g.C3 + nch - 1) / nch;
+        const bool narrow = narrow_tiles(g.C1);
+        const int tiles = narrow ? ((g.C1 + 31) / 32) * ((g.C2 + 7) / 8) : ((g.C1 + 63) / 64) * ((g.C2 + 3) / 4);
+        for (int k = 0; k < g.C3; k += kch) planes.insert(planes.end(), tiles, std::min(kch, g.C3 - k));
+    }
+    std::priority_queue<int, std::vector<int>, std::greater<int>> ends;
+    for (int b = 0; b < E->persist_staged; ++b) ends.push(0);
+    int last = 0;
+    for (int n : planes) {
+        const int end = ends.top() + n + 2;
+        ends.pop();
+        ends.push(end);
+        last = std::max(last, end);
+    }
+    return (int)planes.size() <= E->persist_staged / 2 ? 0.8 * last : last;
+}
+
 // Builds the work lists for the current shape.
 int build_lists(ark_ensemble *E) {
     // Planes per staged Phase1 block, sized over the whole ensemble (about four waves of two
@@ -412,7 +437,21 @@ int build_lists(ark_ensemble *E) {
         const Geom &g = E->S[q].g;
         colplanes += (long long)tiles_x(g) * ((g.C2 + stg::SY - 1) / stg::SY) * g.C3;
     }
-    const int kens = (int)std::max(8ll, std::min(64ll, colplanes / (152 * 2 * 4)));
+    int kens = (int)std::max(8ll, std::min(64ll, colplanes / (152 * 2 * 4)));
+    // A small ensemble (fewer than 64 planes for each resident block) has few enough chunks for their
+    // lengths to leave blocks idle at its end: the length that ends first, if by more than 5%
+    // (members, us per step: 4 of 64x48x48 to 128x64x64, 8 planes 162.4 -> 16 planes 150.6; 8 of 32x32x32
+    // to 96x64x64, 8 planes 141 -> 12 planes 124).
+    if (colplanes < 152 * 2 * 64) {
+        double least = 0.95 * staged_end(E, kens);
+        for (int k : {4, 6, 8, 10, 12, 14, 16, 20, 24, 28, 32, 40, 48, 64}) {
+            const double end = staged_end(E, k);
+            if (end < least || (end == least && k > kens)) {
+                least = end;
+                kens = k;
+            }
+        }
+    }
     for (int kind = 0; kind < WL_COUNT; ++kind) {
         std::vector<int4> info(E->n);
         std::vector<int> extra(E->n, 0);
@@ -783,6 +822,15 @@ ark_ensemble *ark_ensemble_create(const ark_params *params, int n, int *status) 
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kb_phase1<P1_FORCES | P1_RSUM, false>, kTileX * kTileY, 0);
     E->persist = sms * std::max(per, 1) * 2;
     E->persist_staged = prepare_staged_kernels(sms);
+    // segments of the x2 sweep: 32 faces, of a small ensemble (two blocks for each that fits at once) 16
+    // (alone 4 members 162 -> 156 us per step, 8 141 -> 133, 16 467 -> 462, 32 705 -> 703; with
+    // the chunks above 144, 117, 463)
+    long long blocks = 0;
+    for (int q = 0; q < E->n; ++q) {
+        const Geom &g = E->S[q].g;
+        blocks += (long long)col_sweep_blocks(g, 1) * ((g.C2 + 32) / 32);
+    }
+    if (blocks < 2 * 6 * sms) E->shape.seg = 16;
     stg::encode_tiled(); // looked up here, outside any stream capture
     if ((*status = build_lists(E.get())) || (*status = build_jobs(E.get())) || (*status = build_maps(E.get())) ||
         (*status = ens_alloc(E.get(), &E->d_next, 7)))
