@@ -933,12 +933,18 @@ int ark_ensemble_download(ark_ensemble *E, int q, ark_host_state *h) {
     const int c = E->con, n = E->con ^ 1, fc = E->fcur;
     double *cells[8] = {h->roCon, h->u1Con, h->u2Con, h->u3Con, h->ronCon, h->u1nCon, h->u2nCon, h->u3nCon};
     float *dcell[8] = {S.lv[c].ro, S.lv[c].u1, S.lv[c].u2, S.lv[c].u3, S.lv[n].ro, S.lv[n].u1, S.lv[n].u2, S.lv[n].u3};
+    // one staging buffer, one stream: an array's conversion waits for the copy before it, the host for the
+    // last copy only (64 members' eight arrays, 862 MB, after 100 steps: 137.7 -> 136.3 ms)
+    cudaError_t err = cudaSuccess;
+    auto back = [&](double *to, const RowShape &r) {
+        if (err == cudaSuccess)
+            err = cudaMemcpyAsync(to, E->stage, sizeof(double) * r.w * r.rows, cudaMemcpyDeviceToHost, E->st);
+    };
     for (int a = 0; a < 8; ++a) {
         if (!cells[a]) continue;
         const RowShape r = row_shape(S.g, 0);
         rows_to_double<float>(E->stage, dcell[a], r.w, r.rows, r.pitch, (a % 4 == 0) ? ro0 : 0.0, E->st);
-        ENS_CUDA(cudaMemcpyAsync(cells[a], E->stage, sizeof(double) * r.w * r.rows, cudaMemcpyDeviceToHost, E->st));
-        ENS_CUDA(cudaStreamSynchronize(E->st));
+        back(cells[a], r);
     }
     double *faces[3][5] = {{h->p1, h->ro1, h->u11, h->u21, h->u31},
                            {h->p2, h->ro2, h->u12, h->u22, h->u32},
@@ -951,10 +957,12 @@ int ark_ensemble_download(ark_ensemble *E, int q, ark_host_state *h) {
             const RowShape r = row_shape(S.g, 1);
             if (a == 1) rows_face_density<float>(E->stage, F.p, r.w, r.rows, r.pitch, E->K[q].ro0, E->K[q].rc2, E->st);
             else rows_to_double<float>(E->stage, df[a], r.w, r.rows, r.pitch, 0.0, E->st);
-            ENS_CUDA(cudaMemcpyAsync(faces[d][a], E->stage, sizeof(double) * r.w * r.rows, cudaMemcpyDeviceToHost, E->st));
-            ENS_CUDA(cudaStreamSynchronize(E->st));
+            back(faces[d][a], r);
         }
     }
+    const cudaError_t last = cudaStreamSynchronize(E->st); // also after an error: nothing is left in flight
+    ENS_CUDA(err);
+    ENS_CUDA(last);
     if (h->condition) std::memcpy(h->condition, E->cond_host[q].data(), sizeof(double) * E->cond_host[q].size());
     return ARK_OK;
 }
