@@ -290,17 +290,24 @@ __device__ __forceinline__ float narrow(double x) {
     const unsigned m = (((h & 0x7FFFFFFFu) - 0x38000000u) << 3) | (l >> 29), rest = l << 3;
     return __uint_as_float((h & 0x80000000u) | (m + (rest > 0x80000000u || (rest == 0x80000000u && (m & 1u)) ? 1u : 0u)));
 }
+// A zero and a NaN come back as they are.
 __device__ __forceinline__ double root2(double x) {
-    if (!float_range(x)) return x > 0 ? sqrt_call(x) : 0.0;
+    if (!float_range(x)) return x > 0 ? sqrt_call(x) : x;
     const float r = sqrtf(to_float24(x));
     const double y = widen(r);
     return __fma_rn(__fma_rn(-y, y, x), widen(0.5f / r), y);
 }
 __device__ __forceinline__ double root3(double x) {
-    if (!float_range(x)) return x > 0 ? cbrt_call(x) : 0.0;
+    if (!float_range(x)) return x > 0 ? cbrt_call(x) : x;
     const float r = cbrtf(to_float24(x));
     const double y = widen(r);
     return __fma_rn(__fma_rn(-y * y, y, x), widen(1.0f / (3.0f * r * r)), y);
+}
+// By their bits (a comparison of doubles is an FP64 operation): whether x is finite; x, or 0 for a NaN.
+__device__ __forceinline__ bool finite_bits(double x) { return ((unsigned)__double2hiint(x) & 0x7FF00000u) != 0x7FF00000u; }
+__device__ __forceinline__ double or_zero(double x) {
+    const unsigned h = (unsigned)__double2hiint(x) & 0x7FFFFFFFu;
+    return h > 0x7FF00000u || (h == 0x7FF00000u && __double2loint(x) != 0) ? 0.0 : x;
 }
 // features_of for the training data, in FP64 with the fewest operations: with W x = w cross x (the
 // antisymmetric part), W^2 = w w^T - |w|^2 I, so the mixed invariants are dot products of w, S w and
@@ -329,8 +336,10 @@ __device__ __forceinline__ void features_fp64(const double A[3][3], double y, do
     const double c[3] = {w[1] * z[2] - w[2] * z[1], w[2] * z[0] - w[0] * z[2], w[0] * z[1] - w[1] * z[0]};
     const double i4 = dot(w, v) - ww * trS, i5 = dot(v, v) - ww * trS2, i6 = dot(v, c);
     f[0] = trS;
-    f[1] = root2(trS2);
-    f[2] = root2(2.0 * ww);
+    // of a NaN invariant features 1 and 2 are 0 (the root of its positive part), 3 to 6 NaN; a diagonal
+    // that is not finite makes W's diagonal, and so W^2's trace, a NaN
+    f[1] = or_zero(root2(trS2));
+    f[2] = finite_bits(trS) ? or_zero(root2(2.0 * ww)) : 0.0;
     f[3] = copysign(root3(fabs(trS3)), trS3);
     f[4] = copysign(root3(fabs(i4)), i4);
     f[5] = copysign(root2(root2(fabs(i5))), i5);
