@@ -272,9 +272,11 @@ __device__ __forceinline__ void features_of(const R A[3][3], R y, R ly, R yplus_
     f[9] = ((R)0.5 * ly - fabs(y)) * yplus_scale;
 }
 
-// x^(1/2) and x^(1/3) of x >= 0 for the training data: the FP32 root of x (rounded to 24 bits by
-// integer instructions) and one Newton step in FP64, relative error near 1e-14 (the rows are stored
-// as FP32); values outside FP32's comfortable range take the library's FP64 root, as a call.
+// x^(1/2) and x^(1/3) of x >= 0 for the training data: the FP32 root of x (truncated to 24 bits by
+// integer instructions) and two Newton steps in FP64 with the FP32 slope.  The first leaves an error
+// near 2^-46, the second the rounding of its last operation (root3: and a third of an ulp for the cube's
+// square): the square root within 0.501 ulp, the cube root within 1 ulp, the bounds of the FP64 sqrt and
+// cbrt (selftest_roots compares).  Values outside FP32's comfortable range take those, as a call.
 static __device__ __noinline__ double sqrt_call(double x) { return sqrt(x); }
 static __device__ __noinline__ double cbrt_call(double x) { return cbrt(x); }
 __device__ __forceinline__ float to_float24(double x) { // x in [2^-100, 2^100)
@@ -294,14 +296,18 @@ __device__ __forceinline__ float narrow(double x) {
 __device__ __forceinline__ double root2(double x) {
     if (!float_range(x)) return x > 0 ? sqrt_call(x) : x;
     const float r = sqrtf(to_float24(x));
-    const double y = widen(r);
-    return __fma_rn(__fma_rn(-y, y, x), widen(0.5f / r), y);
+    const double h = widen(0.5f / r);
+    double y = widen(r);
+    y = __fma_rn(__fma_rn(-y, y, x), h, y);
+    return __fma_rn(__fma_rn(-y, y, x), h, y);
 }
 __device__ __forceinline__ double root3(double x) {
     if (!float_range(x)) return x > 0 ? cbrt_call(x) : x;
     const float r = cbrtf(to_float24(x));
-    const double y = widen(r);
-    return __fma_rn(__fma_rn(-y * y, y, x), widen(1.0f / (3.0f * r * r)), y);
+    const double h = widen(1.0f / (3.0f * r * r));
+    double y = widen(r);
+    y = __fma_rn(__fma_rn(-y * y, y, x), h, y);
+    return __fma_rn(__fma_rn(-y * y, y, x), h, y);
 }
 // By their bits (a comparison of doubles is an FP64 operation): whether x is finite; x, or 0 for a NaN.
 __device__ __forceinline__ bool finite_bits(double x) { return ((unsigned)__double2hiint(x) & 0x7FF00000u) != 0x7FF00000u; }
@@ -535,6 +541,38 @@ __global__ void __launch_bounds__(256) k_plane_stats_compact(const double *u0, c
         __syncthreads();
     }
     if (threadIdx.x < 9) out[9 * j + threadIdx.x] = red[threadIdx.x][0] / (double)n;
+}
+
+// Self-check of root2 and root3 on n values (random significands, exponents beyond the range that they
+// take themselves on both sides; exact squares and cubes), their errors from FP64 residuals: x - y^2 is
+// one exact FMA, x - y^3 comes from the two-term cube.  Counts square roots off by more than 0.501 ulp,
+// cube roots by more than 1 ulp (the bounds of sqrt and cbrt), and zeros, infinities and NaN that do not
+// come back as they are.
+__global__ void k_selftest_roots(long long n, unsigned long long seed, unsigned long long *bad) {
+    unsigned long long local = 0;
+    auto ulp = [](double y) { return __longlong_as_double((__double_as_longlong(y) & 0x7FF0000000000000ll) - (52ll << 52)); };
+    for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < n; t += (long long)gridDim.x * blockDim.x) {
+        unsigned long long z = seed + 0x9E3779B97F4A7C15ull * (unsigned long long)(t + 1);
+        z = (z ^ (z >> 30)) * 0xBF58476D1CE4E5B9ull;
+        z = (z ^ (z >> 27)) * 0x94D049BB133111EBull;
+        z ^= z >> 31;
+        const long long e = 1023 - 110 + (long long)((z >> 52) % 221); // [2^-110, 2^111)
+        double x = __longlong_as_double((e << 52) | (long long)(z & 0x000FFFFFFFFFFFFFull));
+        const double m = (double)(long long)(z & 0xFFFFull) + 1.0;
+        if ((t & 15) == 7) x = m * m;
+        if ((t & 15) == 11) x = m * m * m;
+        const double y = root2(x), r2 = __fma_rn(-y, y, x);
+        if (!(fabs(r2) <= 0.501 * ulp(y) * (2.0 * y)) || ((t & 15) == 7 && y != m)) ++local;
+        const double w = root3(x), s = __dmul_rn(w, w), ds = __fma_rn(w, w, -s), c = __dmul_rn(s, w);
+        const double dc = __dadd_rn(__fma_rn(s, w, -c), __dmul_rn(ds, w)), r3 = __dadd_rn(__dadd_rn(x, -c), -dc);
+        if (!(fabs(r3) <= ulp(w) * (3.0 * s)) || ((t & 15) == 11 && w != m)) ++local;
+    }
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        const double inf = __longlong_as_double(0x7FF0000000000000ll), nan = __longlong_as_double(0x7FF8000000000000ll);
+        if (root2(0.0) != 0.0 || root3(0.0) != 0.0 || root2(inf) != inf || root3(inf) != inf) ++local;
+        if (root2(nan) == root2(nan) || root3(nan) == root3(nan)) ++local;
+    }
+    if (local) atomicAdd(bad, local);
 }
 
 // ---- training on the tensor cores ---------------------------------------------------------
@@ -1527,6 +1565,10 @@ int ark_mlp_predict(ark_mlp *M, ark_closure_data *d, long long first, long long 
 // the network constants, for ark_api.cu's closure step
 namespace ark {
 const void *mlp_device_net(const ark_mlp *M) { return M ? (const void *)M->net : nullptr; }
+void selftest_roots(long long n, unsigned long long seed, unsigned long long *bad, cudaStream_t st) {
+    cl::k_selftest_roots<<<152 * 4, 256, 0, st>>>(n, seed, bad);
+}
+
 size_t mlp_bytes() { return sizeof(cl::Net); }
 int mlp_snapshot_device(const ark_mlp *M, void *dev_out) {
     if (!M || !dev_out) return ARK_ERR_PARAM;
