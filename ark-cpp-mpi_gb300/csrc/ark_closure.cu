@@ -22,6 +22,7 @@
 
 #include "../../include/ark_gpu.h"
 #include "ark_check.cuh"
+#include "ark_kernels.cuh" // qdiv
 #include "ark_state.h"
 
 namespace ark {
@@ -357,20 +358,32 @@ __device__ __forceinline__ void features_fp64(const double A[3][3], double y, do
 }
 
 // ---- dataset kernels ----------------------------------------------------------------------
-// All bound by the FP64 pipe (1/64 of the FP32 rate): sums of widened values, one multiply by 1/27
-// per box instead of a division per pass, FP32 starting values for the roots.
+// All bound by the FP64 pipe (1/64 of the FP32 rate): sums of widened values, one quotient by 27
+// per box on the integer pipes instead of a division per pass, FP32 starting values for the roots.
+
+// The mean x / 27 of a box from its sum, one rounding where three means of three had three each (the
+// product with RN(1/27), half an ulp from 1/27, was the less precise by a tenth on FP64 fields).  The
+// filter takes the quotient on the integer pipes (256x128x128, the whole call 505 us; on the FP64 pipe
+// 565), k_samples, whose gradients' products are there already, the product and its correction from the
+// exact remainder, within 0.5 + 2^-50 ulp (505; on the integer pipes 536).
+__device__ __forceinline__ double box_mean(double x, const QRecip &q27) { return qdiv(x, 27.0, 1.0 / 27.0, q27); }
+__device__ __forceinline__ double box_mean_fma(double x) {
+    const double q = __dmul_rn(x, 1.0 / 27.0);
+    return __fma_rn(__fma_rn(-27.0, q, x), 1.0 / 27.0, q);
+}
 
 // The velocities of level lvl of a channel (periodic x and z, solid walls in y: a neighbour beyond a
 // wall counts as minus the cell), box-filtered 3 x 3 x 3, into three compact interior arrays
 // ub + m * cells ([k][j][i], FP64).  A block takes 32 x FY cells of a plane and marches up kch planes:
 // the sums along x of FY + 2 rows go through shared memory (two planes' buffers in turn, one barrier
 // per plane), the sums over x and y of the last three planes stay in registers.  Seven FP64 sums
-// per value and a product on the integer pipes (mulq), against six and three divisions in three passes
-// over memory: 700 us (and 32 for a gathered FP64 copy) -> 229 at 256x128x128, 215 with mulq (16 rows per
-// block and three blocks per SM, with spills, the same).
+// per value and a quotient on the integer pipes (box_mean), against six and three divisions in three
+// passes over memory: 700 us (and 32 for a gathered FP64 copy) -> 215 at 256x128x128, the FP64 pipe 69%
+// busy (16 rows per block and three blocks per SM, with spills, the same).
 constexpr int FY = 8;
 template <class T>
-__global__ void __launch_bounds__(32 * (FY + 2), 4) k_filter_velocity(const __grid_constant__ DevState<T> S, int lvl, double *ub, int kch) {
+__global__ void __launch_bounds__(32 * (FY + 2), 4) k_filter_velocity(const __grid_constant__ DevState<T> S, int lvl, double *ub, int kch,
+                                                                      const __grid_constant__ QRecip q27) {
     __shared__ double xs[2][3][FY + 2][32];
     const Geom g = S.g;
     const int tx = threadIdx.x, ty = threadIdx.y;
@@ -402,7 +415,7 @@ __global__ void __launch_bounds__(32 * (FY + 2), 4) k_filter_velocity(const __gr
                 const double neg = __hiloint2double(__double2hiint(x[m]) ^ (int)0x80000000, __double2loint(x[m]));
                 const double lo = j == 1 ? neg : xs[buf][m][ty - 1][tx], hi = j == g.C2 ? neg : xs[buf][m][ty + 1][tx];
                 const double xy = (lo + x[m]) + hi;
-                if (p > k0) ub[m * cells + out] = mulq((z0[m] + z1[m]) + xy, 1.0 / 27.0);
+                if (p > k0) ub[m * cells + out] = box_mean((z0[m] + z1[m]) + xy, q27);
                 z0[m] = z1[m];
                 z1[m] = xy;
             }
@@ -440,8 +453,8 @@ struct SampleArgs {
 // products u_m u_n are needed at the samples only: a thread marches along jc rows of one (a, b), with
 // the nine cells' products of a row summed in x and z, and the sums of three rows in registers
 // (a row beyond a wall counts as the row itself).  Every product filtered everywhere took 18 passes
-// (1400 us) and 55 us of products; the samples of a 4 x 4 lattice 180 -> 165 with the products in them,
-// the FP64 pipe 83% busy (161 with the gradients' products on the integer pipes).
+// (1400 us) and 55 us of products; the samples of a 4 x 4 lattice take 177 us with the products in them, the
+// FP64 pipe 83% busy (before, 180 without them; the gradients' products on the integer pipes save 4).
 template <class T> __global__ void __launch_bounds__(128) k_samples(const __grid_constant__ DevState<T> S, int lvl, SampleArgs s) {
     const Geom g = S.g;
     const int C1 = g.C1, C2 = g.C2, C3 = g.C3;
@@ -492,7 +505,7 @@ template <class T> __global__ void __launch_bounds__(128) k_samples(const __grid
 #pragma unroll
         for (int n = 0; n < 6; ++n) {
             constexpr int p[6] = {0, 0, 0, 1, 1, 2}, q[6] = {0, 1, 2, 1, 2, 2};
-            tau[n] = ((lo[n] + mid[n]) + hi[n]) * (1.0 / 27.0) - v[p[n]] * v[q[n]];
+            tau[n] = box_mean_fma((lo[n] + mid[n]) + hi[n]) - v[p[n]] * v[q[n]];
             lo[n] = mid[n];
             mid[n] = hi[n];
         }
@@ -1282,7 +1295,7 @@ int closure_sample(const DevState<T> &S, int lvl, ark_closure_data *d, double lx
             kch = c;
         }
     }
-    cl::k_filter_velocity<T><<<dim3(bx, by, (C3 + kch - 1) / kch), dim3(32, cl::FY + 2), 0, st>>>(S, lvl, d->scratch, kch);
+    cl::k_filter_velocity<T><<<dim3(bx, by, (C3 + kch - 1) / kch), dim3(32, cl::FY + 2), 0, st>>>(S, lvl, d->scratch, kch, make_qrecip(27.0));
     cl::SampleArgs s;
     for (int m = 0; m < 3; ++m) s.ub[m] = d->scratch + m * cells;
     s.feat = d->feat;
