@@ -1156,8 +1156,6 @@ __device__ __forceinline__ FaceQ<T> face_q(const FaceVal<T> &V, int d, uint8_t f
 template <class T, int MODE, bool INT>
 __global__ void __launch_bounds__(SX *SY, 3) k_phase1_faces(const __grid_constant__ DevState<T> S, int src, int dst, int fcur, int kch) {
     static_assert(!Storage<T>::deviation, "face-centric Phase1: FP64 storage form");
-    grid_release();
-    grid_wait();
     constexpr bool STRESS = (MODE & P1_STRESS) != 0;
     // two generations of a plane's x and y face quantities (face_smem bytes), alternating by
     // plane: a thread may write plane k+1's while others still read plane k's, and the barrier
@@ -2618,7 +2616,7 @@ void Launch<T>::phase1(const DevState<T> &S, int src, int dst, int fcur, int mod
             const dim3 grid((S.g.C1 + fcs::SX - 1) / fcs::SX, (S.g.C2 + fcs::SY - 1) / fcs::SY, (S.g.C3 + kch - 1) / kch);
             const dim3 block(fcs::SX, fcs::SY);
             constexpr int A = P1_STRESS | P1_FORCES | P1_RMAX, B = A | P1_BULK, C = P1_FORCES | P1_RSUM;
-            auto go = [&](auto kernel) { launch_early(false, kernel, grid, block, fcs::face_smem<T>(), st, S, src, dst, fcur, kch); };
+            auto go = [&](auto kernel) { kernel<<<grid, block, fcs::face_smem<T>(), st>>>(S, src, dst, fcur, kch); };
             auto pick = [&](auto m) {
                 constexpr int M = decltype(m)::value;
                 if (int_products(S.g)) go(fcs::k_phase1_faces<T, M, true>);
