@@ -651,9 +651,10 @@ __device__ __forceinline__ void gelu_both(float z, float &h, float &d) {
 }
 
 // Training alternates two short kernels, each launched while the one before still runs (launch_early).
-// Before grid_wait a kernel reads only what the other does not write (the samples; the moments and
-// masters, which k_mlp_update alone writes).
-constexpr int kMaxRows = 608; // rows of block partials: at most four blocks per SM
+// Before grid_wait a kernel reads only the samples.  What the other one writes (the weights, the
+// partials) is written while this one is resident, so it is no constant of the kernel: no parameter is
+// const __restrict__, which would allow read-only loads, and those arrays are read from L2 (__ldcg).
+constexpr int kMaxRows = 608; // rows of block partials, so also the most blocks: two waves of two per SM
 
 struct GradSmem {
     unsigned f1[FR1][32], f2[FR2][32], f2t[FR2][32]; // the weights' B fragments, per lane
@@ -665,9 +666,9 @@ struct GradSmem {
 // Gradient of the mean squared error over samples [first, first + count) of the batch map
 // (sample index = (first + q) * stride + offset), into block partials part[block][NPARAM + 1]
 // (the last entry: the block's sum of squared errors).  scale = 2 / (samples of the batch).
-__global__ void __launch_bounds__(32 * GW, 2) k_mlp_grad(const float *__restrict__ feat, const float *__restrict__ targ,
+__global__ void __launch_bounds__(32 * GW, 2) k_mlp_grad(const float *feat, const float *targ,
                                                          long long first, long long count, long long stride, long long offset,
-                                                         const Net *__restrict__ net, float scale, float *part) {
+                                                         const Net *net, float scale, float *part) {
     extern __shared__ __align__(16) unsigned char grad_raw[];
     GradSmem &sm = *reinterpret_cast<GradSmem *>(grad_raw);
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, g = lane >> 2, t = lane & 3;
@@ -692,10 +693,10 @@ __global__ void __launch_bounds__(32 * GW, 2) k_mlp_grad(const float *__restrict
     grid_wait();
 #pragma unroll
     for (int q = 0; q < (NPARAM + 32 * GW - 1) / (32 * GW); ++q)
-        if (tid + q * 32 * GW < NPARAM) w[tid + q * 32 * GW] = net->w[tid + q * 32 * GW];
+        if (tid + q * 32 * GW < NPARAM) w[tid + q * 32 * GW] = __ldcg(net->w + tid + q * 32 * GW);
     if (tid < 16) {
-        sm.mu[tid] = tid < NIN ? net->mu[tid] : 0.f;
-        sm.rsd[tid] = tid < NIN ? net->rsd[tid] : 0.f;
+        sm.mu[tid] = tid < NIN ? __ldcg(net->mu + tid) : 0.f;
+        sm.rsd[tid] = tid < NIN ? __ldcg(net->rsd + tid) : 0.f;
     }
     __syncthreads();
     for (int f = wid; f < FR1 + 2 * FR2; f += GW) {
@@ -905,18 +906,18 @@ struct Adam {
 // (the network's working weights are the BF16 roundings of its masters) and the batch's error added
 // to *A.loss.  One thread per parameter loading as it added 512 partials, and two more launches for
 // the step and the loss, took 22.7 + 3.7 + 2.8 us, this 7 (a batch of 65536: 68 -> 26.6 us in all).
-__global__ void __launch_bounds__(512) k_mlp_update(const float *__restrict__ part, int nblocks, float *grad, const Adam A) {
+__global__ void __launch_bounds__(512) k_mlp_update(const float *part, int nblocks, float *grad, const Adam A) {
     extern __shared__ float rows[]; // [nblocks][32]
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, p = blockIdx.x * 32 + lane;
     const bool step = wid == 0 && p < NPARAM && A.master;
-    const float m0 = step ? __ldcg(A.m + p) : 0.f, v0 = step ? __ldcg(A.v + p) : 0.f, x0 = step ? __ldcg(A.master + p) : 0.f;
     const float c1 = 1.f - powf(A.beta1, (float)A.step), c2 = 1.f - powf(A.beta2, (float)A.step);
     grid_wait();
+    const float m0 = step ? __ldcg(A.m + p) : 0.f, v0 = step ? __ldcg(A.v + p) : 0.f, x0 = step ? __ldcg(A.master + p) : 0.f;
     if (p <= NPARAM) {
 #pragma unroll
         for (int q = 0; q < kMaxRows / 16; ++q) {
             const int b = wid + 16 * q;
-            if (b < nblocks) rows[32 * b + lane] = part[(size_t)b * (NPARAM + 1) + p];
+            if (b < nblocks) rows[32 * b + lane] = __ldcg(part + (size_t)b * (NPARAM + 1) + p);
         }
     }
     grid_release();

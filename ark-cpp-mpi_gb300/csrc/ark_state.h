@@ -464,7 +464,8 @@ constexpr int kStatWarps = 8;
 // Kernels launched while the one before still runs (programmatic stream serialization, launch_early):
 // grid_release lets the next grid of the stream start once every block of this one has come to it,
 // grid_wait waits for the grids before to have ended with their writes visible.  A kernel launched so
-// touches no global memory that the others write, and writes none, before grid_wait; in a kernel
+// touches no global memory that the others write, and writes none, before grid_wait, and has no
+// const __restrict__ parameter (what it points to changes while the kernel is resident); in a kernel
 // launched the ordinary way both do nothing that matters.  Taken by the
 // FP32 steps of small grids (early_grid), whose kernels fit the SMs at once: 32x32x32 20.5 -> 18.9 us
 // per step, 64x48x48 27.8 -> 26.6.  The blocks of a larger next grid, waiting in slots as they come
