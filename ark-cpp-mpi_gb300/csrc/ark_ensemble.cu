@@ -208,7 +208,7 @@ __global__ void __launch_bounds__(128) kb_sweep_x(const DS *__restrict__ inst, W
     __shared__ int slot;
     for (int b = next_item(next, slot); b < W.total; b = next_item(next, slot)) {
         const int q = find_member(W, b);
-        sweep_x_body<float>(inst[q], con, fcur, W.extra[q], decode(W, q, b));
+        sweep_x_body<float, false>(inst[q], con, fcur, W.extra[q], decode(W, q, b));
     }
 }
 
@@ -217,7 +217,7 @@ __global__ void __launch_bounds__(128, 5) kb_sweep_col(const DS *__restrict__ in
     __shared__ int slot;
     for (int b = next_item(next, slot); b < W.total; b = next_item(next, slot)) {
         const int q = find_member(W, b);
-        sweep_col_body<float, AX>(inst[q], con, fcur, W.extra[q], decode(W, q, b));
+        sweep_col_body<float, AX, false>(inst[q], con, fcur, W.extra[q], decode(W, q, b));
     }
 }
 
@@ -243,7 +243,7 @@ __global__ void __launch_bounds__(128, 5) kb_sweep_z_seams(const DS *__restrict_
         const int kch = W.extra[q], C3 = inst[q].g.C3, nch = (C3 + kch - 1) / kch;
         BIx bx = decode(W, q, b);
         bx.z = bx.z < nch ? bx.z * kch : C3;
-        sweep_col_body<float, 2>(inst[q], con, fcur, 1, bx);
+        sweep_col_body<float, 2, false>(inst[q], con, fcur, 1, bx);
     }
 }
 

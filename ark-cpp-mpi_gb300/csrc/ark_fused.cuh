@@ -354,7 +354,7 @@ __global__ void __launch_bounds__(NT, 2)
                 ea.qb = ez.qb;
                 ea.ab = ez.ab;
                 ea.bb = ez.bb;
-                const FaceNew<T> v = face_values<T, false>(NCZ, g.ci(i, j, p - 1), g.ci(i, j, p), (uint8_t)zb.fl, fl, zb.un,
+                const FaceNew<T> v = face_values<T, false, false>(NCZ, g.ci(i, j, p - 1), g.ci(i, j, p), (uint8_t)zb.fl, fl, zb.un,
                                                            un, eb, ea, zlo[1], zlo[2], qz);
                 if (p <= k1 || p == g.C3 + 1) face_store(WZ, g.fi(i, j, p), v);
                 zn[0] = v.p;
@@ -488,7 +488,7 @@ __global__ void __launch_bounds__(NT, 2)
                 ea.qb = ex.qb;
                 ea.ab = ex.ab;
                 ea.bb = ex.bb;
-                const FaceNew<T> v = face_values<T, false>(NCX, g.ci(i - 1, j, p), g.ci(i, j, p), (uint8_t)b.fl, fl, b.un,
+                const FaceNew<T> v = face_values<T, false, false>(NCX, g.ci(i - 1, j, p), g.ci(i, j, p), (uint8_t)b.fl, fl, b.un,
                                                            unx, eb, ea, st[off_fx(2, ty, x)], st[off_fx(3, ty, x)], qx);
                 face_store(WX, g.fi(i, j, p), v);
                 nfx[0] = v.p;
@@ -505,7 +505,7 @@ __global__ void __launch_bounds__(NT, 2)
                     ea2.qb = a.qb;
                     ea2.ab = a.ab;
                     ea2.bb = a.bb;
-                    const FaceNew<T> w = face_values<T, false>(NCX, g.ci(i, j, p), g.ci(i + 1, j, p), fl, (uint8_t)a.fl,
+                    const FaceNew<T> w = face_values<T, false, false>(NCX, g.ci(i, j, p), g.ci(i + 1, j, p), fl, (uint8_t)a.fl,
                                                                unx, a.un, eb2, ea2, st[off_fx(2, ty, x + 1)],
                                                                st[off_fx(3, ty, x + 1)], qx);
                     if (i == g.C1) face_store(WX, g.fi(i + 1, j, p), w);
@@ -521,7 +521,7 @@ __global__ void __launch_bounds__(NT, 2)
                 ea.qb = ey.qb;
                 ea.ab = ey.ab;
                 ea.bb = ey.bb;
-                const FaceNew<T> v = face_values<T, true>(NCY, g.ci(i, j - 1, p), g.ci(i, j, p), (uint8_t)b.fl, fl, b.un,
+                const FaceNew<T> v = face_values<T, true, false>(NCY, g.ci(i, j - 1, p), g.ci(i, j, p), (uint8_t)b.fl, fl, b.un,
                                                           uny, eb, ea, st[off_fy(1, r, x)], st[off_fy(3, r, x)], qy);
                 face_store(WY, g.fi(i, j, p), v);
                 nfy[0] = v.p;
@@ -538,7 +538,7 @@ __global__ void __launch_bounds__(NT, 2)
                     ea2.qb = a.qb;
                     ea2.ab = a.ab;
                     ea2.bb = a.bb;
-                    const FaceNew<T> w = face_values<T, true>(NCY, g.ci(i, j, p), g.ci(i, j + 1, p), fl, (uint8_t)a.fl,
+                    const FaceNew<T> w = face_values<T, true, false>(NCY, g.ci(i, j, p), g.ci(i, j + 1, p), fl, (uint8_t)a.fl,
                                                               uny, a.un, eb2, ea2, st[off_fy(1, r + 1, x)],
                                                               st[off_fy(3, r + 1, x)], qy);
                     if (j == g.C2) face_store(WY, g.fi(i, j + 1, p), w);

@@ -1450,7 +1450,7 @@ template <class T> __device__ __forceinline__ RQ<T> face_rq(T u_n, T p, const Sw
 
 // The extrapolation with the invariants of the forward (f) and backward (b) face given.  INT: FP64 products on the integer
 // pipes (mulq).
-template <class T, bool Q_USES_R, bool INT = true>
+template <class T, bool Q_USES_R, bool INT>
 __device__ __forceinline__ Ext<T> extrapolate_rq(RQ<T> f, RQ<T> b, T u1_cn, T u1_c, T u2_f, T u2_b, T u2_cn, T u2_c,
                                                  T u3_f, T u3_b, T u3_cn, T u3_c, T ro_cn, T ro_c, const SweepK<T> &q) {
     constexpr bool DEV = Storage<T>::deviation;
@@ -1506,7 +1506,7 @@ template <class T, bool Q_USES_R>
 __device__ __forceinline__ Ext<T> extrapolate(T u1_f, T u1_b, T u1_cn, T u1_c, T u2_f, T u2_b, T u2_cn,
                                               T u2_c, T u3_f, T u3_b, T u3_cn, T u3_c, T ro_cn, T ro_c,
                                               T p_f, T p_b, const SweepK<T> &q) {
-    return extrapolate_rq<T, Q_USES_R>(face_rq(u1_f, p_f, q), face_rq(u1_b, p_b, q), u1_cn, u1_c, u2_f, u2_b, u2_cn,
+    return extrapolate_rq<T, Q_USES_R, false>(face_rq(u1_f, p_f, q), face_rq(u1_b, p_b, q), u1_cn, u1_c, u2_f, u2_b, u2_cn,
                                        u2_c, u3_f, u3_b, u3_cn, u3_c, ro_cn, ro_c, q);
 }
 
@@ -1554,7 +1554,7 @@ template <class T> struct NVals {
 // their flags and ucb/ucf their half-step normal velocities.  uA_old/uB_old: the face's
 // previous tangential velocities.  WALL_A_FROM_N: the x2 sweep takes the tangential u1 from
 // u2nCon in its wall branches (main.cpp:2219, 2238).
-template <class T, bool WALL_A_FROM_N, bool INT = true, class NV>
+template <class T, bool WALL_A_FROM_N, bool INT, class NV>
 __device__ __forceinline__ FaceNew<T> face_values_v(const NV &V, uint8_t flb, uint8_t flf, T ucb, T ucf, const Ext<T> &prev,
                                                     const Ext<T> &cur, T uA_old, T uB_old, const SweepK<T> &q) {
     constexpr bool DEV = Storage<T>::deviation;
@@ -1636,7 +1636,7 @@ __device__ __forceinline__ FaceNew<T> face_values_v(const NV &V, uint8_t flb, ui
     return v;
 }
 // cb / cf index the cells behind and ahead in the half-step level N
-template <class T, bool WALL_A_FROM_N, bool INT = true>
+template <class T, bool WALL_A_FROM_N, bool INT>
 __device__ __forceinline__ FaceNew<T> face_values(const NCell<T> &N, int cb, int cf, uint8_t flb, uint8_t flf, T ucb,
                                                   T ucf, const Ext<T> &prev, const Ext<T> &cur, T uA_old, T uB_old,
                                                   const SweepK<T> &q) {
@@ -1652,7 +1652,7 @@ template <class T> __device__ __forceinline__ void face_store(const FaceOut<T> &
 }
 
 // face_values stored into the new face generation at face fc
-template <class T, bool WALL_A_FROM_N, bool INT = true>
+template <class T, bool WALL_A_FROM_N, bool INT>
 __device__ __forceinline__ void face_update(const NCell<T> &N, const FaceOut<T> &W, int cb, int cf, int fc,
                                             uint8_t flb, uint8_t flf, T ucb, T ucf, const Ext<T> &prev,
                                             const Ext<T> &cur, T uA_old, T uB_old, const SweepK<T> &q) {
@@ -1774,7 +1774,7 @@ __device__ __forceinline__ int zface(int s, int C3, bool periodic) {
 // neighbouring lane, or the carry from the previous chunk's last lane.  Old faces come from
 // generation fcur, new faces go to fcur^1.
 
-template <class T, bool INT = true>
+template <class T, bool INT>
 __device__ __forceinline__ void sweep_x_body(const DevState<T> &S, int con, int fcur, int glines, const BIx &bx, int nch = 0) {
     const Geom g = S.g;
     const int lane = threadIdx.x & 31;
@@ -1914,10 +1914,10 @@ __device__ __forceinline__ void sweep_x_body(const DevState<T> &S, int con, int 
     }
 }
 
-template <class T>
+template <class T, bool INT>
 __global__ void __launch_bounds__(128, sizeof(T) == 4 ? 6 : 3)
     k_sweep_x(const __grid_constant__ DevState<T> S, int con, int fcur, int glines, int nch) {
-    sweep_x_body<T>(S, con, fcur, glines, bix_here(), nch);
+    sweep_x_body<T, INT>(S, con, fcur, glines, bix_here(), nch);
 }
 
 // The x faces that Phase1 + stress with the x1 sweep folded in leaves (stg::phase1_tma_body
@@ -1961,7 +1961,7 @@ __device__ __forceinline__ void sweep_x_seams_body(const DevState<T> &S, int con
             const bool lo = b == 0; // ghost position 0 (cell C1; faces 1 ahead, C1 behind) or C1 + 1
             const int c = ARK_CK(c0 + (lo ? g.C1 : 1), R.nc);
             const int ff = ARK_CK(f0 + (lo ? 1 : 2), R.nf), fb = ARK_CK(f0 + (lo ? g.C1 : g.C1 + 1), R.nf);
-            const Ext<T> e = extrapolate_rq<T, true>(face_rq(R.FN[ff], R.FP[ff], q), face_rq(R.FN[fb], R.FP[fb], q), R.nN[c],
+            const Ext<T> e = extrapolate_rq<T, true, false>(face_rq(R.FN[ff], R.FP[ff], q), face_rq(R.FN[fb], R.FP[fb], q), R.nN[c],
                                                      R.cN[c], R.FA[ff], R.FA[fb], R.nA[c], R.cA[c], R.FB[ff], R.FB[fb], R.nB[c],
                                                      R.cB[c], R.nR[c], R.cR[c], q);
             if (lo) {
@@ -1986,7 +1986,7 @@ __device__ __forceinline__ void sweep_x_seams_body(const DevState<T> &S, int con
     const uint8_t flb = (uint8_t)__float_as_int(X.b[7][w]), flf = (uint8_t)__float_as_int(X.a[7][w]);
     const FaceOut<T> W = sweep_out(S, fcur, 0);
     face_store(W, ARK_CK(g.fi(s, j, k), W.nf),
-               face_values_v<T, false>(V, flb, flf, X.b[3][wb], X.a[3][wa], prev, cur, X.a[8][w], X.a[9][w], q));
+               face_values_v<T, false, false>(V, flb, flf, X.b[3][wb], X.a[3][wa], prev, cur, X.a[8][w], X.a[9][w], q));
 }
 template <class T>
 __global__ void __launch_bounds__(256) k_sweep_x_seams(const __grid_constant__ DevState<T> S, int con, int fcur,
@@ -2005,7 +2005,7 @@ __global__ void __launch_bounds__(256) k_sweep_x_seams(const __grid_constant__ D
 __host__ __device__ inline int col_sweep_blocks(const Geom &g, int axis) {
     return (((g.C1 + 31) >> 5) * (axis == 1 ? g.C3 : g.C2) + 3) >> 2;
 }
-template <class T, int AX, bool INT = true>
+template <class T, int AX, bool INT>
 __device__ __forceinline__ void sweep_col_body(const DevState<T> &S, int con, int fcur, int seg, const BIx &bx) {
     const Geom g = S.g;
     const int nic = (g.C1 + 31) >> 5;
@@ -2056,9 +2056,9 @@ __device__ __forceinline__ void sweep_col_body(const DevState<T> &S, int con, in
     }
 }
 
-template <class T, int AX>
+template <class T, int AX, bool INT>
 __global__ void __launch_bounds__(128) k_sweep_col(const __grid_constant__ DevState<T> S, int con, int fcur, int seg) {
-    sweep_col_body<T, AX>(S, con, fcur, seg, bix_here());
+    sweep_col_body<T, AX, INT>(S, con, fcur, seg, bix_here());
 }
 
 // The z faces that Phase1 + stress with the x3 sweep folded in leaves (stg::phase1_tma_body with
@@ -2070,7 +2070,7 @@ __global__ void __launch_bounds__(128) k_sweep_z_seams(const __grid_constant__ D
     BIx bx = bix_here();
     const int nch = (S.g.C3 + kch - 1) / kch;
     bx.z = (int)blockIdx.z < nch ? (int)blockIdx.z * kch : S.g.C3;
-    sweep_col_body<T, 2>(S, con, fcur, 1, bx);
+    sweep_col_body<T, 2, false>(S, con, fcur, 1, bx);
 }
 
 // What is left of a small grid's Phase2 after Phase1 + stress with the x1 (and x3) sweeps folded in, in one
@@ -2092,7 +2092,7 @@ __global__ void __launch_bounds__(128, 9) k_sweep_y_seams(const __grid_constant_
     if (b >= 0 && b < ny) {
         bx.z = b / yc;
         bx.x = b - bx.z * yc;
-        sweep_col_body<T, 1>(S, con, fcur, seg, bx);
+        sweep_col_body<T, 1, false>(S, con, fcur, seg, bx);
         return;
     }
     b = first ? (int)blockIdx.x : b - ny; // x seams, then z seams
@@ -2103,7 +2103,7 @@ __global__ void __launch_bounds__(128, 9) k_sweep_y_seams(const __grid_constant_
         const int p = b / zc, nch = (S.g.C3 + X.kch - 1) / X.kch;
         bx.x = b - p * zc;
         bx.z = p < nch ? p * X.kch : S.g.C3;
-        sweep_col_body<T, 2>(S, con, fcur, 1, bx);
+        sweep_col_body<T, 2, false>(S, con, fcur, 1, bx);
     }
 }
 
@@ -2228,27 +2228,27 @@ __global__ void __launch_bounds__(SX *SY, 2) k_phase2_fused(const __grid_constan
             const int c = g.ci(i, j, k), f = g.fi(i, j, k);
             {   // x faces i (and C1 + 1)
                 const CellExt<T> &b = EX[ty][tx], &a = EX[ty][tx + 1];
-                face_update<T, false>(NX, WX, c - 1, c, f, b.fl, a.fl, b.un, a.un, b.e, a.e, RX.FA[f], RX.FB[f], qx);
+                face_update<T, false, false>(NX, WX, c - 1, c, f, b.fl, a.fl, b.un, a.un, b.e, a.e, RX.FA[f], RX.FB[f], qx);
                 if (i == g.C1) {
                     const CellExt<T> &z = EX[ty][tx + 2];
-                    face_update<T, false>(NX, WX, c, c + 1, f + 1, a.fl, z.fl, a.un, z.un, a.e, z.e, RX.FA[f + 1],
+                    face_update<T, false, false>(NX, WX, c, c + 1, f + 1, a.fl, z.fl, a.un, z.un, a.e, z.e, RX.FA[f + 1],
                                           RX.FB[f + 1], qx);
                 }
             }
             {   // y faces j (and C2 + 1)
                 const CellExt<T> &b = EY[ty][tx], &a = EY[ty + 1][tx];
-                face_update<T, true>(NY, WY, c - cs1, c, f, b.fl, a.fl, b.un, a.un, b.e, a.e, RY.FA[f], RY.FB[f], qy);
+                face_update<T, true, false>(NY, WY, c - cs1, c, f, b.fl, a.fl, b.un, a.un, b.e, a.e, RY.FA[f], RY.FB[f], qy);
                 if (j == g.C2) {
                     const CellExt<T> &z = EY[ty + 2][tx];
-                    face_update<T, true>(NY, WY, c, c + cs1, f + fs1, a.fl, z.fl, a.un, z.un, a.e, z.e, RY.FA[f + fs1],
+                    face_update<T, true, false>(NY, WY, c, c + cs1, f + fs1, a.fl, z.fl, a.un, z.un, a.e, z.e, RY.FA[f + fs1],
                                          RY.FB[f + fs1], qy);
                 }
             }
             // z faces k (and C3 + 1)
-            face_update<T, false>(NZ, WZ, c - cs2, c, f, zlo.fl, zc.fl, zlo.un, zc.un, zlo.e, zc.e, RZ.FA[f], RZ.FB[f], qz);
+            face_update<T, false, false>(NZ, WZ, c - cs2, c, f, zlo.fl, zc.fl, zlo.un, zc.un, zlo.e, zc.e, RZ.FA[f], RZ.FB[f], qz);
             if (k == g.C3) {
                 const CellExt<T> zg = cell_ext<T, 2>(RZ, qz, c + cs2, f + fs2, fs2);
-                face_update<T, false>(NZ, WZ, c, c + cs2, f + fs2, zc.fl, zg.fl, zc.un, zg.un, zc.e, zg.e, RZ.FA[f + fs2],
+                face_update<T, false, false>(NZ, WZ, c, c + cs2, f + fs2, zc.fl, zg.fl, zc.un, zg.un, zc.e, zg.e, RZ.FA[f + fs2],
                                       RZ.FB[f + fs2], qz);
             }
         }
@@ -2792,22 +2792,27 @@ template <class T> void Launch<T>::use_forces(const DevState<T> &S, int ncon, cu
 
 template <class T>
 void Launch<T>::sweep(const DevState<T> &S, int con, int fcur, int axis, cudaStream_t st, int target, int xlines) {
+    constexpr bool fp64 = sizeof(T) == 8;
+    const bool ints = fp64 && int_products(S.g);
     if (axis == 0) {
-        const int lines_x = S.g.C2 * S.g.C3, gl = xlines > 0 ? xlines : x_lines_per_warp(S.g, sizeof(T) == 8);
-        const int nch = xlines > 0 ? 0 : x_chunks_per_warp(S.g, gl, sizeof(T) == 8);
+        const int lines_x = S.g.C2 * S.g.C3, gl = xlines > 0 ? xlines : x_lines_per_warp(S.g, fp64);
+        const int nch = xlines > 0 ? 0 : x_chunks_per_warp(S.g, gl, fp64);
         // 4 warps of nch chunks, or of gl lines
         const dim3 grid(nch ? x_chunk_blocks(S.g, nch) : (lines_x + 4 * gl - 1) / (4 * gl));
-        k_sweep_x<T><<<grid, 128, 0, st>>>(S, con, fcur, gl, nch);
+        if (ints) k_sweep_x<T, fp64><<<grid, 128, 0, st>>>(S, con, fcur, gl, nch);
+        else k_sweep_x<T, false><<<grid, 128, 0, st>>>(S, con, fcur, gl, nch);
     } else if (axis == 1) {
         int nseg;
-        const int seg = sweep_segment(S.g.C2 + 1, target, col_sweep_blocks(S.g, 1), sizeof(T) == 8, &nseg);
+        const int seg = sweep_segment(S.g.C2 + 1, target, col_sweep_blocks(S.g, 1), fp64, &nseg);
         const dim3 grid(col_sweep_blocks(S.g, 1), 1, nseg);
-        k_sweep_col<T, 1><<<grid, 128, 0, st>>>(S, con, fcur, seg);
+        if (ints) k_sweep_col<T, 1, fp64><<<grid, 128, 0, st>>>(S, con, fcur, seg);
+        else k_sweep_col<T, 1, false><<<grid, 128, 0, st>>>(S, con, fcur, seg);
     } else {
         int nseg;
-        const int seg = sweep_segment(S.g.C3 + 1, target, col_sweep_blocks(S.g, 2), sizeof(T) == 8, &nseg);
+        const int seg = sweep_segment(S.g.C3 + 1, target, col_sweep_blocks(S.g, 2), fp64, &nseg);
         const dim3 grid(col_sweep_blocks(S.g, 2), 1, nseg);
-        k_sweep_col<T, 2><<<grid, 128, 0, st>>>(S, con, fcur, seg);
+        if (ints) k_sweep_col<T, 2, fp64><<<grid, 128, 0, st>>>(S, con, fcur, seg);
+        else k_sweep_col<T, 2, false><<<grid, 128, 0, st>>>(S, con, fcur, seg);
     }
 }
 

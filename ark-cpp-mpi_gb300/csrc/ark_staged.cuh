@@ -804,7 +804,7 @@ __device__ __forceinline__ void phase1_tma_body(const DevState<float> &S, const 
                         nv.b[1] = xc.un[1];
                         nv.r[1] = xc.ro_n;
                         face_store(WZ, ARK_CK(g.fi(i, j, k), WZ.nf),
-                                   face_values_v<T, false>(nv, zfl, xc.fl, zun, xc.un[2], zprev, ez, Z(fm, 1), Z(fm, 2), qz));
+                                   face_values_v<T, false, false>(nv, zfl, xc.fl, zun, xc.un[2], zprev, ez, Z(fm, 1), Z(fm, 2), qz));
                     }
                     zprev = ez;
                     zun = xc.un[2];
@@ -879,7 +879,7 @@ __device__ __forceinline__ void phase1_tma_body(const DevState<float> &S, const 
                 }
                 if (valid && tx != 0) // the face below the cell (main.cpp:1920-2008)
                     face_store(WX, ARK_CK(g.fi(i, j, k), WX.nf),
-                               face_values_v<T, false>(nv, (uint8_t)flb, xc.fl, ucb, xc.un[0], pv, e, uAo, uBo, qx));
+                               face_values_v<T, false, false>(nv, (uint8_t)flb, xc.fl, ucb, xc.un[0], pv, e, uAo, uBo, qx));
                 const bool px = S.k.periodic_x;
                 const uint8_t *flm = sk;
                 if (valid && tx == 0) { // the tile's seam b = bx.x: the cell ahead of its face
