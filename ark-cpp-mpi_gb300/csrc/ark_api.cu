@@ -1030,8 +1030,11 @@ static int ensure_graph(ark_ctx *ctx) {
 // about 3 us, which a step of a small grid is not much longer than (us per step, one step to a graph and
 // eight: FP32 32x32x32 20.5 -> 17.3, 64x48x48 27.3 -> 24.2, with the closure 39.2 -> 34.4, 128x64x64 53.1 ->
 // 49.5; FP64 64x32x32 91.3 -> 88.6, 200x60x1 47.2 -> 44.2).  An even count, so that a graph begins and
-// ends with the same face generation; long runs only (the capture takes as long as the gaps of about a
-// hundred steps), on grids whose step takes up to about a hundred of those gaps.
+// ends with the same face generation; runs of 64 steps on, which pay for the capture at once (a context's
+// first run of 64 after its single-step graphs exist, wall us: FP32 32x32x32 1,202 with those, 1,205 so,
+// 64x48x48 1,722 and 1,670, FP64 64x32x32 5,693 and 5,594, 200x60x1 3,104 and 2,985; of 100: 1,866 and
+// 1,816, 2,680 and 2,540, 8,896 and 8,687, 4,838 and 4,608), on grids whose step takes up to about a hundred
+// of those gaps.
 constexpr int kChain = 8, kChainFrom = 64;
 static bool chains(ark_ctx *ctx, int nsteps) {
     return (nsteps >= kChainFrom || (nsteps >= kChain && ctx->chain[ctx->con][ctx->fcur])) && !ctx->eng->rotates() &&
