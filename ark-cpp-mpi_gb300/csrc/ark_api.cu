@@ -1261,7 +1261,7 @@ int ark_selftest_division(long long n, unsigned long long seed, long long *misma
     ARK_CUDA(cudaMalloc(&bad, sizeof(unsigned long long)));
     cudaMemset(bad, 0, sizeof(unsigned long long));
     const int rc = selftest_division(n, seed, bad, 0);
-    selftest_roots(n, seed, bad, 0);
+    selftest_closure(n, seed, bad, 0);
     cudaError_t e = cudaGetLastError();
     if (rc && e == cudaSuccess) e = cudaErrorMemoryAllocation;
     unsigned long long h = 0;

@@ -277,7 +277,7 @@ __device__ __forceinline__ void features_of(const R A[3][3], R y, R ly, R yplus_
 // integer instructions) and two Newton steps in FP64 with the FP32 slope.  The first leaves an error
 // near 2^-46, the second the rounding of its last operation (root3: and a third of an ulp for the cube's
 // square): the square root within 0.501 ulp, the cube root within 1 ulp, the bounds of the FP64 sqrt and
-// cbrt (selftest_roots compares).  Values outside FP32's comfortable range take those, as a call.
+// cbrt (k_selftest_closure compares).  Values outside FP32's comfortable range take those, as a call.
 static __device__ __noinline__ double sqrt_call(double x) { return sqrt(x); }
 static __device__ __noinline__ double cbrt_call(double x) { return cbrt(x); }
 __device__ __forceinline__ float to_float24(double x) { // x in [2^-100, 2^100)
@@ -560,8 +560,9 @@ __global__ void __launch_bounds__(256) k_plane_stats_compact(const double *u0, c
 // take themselves on both sides; exact squares and cubes), their errors from FP64 residuals: x - y^2 is
 // one exact FMA, x - y^3 comes from the two-term cube.  Counts square roots off by more than 0.501 ulp,
 // cube roots by more than 1 ulp (the bounds of sqrt and cbrt), and zeros, infinities and NaN that do not
-// come back as they are.
-__global__ void k_selftest_roots(long long n, unsigned long long seed, unsigned long long *bad) {
+// come back as they are.  Also narrow against the conversion: any bits, and values about FP32's range
+// with halves of the last place and their neighbours (results that are subnormal or overflow included).
+__global__ void k_selftest_closure(long long n, unsigned long long seed, unsigned long long *bad) {
     unsigned long long local = 0;
     auto ulp = [](double y) { return __longlong_as_double((__double_as_longlong(y) & 0x7FF0000000000000ll) - (52ll << 52)); };
     for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < n; t += (long long)gridDim.x * blockDim.x) {
@@ -579,6 +580,15 @@ __global__ void k_selftest_roots(long long n, unsigned long long seed, unsigned 
         const double w = root3(x), s = __dmul_rn(w, w), ds = __fma_rn(w, w, -s), c = __dmul_rn(s, w);
         const double dc = __dadd_rn(__fma_rn(s, w, -c), __dmul_rn(ds, w)), r3 = __dadd_rn(__dadd_rn(x, -c), -dc);
         if (!(fabs(r3) <= ulp(w) * (3.0 * s)) || ((t & 15) == 11 && w != m)) ++local;
+        unsigned long long v = z * 0xD1342543DE82EF95ull + 1;
+        v ^= v >> 29;
+        if (t & 1) {
+            v = (v & 0x800FFFFFFFFFFFFFull) | ((unsigned long long)(870 + (z >> 40) % 284) << 52);
+            if (t & 2) v = (v & ~0x1FFFFFFFull) | (0x10000000ull + (z >> 20) % 3 - 1);
+        }
+        const double d = __longlong_as_double((long long)v);
+        const float want = (float)d, got = narrow(d);
+        if (__float_as_uint(want) != __float_as_uint(got) && (want == want || got == got)) ++local;
     }
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         const double inf = __longlong_as_double(0x7FF0000000000000ll), nan = __longlong_as_double(0x7FF8000000000000ll);
@@ -1579,8 +1589,8 @@ int ark_mlp_predict(ark_mlp *M, ark_closure_data *d, long long first, long long 
 // the network constants, for ark_api.cu's closure step
 namespace ark {
 const void *mlp_device_net(const ark_mlp *M) { return M ? (const void *)M->net : nullptr; }
-void selftest_roots(long long n, unsigned long long seed, unsigned long long *bad, cudaStream_t st) {
-    cl::k_selftest_roots<<<152 * 4, 256, 0, st>>>(n, seed, bad);
+void selftest_closure(long long n, unsigned long long seed, unsigned long long *bad, cudaStream_t st) {
+    cl::k_selftest_closure<<<152 * 4, 256, 0, st>>>(n, seed, bad);
 }
 
 size_t mlp_bytes() { return sizeof(cl::Net); }

@@ -21,7 +21,9 @@ template void rows_face_density<double>(double *, const double *, int, int64_t, 
 // host (powers of two, the significands 2^52 + 1 and 2^53 - 1, the channel's constants, random
 // values), where the device's own make_qrecip must also agree with the host's, and qrecip_var
 // (the per-cell divisor's reciprocal) with make_qrecip; qdiv2 against the division of 2a, and
-// dhalf against a / 2, and the integer fixed-point image (fixed32) against its FP64 form.
+// dhalf against a / 2, and the integer fixed-point image (fixed32) against its FP64 form.  The integer
+// product (mulq) against the multiply, and a float's widening by integers (widen) against the
+// conversion, on operands of their own (product_operand, t & 3 the kind).
 __device__ __forceinline__ unsigned long long mix64(unsigned long long z) {
     z += 0x9E3779B97F4A7C15ull;
     z = (z ^ (z >> 30)) * 0xBF58476D1CE4E5B9ull;
@@ -40,6 +42,24 @@ struct QCase {
     QRecip q;
 };
 __device__ __forceinline__ bool same(double x, double y) { return __double_as_longlong(x) == __double_as_longlong(y); }
+__device__ __forceinline__ bool same_or_nan(double x, double y) { return same(x, y) || (x != x && y != y); }
+// A product's operand from random bits z and r: any bits; short significands (products that are ties of the
+// rounding, or exact); ordinary exponents, one operand in two with a long run of ones; and exponents at the
+// edges of what mulq takes (2^-511 .. 2^512), zero, subnormal and non-finite ones among them.
+__device__ __forceinline__ double product_operand(unsigned long long z, unsigned long long r, int kind) {
+    constexpr unsigned long long SM = 0x800FFFFFFFFFFFFFull;
+    const int edge[10] = {0, 1, 511, 512, 513, 1534, 1535, 1536, 2046, 2047};
+    if (kind == 1) {
+        z &= ~((1ull << (r % 53)) - 1);
+        if (r & 0x10000) z = (z & SM) | ((983 + (r >> 20) % 81) << 52);
+    } else if (kind == 2) {
+        z = (z & SM) | ((983 + r % 81) << 52) | ((r & 0x10000) ? 0x000FFFFFFFFFFF00ull : 0ull);
+    } else if (kind == 3) {
+        z = (z & SM) | ((unsigned long long)edge[r % 10] << 52);
+        if ((r & 0x30000) == 0) z &= 0xFFF0000000000000ull; // powers of two, zeros, infinities
+    }
+    return __longlong_as_double((long long)z);
+}
 __global__ void k_selftest_division(long long n, unsigned long long seed, const QCase *qc, int nqc,
                                     unsigned long long *bad) {
     unsigned long long local = 0;
@@ -79,6 +99,21 @@ __global__ void k_selftest_division(long long n, unsigned long long seed, const 
         // a numerator with the divisor's significand bits: exact and near-exact quotients
         const double a3 = c.b * (double)(long long)(t % 4097 - 2048) * ((t & 4) ? 0.75 : 1.0);
         if (!same(a3 / c.b, qdiv(a3, c.b, 1.0 / c.b, c.q))) ++local;
+        const int kind = (int)(t & 3);
+        const unsigned long long zx = mix64(~seed + 4 * (unsigned long long)t), zy = mix64(zx), rx = mix64(zy), ry = mix64(rx);
+        const double x = product_operand(zx, rx, kind), y = product_operand(zy, ry, kind);
+        if (!same_or_nan(x * y, mulq(x, y))) ++local;
+        // a product's exponent at the ends of the normal range: y's chosen for it
+        const int ex = 512 + (int)(rx % 1024), sum = ((ry & 1) ? 2040 : -4) + (int)((ry >> 1) % 10), ey = sum + 1023 - ex;
+        if (ey > 0 && ey < 2047) {
+            const double u = __longlong_as_double((long long)((zx & 0x800FFFFFFFFFFFFFull) | ((unsigned long long)ex << 52)));
+            const double v = __longlong_as_double((long long)((zy & 0x800FFFFFFFFFFFFFull) | ((unsigned long long)ey << 52)));
+            if (!same_or_nan(u * v, mulq(u, v))) ++local;
+        }
+        // every exponent of a float alike, subnormals, infinities and NaN included
+        const float f2 = __uint_as_float((unsigned)zx), f3 = __uint_as_float(((unsigned)zy & 0x807FFFFFu) | ((kind & 1) ? 0u : 0x7F800000u));
+        const float f4 = __uint_as_float((unsigned)zx & 0xFF800000u);
+        if (!same_or_nan((double)f2, widen(f2)) || !same_or_nan((double)f3, widen(f3)) || !same_or_nan((double)f4, widen(f4))) ++local;
     }
     if (local) atomicAdd(bad, local);
 }

@@ -541,8 +541,8 @@ long long closure_count(int C1, int C2, int C3, int sx, int sz, int ox, int oz);
 
 // div_rn and qdiv against the hardware division on n random operand pairs (mismatches added to *bad)
 int selftest_division(long long n, unsigned long long seed, unsigned long long *bad, cudaStream_t st);
-// the training features' roots against their error bounds (ark_closure.cu)
-void selftest_roots(long long n, unsigned long long seed, unsigned long long *bad, cudaStream_t st);
+// the training features' roots against their error bounds and narrow against the conversion (ark_closure.cu)
+void selftest_closure(long long n, unsigned long long seed, unsigned long long *bad, cudaStream_t st);
 
 // Between a contiguous double staging buffer (rows of w values) and the device's padded rows
 // (pitch): dst = (T)(src - offset), dst = (double)src + offset, and for FP32 contexts the face

@@ -253,8 +253,10 @@ int ark_vorticity(ark_ctx *ctx, double *out);
  * with a prepared significand reciprocal (run constants, dt), the same with the numerator
  * doubled, the per-cell divisor's reciprocal built by integer Newton steps and its quotients,
  * the exact halving, and the Markstein form q = a*RN(1/b) with two corrections that the rare
- * cases fall back to; also that the device prepares the same reciprocals as the host, and that the
- * square and cube roots of the closure's training features are within their FP64 error bounds.
+ * cases fall back to; also that the device prepares the same reciprocals as the host, that the
+ * products on the integer pipes and the integer conversions between FP32 and FP64 equal the GPU's own
+ * bit for bit over the whole exponent range, and that the square and cube roots of the closure's training
+ * features are within their FP64 error bounds.
  * *mismatches receives the count (0 expected).
  * Runs on the current device. */
 int ark_selftest_division(long long n, unsigned long long seed, long long *mismatches);
