@@ -36,14 +36,10 @@ static_assert(O_B3 + 1 == NPARAM, "parameter layout");
 
 // ---- network ------------------------------------------------------------------------------
 
-// GELU in its tanh form, z (1 + tanh(k0 (z + k1 z^3))) / 2, and its derivative (training:
-// accurate tanhf)
+// GELU in its tanh form, z (1 + tanh(k0 (z + k1 z^3))) / 2 (accurate tanhf; with its derivative, for
+// training: gelu_both)
 constexpr float GK0 = 0.79788456080286536f, GK1 = 0.044715f;
 __device__ __forceinline__ float gelu(float z) { return 0.5f * z * (1.0f + tanhf(GK0 * (z + GK1 * z * z * z))); }
-__device__ __forceinline__ float gelu_grad(float z) {
-    const float th = tanhf(GK0 * (z + GK1 * z * z * z));
-    return 0.5f * (1.0f + th) + 0.5f * z * (1.0f - th * th) * GK0 * (1.0f + 3.0f * GK1 * z * z);
-}
 // inference: the same form with the hardware tanh approximation (relative error below 2^-10)
 __device__ __forceinline__ float tanh_approx(float x) {
     float y;
@@ -60,28 +56,6 @@ struct Net {
     float w[NPARAM];
     float mu[NIN], rsd[NIN];
 };
-
-// nu_t / nu of one normalised input, fully unrolled (with the parameters a kernel argument,
-// every multiply-add takes its weight from the constant bank)
-__device__ __forceinline__ float mlp_forward_unrolled(const float *w, const float xn[NIN]) {
-    float h1[NH];
-#pragma unroll
-    for (int k = 0; k < NH; ++k) {
-        float z = w[O_B1 + k];
-#pragma unroll
-        for (int i = 0; i < NIN; ++i) z += w[O_W1 + k * NIN + i] * xn[i];
-        h1[k] = gelu(z);
-    }
-    float z3 = w[O_B3];
-#pragma unroll
-    for (int k = 0; k < NH; ++k) {
-        float z = w[O_B2 + k];
-#pragma unroll
-        for (int m = 0; m < NH; ++m) z += w[O_W2 + k * NH + m] * h1[m];
-        z3 += w[O_W3 + k] * gelu(z);
-    }
-    return softplus(z3);
-}
 
 // nu_t / nu of one normalised input (w: the parameters, in shared memory)
 __device__ __forceinline__ float mlp_forward(const float *w, const float xn[NIN]) {
@@ -221,15 +195,11 @@ __device__ __forceinline__ float tc_warp(const float *w, const TcWeights &B, __n
 __device__ __forceinline__ float sroot3(float x) { return cbrtf(x); }
 __device__ __forceinline__ float sroot4(float x) { return copysignf(sqrtf(sqrtf(fabsf(x))), x); }
 __device__ __forceinline__ float sroot6(float x) { return copysignf(cbrtf(sqrtf(fabsf(x))), x); }
-__device__ __forceinline__ double sroot3(double x) { return cbrt(x); }
-__device__ __forceinline__ double sroot4(double x) { return copysign(sqrt(sqrt(fabs(x))), x); }
-__device__ __forceinline__ double sroot6(double x) { return copysign(cbrt(sqrt(fabs(x))), x); }
 
-// The 10 raw features from the velocity gradient A[m][d] = d u_m / d x_d of a cell at height y
-// (R = float for inference, double for training data).
-template <class R>
-__device__ __forceinline__ void features_of(const R A[3][3], R y, R ly, R yplus_scale, R f[NIN]) {
-    R S[3][3], W[3][3];
+// The 10 raw features from the velocity gradient A[m][d] = d u_m / d x_d of a cell at height y, for
+// inference (training data: features_fp64).
+__device__ __forceinline__ void features_of(const float A[3][3], float y, float ly, float yplus_scale, float f[NIN]) {
+    float S[3][3], W[3][3];
 #pragma unroll
     for (int a = 0; a < 3; ++a)
 #pragma unroll
@@ -237,15 +207,15 @@ __device__ __forceinline__ void features_of(const R A[3][3], R y, R ly, R yplus_
             S[a][b] = 0.5f * (A[a][b] + A[b][a]);
             W[a][b] = 0.5f * (A[a][b] - A[b][a]);
         }
-    R S2[3][3], W2[3][3], W2S[3][3], W2S2[3][3], WS2[3][3];
-    auto mul = [](const R X[3][3], const R Y[3][3], R Z[3][3]) {
+    float S2[3][3], W2[3][3], W2S[3][3], W2S2[3][3], WS2[3][3];
+    auto mul = [](const float X[3][3], const float Y[3][3], float Z[3][3]) {
 #pragma unroll
         for (int a = 0; a < 3; ++a)
 #pragma unroll
             for (int b = 0; b < 3; ++b) Z[a][b] = X[a][0] * Y[0][b] + X[a][1] * Y[1][b] + X[a][2] * Y[2][b];
     };
-    auto tr_of = [](const R X[3][3], const R Y[3][3]) {
-        R t = 0;
+    auto tr_of = [](const float X[3][3], const float Y[3][3]) {
+        float t = 0.f;
 #pragma unroll
         for (int a = 0; a < 3; ++a)
 #pragma unroll
@@ -257,20 +227,20 @@ __device__ __forceinline__ void features_of(const R A[3][3], R y, R ly, R yplus_
     mul(W2, S, W2S);
     mul(W2S, S, W2S2);
     mul(W, S2, WS2);
-    const R trS = S[0][0] + S[1][1] + S[2][2];
-    const R trS2 = S2[0][0] + S2[1][1] + S2[2][2];
-    const R trW2 = W2[0][0] + W2[1][1] + W2[2][2];
+    const float trS = S[0][0] + S[1][1] + S[2][2];
+    const float trS2 = S2[0][0] + S2[1][1] + S2[2][2];
+    const float trW2 = W2[0][0] + W2[1][1] + W2[2][2];
     f[0] = trS;
-    f[1] = sqrt(trS2 > 0 ? trS2 : (R)0);
-    f[2] = sqrt(-trW2 > 0 ? -trW2 : (R)0);
+    f[1] = sqrtf(trS2 > 0 ? trS2 : 0.f);
+    f[2] = sqrtf(-trW2 > 0 ? -trW2 : 0.f);
     f[3] = sroot3(tr_of(S2, S));
     f[4] = sroot3(W2S[0][0] + W2S[1][1] + W2S[2][2]);
     f[5] = sroot4(W2S2[0][0] + W2S2[1][1] + W2S2[2][2]);
     f[6] = sroot6(tr_of(W2S, WS2));
-    const R sg = y > 0 ? (R)-1 : (y < 0 ? (R)1 : (R)0);
+    const float sg = y > 0 ? -1.f : (y < 0 ? 1.f : 0.f);
     f[7] = sg * S[0][1];
     f[8] = sg * W[0][1];
-    f[9] = ((R)0.5 * ly - fabs(y)) * yplus_scale;
+    f[9] = (0.5f * ly - fabsf(y)) * yplus_scale;
 }
 
 // x^(1/2) and x^(1/3) of x >= 0 for the training data: the FP32 root of x (truncated to 24 bits by
@@ -653,7 +623,7 @@ template <class FA, class FB> __device__ __forceinline__ void mma_samples(float 
         mma_bf16(c, alo, b0.hi, b1.hi);
     }
 }
-// GELU and its derivative (gelu, gelu_grad) from one tanh
+// GELU and its derivative from one tanh
 __device__ __forceinline__ void gelu_both(float z, float &h, float &d) {
     const float th = tanhf(GK0 * (z + GK1 * z * z * z));
     h = 0.5f * z * (1.0f + th);
@@ -1089,7 +1059,7 @@ template <class T> __global__ void __launch_bounds__(128)
                 A[m][2] = (v[5] - v[4]) * K.rdx2[2];
             }
             const float y = -0.5f * K.ly + ((float)j - 0.5f) * K.dy;
-            features_of<float>(A, y, K.ly, K.yplus, f);
+            features_of(A, y, K.ly, K.yplus, f);
 #pragma unroll
             for (int q = 0; q < NIN; ++q) f[q] = (f[q] - net.mu[q]) * net.rsd[q];
         }
