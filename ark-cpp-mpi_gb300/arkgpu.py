@@ -30,7 +30,7 @@ EXPORTS = ("ark_create", "ark_destroy", "ark_last_error", "ark_status_string", "
            "ark_time_step_size", "ark_phase1", "ark_stress_tensor", "ark_use_forces", "ark_phase2",
            "ark_boundary_fill", "ark_boundary_conditions", "ark_set_dt", "ark_step", "ark_sync", "ark_time_steps",
            "ark_get_scalars", "ark_set_scalars", "ark_conservation_sums", "ark_channel_init",
-           "ark_kernel_times", "ark_kernel_name", "ark_step_kernel_name", "ark_alloc_host_state", "ark_free_host_state",
+           "ark_captured_launches", "ark_kernel_times", "ark_kernel_name", "ark_step_kernel_name", "ark_alloc_host_state", "ark_free_host_state",
            "ark_conservation_sums_noalloc", "ark_mean_profile", "ark_selftest_division", "ark_selftest_staging_timeout",
            "ark_ensemble_create", "ark_ensemble_destroy", "ark_ensemble_last_error", "ark_ensemble_size",
            "ark_ensemble_upload", "ark_ensemble_download", "ark_ensemble_step", "ark_ensemble_sync",
@@ -129,6 +129,7 @@ def lib():
         L.ark_conservation_sums.argtypes = [vp, ctypes.POINTER(Sums)]
         L.ark_channel_init.argtypes = [ctypes.POINTER(Params), ctypes.c_uint64, ctypes.c_double,
                                        ctypes.POINTER(HostState)]
+        L.ark_captured_launches.argtypes = [vp, ip]
         L.ark_kernel_times.argtypes = [vp, ctypes.c_int, _DP, ctypes.c_int, ip]
         L.ark_kernel_name.restype = ctypes.c_char_p
         L.ark_kernel_name.argtypes = [ctypes.c_int]
@@ -386,6 +387,12 @@ class Context:
         ms = ctypes.c_double(0.0)
         self._call("ark_time_steps", int(n), ctypes.byref(ms))
         return ms.value
+
+    def captured_launches(self):
+        """Kernels that one step() launches (a step's captured graph)."""
+        n = ctypes.c_int(0)
+        self._call("ark_captured_launches", ctypes.byref(n))
+        return n.value
 
     def kernel_times(self, nsteps):
         """Mean device ms of each launch of the fused step: list of (name, ms)."""

@@ -1001,9 +1001,21 @@ static int capture_steps(ark_ctx *ctx, int n, cudaGraphExec_t *exec) {
         if (graph) cudaGraphDestroy(graph);
         return fail(ARK_ERR_CUDA, std::string("step capture: ") + cudaGetErrorString(le != cudaSuccess ? le : ce));
     }
-    cudaError_t ie = cudaGraphInstantiate(exec, graph, 0);
+    size_t nodes = 0;
+    cudaError_t ie = cudaGraphGetNodes(graph, nullptr, &nodes);
+    std::vector<cudaGraphNode_t> node(nodes);
+    if (ie == cudaSuccess) ie = cudaGraphGetNodes(graph, node.data(), &nodes);
+    int kernels = 0;
+    for (size_t q = 0; q < nodes && ie == cudaSuccess; ++q) {
+        cudaGraphNodeType type;
+        ie = cudaGraphNodeGetType(node[q], &type);
+        kernels += ie == cudaSuccess && type == cudaGraphNodeTypeKernel;
+    }
+    if (ie == cudaSuccess) ie = cudaGraphInstantiate(exec, graph, 0);
     cudaGraphDestroy(graph);
-    if (ie != cudaSuccess) {
+    if (ie == cudaSuccess) {
+        ctx->step_kernels = kernels / n;
+    } else {
         *exec = nullptr;
         return fail(ARK_ERR_CUDA, std::string("graph instantiate: ") + cudaGetErrorString(ie));
     }
@@ -1101,6 +1113,14 @@ int ark_time_steps(ark_ctx *ctx, int nsteps, double *ms) {
     ARK_CUDA(cudaEventElapsedTime(&f, ctx->ev0, ctx->ev1));
     *ms = (double)f;
     return ark_sync(ctx);
+}
+
+int ark_captured_launches(ark_ctx *ctx, int *kernels) {
+    if (int rc = check_ctx(ctx, true)) return rc;
+    if (!kernels) return fail(ARK_ERR_PARAM, "kernels is NULL");
+    if (int rc = ensure_graph(ctx)) return rc; // (a graph in hand was captured with the same shapes)
+    *kernels = ctx->step_kernels;
+    return ARK_OK;
 }
 
 int ark_kernel_times(ark_ctx *ctx, int nsteps, double *ms, int cap, int *count) {

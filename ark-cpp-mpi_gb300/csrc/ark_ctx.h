@@ -85,6 +85,7 @@ struct ark_ctx {
     int march[2] = {1, 0};    // Phase1 kernel shape of the two Phase1 launches of a step
     cudaGraphExec_t graph[2][2] = {{nullptr, nullptr}, {nullptr, nullptr}}; // [con][fcur]
     cudaGraphExec_t chain[2][2] = {{nullptr, nullptr}, {nullptr, nullptr}}; // the same of kChain steps
+    int step_kernels = 0;     // kernels of the step captured last
     const void *graph_levels[2][2][3] = {};  // the level buffers each graph was captured with
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     double *stage = nullptr; // contiguous double staging for host transfers

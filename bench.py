@@ -88,12 +88,6 @@ def ncu_traffic_per_cell():
     return out
 
 
-def captured_launches(ktimes, fp64):
-    """Kernels of a captured step, of the launches timed one by one: dt and the ghost fill are one, and in
-    FP64 the three sweeps are one."""
-    return len(ktimes) - 1 - (2 if fp64 else 0)
-
-
 def ncu_fp64_pipe():
     """FP64 pipe activity (fraction of its peak) of each FP64 kernel from the committed ncu
     summary (or {})."""
@@ -224,9 +218,10 @@ def gpu_leg(arkgpu, C, re_b, precision, steps, warmup, device, seed, kernel_step
         with ClockSampler(device) as clk:
             ms = ctx.time_steps(steps)
         clocks = clk.summary()
+        launches = ctx.captured_launches()
         ktimes = ctx.kernel_times(kernel_steps)
         sc = ctx.scalars()
-    return {"cells": cells, "ms": ms, "clocks": clocks, "ktimes": ktimes, "dt": sc.dt, "ub": sc.bulk_velocity,
+    return {"cells": cells, "ms": ms, "clocks": clocks, "ktimes": ktimes, "launches": launches, "dt": sc.dt, "ub": sc.bulk_velocity,
             "shapes": shapes}
 
 
@@ -476,7 +471,7 @@ def main():
     ms = max_over_ranks(dist, g["ms"])
     total_cells = g["cells"] * world
     value = total_cells * args.steps / (ms * 1e-3) / 1e6
-    launches_per_step = captured_launches(g["ktimes"], True)
+    launches_per_step = g["launches"]
 
     line = {"metric": METRIC, "value": round(value, 3), "unit": UNIT, "n_gpus": world, "steps": args.steps,
             "warmup": args.warmup, "ms_per_step": round(ms / args.steps, 4), "higher_is_better": True,
@@ -509,7 +504,7 @@ def main():
                                           "frac": round(f["cells"] * STEP_VALUES * 4 / f_step_s / 1e9 / peak, 4)},
                         "kernels_ms": {k: round(v, 4) for k, v in f["ktimes"]}, "clocks": f["clocks"],
                         "kernel_shapes": f["shapes"], "error": fp32_error_report()}
-        line["gpu_launches"] += captured_launches(f["ktimes"], False) * f_steps
+        line["gpu_launches"] += f["launches"] * f_steps
 
     if rank == 0 and args.ensemble > 0:
         e = ensemble_leg(arkgpu, args.ensemble, args.ensemble_steps, args.warmup, device, shape=args.ensemble_shape)

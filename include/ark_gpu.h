@@ -182,6 +182,10 @@ int ark_sync(ark_ctx *ctx);
  * the context's stream around them (milliseconds). */
 int ark_time_steps(ark_ctx *ctx, int nsteps, double *ms);
 
+/* The kernels that a step of ark_step launches with ctx's current shapes (its captured graph's kernel
+ * nodes: some of ark_kernel_times' launches are one there). */
+int ark_captured_launches(ark_ctx *ctx, int *kernels);
+
 /* Runs nsteps un-graphed fused steps with a CUDA event after every launch and writes the
  * mean device time of each launch (ms) into ms[0..cap-1], in step order; *count receives the
  * number of launches per step.  ark_kernel_name(i) names launch i. */
