@@ -2108,11 +2108,12 @@ __global__ void __launch_bounds__(128, 9) k_sweep_y_seams(const __grid_constant_
 }
 
 // The three sweeps in one launch of independent blocks: x1 (n1 blocks), x2 (n2, c2 to a segment), x3 (c3 to
-// a segment).  One after the other, each ends in a wave that leaves most SMs idle: FP64 64x32x32 96 -> 90
-// us per step, 200x60x1 56 -> 47, 128x96x96 1082 -> 1021, 256x128x128 3383 -> 3358; FP32 with the closure
-// 64x48x48 43 -> 40.  The registers are the x1 sweep's for all (FP64 three blocks per SM, where the
-// column sweeps alone have four; FP32 six instead of nine, so only for grids of a few waves).  (FP64
-// figures before mulq.)
+// a segment).  One after the other, each ends in a wave that leaves most SMs idle: FP64 64x32x32 90 -> 85
+// us per step, 200x60x1 54 -> 44, 128x64x64 446 -> 425, 192x96x96 1,375 -> 1,302, 256x128x96 2,274 -> 2,223;
+// FP32 with the closure 64x48x48 43 -> 40.  The registers are the x1 sweep's for all (FP64 three blocks
+// per SM, where the column sweeps alone have four; FP32 six instead of nine), so only for grids of a few
+// waves: FP32 three, FP64 nine (256x128x128, of eleven: 2,867 in one launch, 2,836 in three;
+// 512x256x128 11,090 and 11,000; at eight and nine either way within 2%).
 template <class T, bool INT>
 __global__ void __launch_bounds__(128, sizeof(T) == 4 ? 6 : 3) k_sweeps(const __grid_constant__ DevState<T> S, int con, int fcur, int gl,
                                                                        int nch, int n1, int seg2, int n2, int c2, int seg3, int c3) {
@@ -2701,7 +2702,7 @@ template <class T> void Launch<T>::sweep_z_seams(const DevState<T> &S, int con, 
 template <class T> bool Launch<T>::sweeps(const DevState<T> &S, int con, int fcur, cudaStream_t st, int target) {
     constexpr bool fp64 = sizeof(T) == 8;
     const SweepCut c = sweep_cut(S.g, target, fp64);
-    if (!fp64 && c.n1 + c.n2 + c.n3 > 3 * 6 * 152) return false;
+    if (c.n1 + c.n2 + c.n3 > (fp64 ? 9 * 3 : 3 * 6) * 152) return false; // waves of three and six blocks per SM
     auto go = [&](auto kernel) {
         launch_early(!fp64 && early_grid(S.g), kernel, dim3(c.n1 + c.n2 + c.n3), dim3(128), 0, st, S, con, fcur, c.gl, c.nch, c.n1,
                      c.seg2, c.n2, c.c2, c.seg3, c.c3);

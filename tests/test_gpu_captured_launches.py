@@ -7,12 +7,14 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("C,prec,form,want", [
-    ((20, 10, 12), "fp64", None, 4),    # the three sweeps in one launch
-    ((20, 10, 12), "fp64", "1", 5),     # one sweep kernel, behind its own ghost fill
-    ((20, 10, 12), "fp32", None, 4),    # x1 and x3 folded in, the seams with the x2 sweep
+    ((20, 10, 12), "fp64", None, 4),     # the three sweeps in one launch
+    ((256, 128, 96), "fp64", None, 4),   # eight waves of them
+    ((256, 128, 128), "fp64", None, 6),  # eleven: three launches
+    ((20, 10, 12), "fp64", "1", 5),      # one sweep kernel, behind its own ghost fill
+    ((20, 10, 12), "fp32", None, 4),     # x1 and x3 folded in, the seams with the x2 sweep
     ((20, 10, 12), "fp32", "0", 4),
-    ((512, 128, 64), "fp32", None, 6),  # the two seam kernels beside the x2 sweep
-    ((512, 128, 64), "fp32", "0", 6),   # three sweeps of more than a few waves
+    ((512, 128, 64), "fp32", None, 6),   # the two seam kernels beside the x2 sweep
+    ((512, 128, 64), "fp32", "0", 6),    # three sweeps of more than a few waves
 ])
 def test_captured_launches(ark, monkeypatch, C, prec, form, want):
     if form is not None:
