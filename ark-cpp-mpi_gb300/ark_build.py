@@ -11,8 +11,9 @@ Translation units are compiled in parallel:
   ark_noalloc.cu  conservation sums over caller-owned device arrays, static scratch (--fmad=false)
   ark_ensemble.cu batched ensembles: persistent kernels over a member table (--fmad=false)
   ark_slabs.cu    one channel split along z into slabs with halo exchanges (host code)
-  ark_output.cu   VTK packing, time averages, kinetic energy (--fmad=false: the averages and
-                  the energy terms round as the reference's)
+  ark_output.cu   VTK packing, time averages, kinetic energy, plane moments (--fmad=false: the averages
+                  round as the reference's; the energy and the moments add their squares by FMA, one
+                  rounding less each)
   ark_closure.cu  learned eddy-viscosity closure: training data, network kernels, inference
   ark_host.cpp host-only helpers (seeded channel init)
 Outputs go to ark-cpp-mpi_gb300/lib/ (git-ignored).

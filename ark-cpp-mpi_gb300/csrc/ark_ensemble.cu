@@ -934,7 +934,8 @@ int ark_ensemble_download(ark_ensemble *E, int q, ark_host_state *h) {
     double *cells[8] = {h->roCon, h->u1Con, h->u2Con, h->u3Con, h->ronCon, h->u1nCon, h->u2nCon, h->u3nCon};
     float *dcell[8] = {S.lv[c].ro, S.lv[c].u1, S.lv[c].u2, S.lv[c].u3, S.lv[n].ro, S.lv[n].u1, S.lv[n].u2, S.lv[n].u3};
     // one staging buffer, one stream: an array's conversion waits for the copy before it, the host for the
-    // last copy only (64 members' eight arrays, 862 MB, after 100 steps: 137.7 -> 136.3 ms)
+    // last copy only (64 members' eight arrays, 862 MB, after 100 steps: 136.2 -> 134.8 ms, medians of five
+    // alternating runs, 0.2 ms apart)
     cudaError_t err = cudaSuccess;
     auto back = [&](double *to, const RowShape &r) {
         if (err == cudaSuccess)

@@ -2361,8 +2361,8 @@ inline double sm_load(long long blocks, double least) {
     return per > least ? (double)per : least;
 }
 // Chunks of 32 positions per warp of the x1 sweep (0: whole lines, gl per warp): taken where they
-// cost at least 5% less.  FP64, us: 64x32x32 34 -> 13 (2 chunks; 1 chunk 16, 3 chunks 18),
-// 200x60x1 136 -> 17 (1 chunk), 128x64x64 83 -> 71; 256x128x128 keeps its lines.
+// cost at least 5% less.  FP64, us: 64x32x32 41 -> 16 (2 chunks; 1 chunk 17, 3 chunks 20),
+// 200x60x1 69 -> 10 (1 chunk), 96x64x64 68 -> 48, 128x64x64 86 -> 79; 256x128x128 keeps its lines.
 inline int x_chunk_blocks(const Geom &g, int nch) {
     const long long total = (long long)g.C2 * g.C3 * (g.C1 + 2), per = 32 * nch - 1;
     return (int)(((total - 1 + per - 1) / per + 3) / 4);
@@ -2384,8 +2384,8 @@ inline int x_chunks_per_warp(const Geom &g, int gl, bool fp64) {
 }
 // Segments of the x2 / x3 sweeps: of at most `target` faces, balanced so no thread gets a short
 // tail; where those are fewer than two waves of four blocks per SM (FP32: one wave of nine), the
-// count with the least load instead, if it is larger.  FP64 (before mulq), us: 64x32x32 66 / 56 -> 23 / 16 (2 faces; 1 face 27 /
-// 19, 4 faces 26 / 18), 200x60x1 x2 153 -> 28 (1 face), 96x64x64 89 / 77 -> 69 / 61.  FP32: 64x48x48
+// count with the least load instead, if it is larger.  FP64, us: 64x32x32 65 / 66 -> 18 / 18 (2 faces; 1 face 21 /
+// 21, 4 faces 23 / 23), 200x60x1 x2 72 -> 12 (1 face), 96x64x64 76 / 78 -> 57 / 57.  FP32: 64x48x48
 // x2 13.6 -> 5.5 (2 faces instead of 13), 150x67x93 17.7 -> 15 (8 instead of 14).
 inline int sweep_segment(int nd, int target, int blocks, bool fp64, int *nseg) {
     const double least = fp64 ? 1.4 : 5.0;
@@ -2424,9 +2424,9 @@ inline SweepCut sweep_cut(const Geom &g, int target, bool fp64) {
     c.n2 = c.c2 * m2;
     c.n3 = c.c3 * m3;
     if (!fp64 || c.n1 + c.n2 + c.n3 > 4 * 3 * 152) return c;
-    // FP64 grids of a few waves (figures before mulq): segments of the x2 and x3 sweeps that fill whole waves of three blocks
-    // per SM (96x64x64: 384 blocks of 18 cells 403 us per step, 576 of 12 cells 430; 128x64x64: 896 of 11
-    // cells 469, 512 of 18 cells 499, 1408 of 7 cells 489)
+    // FP64 grids of a few waves: segments of the x2 and x3 sweeps that fill whole waves of three blocks per
+    // SM (128x64x64, us per step: 10 faces, taken here, 426, 17 faces 458, 6 faces 433; 96x64x64: 17 faces,
+    // taken here, 389, 11 faces 390, and 7 faces, which the count puts later, 365)
     int least = 1 << 30;
     for (int most = 1; most <= target; ++most) {
         const int k2 = (nd2 + most - 1) / most, k3 = (nd3 + most - 1) / most;
