@@ -357,8 +357,9 @@ __global__ void __launch_bounds__(32 * (FY + 2), 4) k_filter_velocity(const __gr
     __shared__ double xs[2][3][FY + 2][32];
     const Geom g = S.g;
     const int tx = threadIdx.x, ty = threadIdx.y;
-    const int i = (int)blockIdx.x * 32 + tx + 1, j = (int)blockIdx.y * FY + ty; // j: rows j0 - 1 .. j0 + FY
-    const int k0 = (int)blockIdx.z * kch + 1, k1 = k0 + kch - 1 < g.C3 ? k0 + kch - 1 : g.C3;
+    const int by = (int)blockIdx.x / ((g.C1 + 31) / 32), bx = (int)blockIdx.x - by * ((g.C1 + 31) / 32);
+    const int i = bx * 32 + tx + 1, j = by * FY + ty; // j: rows j0 - 1 .. j0 + FY
+    const int k0 = (int)blockIdx.y * kch + 1, k1 = k0 + kch - 1 < g.C3 ? k0 + kch - 1 : g.C3;
     const bool live = i <= g.C1 && j >= 1 && j <= g.C2;  // a cell whose x sum is taken
     const bool mine = live && ty >= 1 && ty <= FY;       // and whose box is this thread's
     const int im = i == 1 ? g.C1 : i - 1, ip = i == g.C1 ? 1 : i + 1;
@@ -1268,7 +1269,7 @@ int closure_sample(const DevState<T> &S, int lvl, ark_closure_data *d, double lx
     const int bx = (C1 + 31) / 32, by = (C2 + cl::FY - 1) / cl::FY;
     int kch = C3;
     long long least = 1ll << 60;
-    for (int n = 1; n <= C3; ++n) {
+    for (int n = 1; n <= std::min(C3, 65535); ++n) { // (a grid's y extent)
         const int c = (C3 + n - 1) / n;
         const long long per = ((long long)bx * by * ((C3 + c - 1) / c) + 151) / 152, load = std::max(2ll, per) * (c + 2);
         if (load < least) {
@@ -1276,7 +1277,7 @@ int closure_sample(const DevState<T> &S, int lvl, ark_closure_data *d, double lx
             kch = c;
         }
     }
-    cl::k_filter_velocity<T><<<dim3(bx, by, (C3 + kch - 1) / kch), dim3(32, cl::FY + 2), 0, st>>>(S, lvl, d->scratch, kch, make_qrecip(27.0));
+    cl::k_filter_velocity<T><<<dim3((unsigned)bx * by, (C3 + kch - 1) / kch), dim3(32, cl::FY + 2), 0, st>>>(S, lvl, d->scratch, kch, make_qrecip(27.0));
     cl::SampleArgs s;
     for (int m = 0; m < 3; ++m) s.ub[m] = d->scratch + m * cells;
     s.feat = d->feat;
