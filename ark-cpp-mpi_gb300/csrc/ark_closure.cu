@@ -332,15 +332,10 @@ __device__ __forceinline__ void features_fp64(const double A[3][3], double y, do
 // per box on the integer pipes instead of a division per pass, FP32 starting values for the roots.
 
 // The mean x / 27 of a box from its sum, one rounding where three means of three had three each (the
-// product with RN(1/27), half an ulp from 1/27, was the less precise by a tenth on FP64 fields).  The
-// filter takes the quotient on the integer pipes (256x128x128, the whole call 505 us; on the FP64 pipe
-// 565), k_samples, whose gradients' products are there already, the product and its correction from the
-// exact remainder, within 0.5 + 2^-50 ulp (505; on the integer pipes 536).
+// product with RN(1/27), half an ulp from 1/27, was the less precise by a tenth on FP64 fields), as the
+// quotient on the integer pipes (by a product and its correction on the FP64 pipe the filter takes 60 us
+// more at 256x128x128).
 __device__ __forceinline__ double box_mean(double x, const QRecip &q27) { return qdiv(x, 27.0, 1.0 / 27.0, q27); }
-__device__ __forceinline__ double box_mean_fma(double x) {
-    const double q = __dmul_rn(x, 1.0 / 27.0);
-    return __fma_rn(__fma_rn(-27.0, q, x), 1.0 / 27.0, q);
-}
 
 // The velocities of level lvl of a channel (periodic x and z, solid walls in y: a neighbour beyond a
 // wall counts as minus the cell), box-filtered 3 x 3 x 3, into three compact interior arrays
@@ -416,7 +411,7 @@ struct SampleArgs {
     float *feat, *targ;  // dataset rows written from `at`
     long long at;
     int sx, sz, ox, oz, nx, nz, jc;
-    double rdx2[3], ly, dy, yplus_scale, rnu;
+    double rdx2[3], ly, dy, yplus_scale, rnu27; // rnu27: 1 / (27 nu)
 };
 
 // Features of the filtered field and the least-squares target at the sampled cells (i = ox +
@@ -424,7 +419,7 @@ struct SampleArgs {
 // products u_m u_n are needed at the samples only: a thread marches along jc rows of one (a, b), with
 // the nine cells' products of a row summed in x and z, and the sums of three rows in registers
 // (a row beyond a wall counts as the row itself).  Every product filtered everywhere took 18 passes
-// (1400 us) and 55 us of products; the samples of a 4 x 4 lattice take 177 us with the products in them, the
+// (1400 us) and 55 us of products; the samples of a 4 x 4 lattice take 169 us with the products in them, the
 // FP64 pipe 83% busy (before, 180 without them; the gradients' products on the integer pipes save 4).
 template <class T> __global__ void __launch_bounds__(128) k_samples(const __grid_constant__ DevState<T> S, int lvl, SampleArgs s) {
     const Geom g = S.g;
@@ -472,11 +467,14 @@ template <class T> __global__ void __launch_bounds__(128) k_samples(const __grid
         features_fp64(A, y, s.ly, s.yplus_scale, f);
         const size_t c = ((size_t)k * C2 + j) * C1 + i;
         const double v[3] = {s.ub[0][c], s.ub[1][c], s.ub[2][c]};
+        // 27 tau, of the products' sums as they are: the target's last factor holds the 1/27 (as precise as
+        // six rounded means, 1.79 against 1.84 of 2^-53 u^2 on FP64 fields, by nine FP64 operations for 24)
+        const double v27[3] = {27.0 * v[0], 27.0 * v[1], 27.0 * v[2]};
         double tau[6];
 #pragma unroll
         for (int n = 0; n < 6; ++n) {
             constexpr int p[6] = {0, 0, 0, 1, 1, 2}, q[6] = {0, 1, 2, 1, 2, 2};
-            tau[n] = box_mean_fma((lo[n] + mid[n]) + hi[n]) - v[p[n]] * v[q[n]];
+            tau[n] = __fma_rn(-v27[p[n]], v[q[n]], (lo[n] + mid[n]) + hi[n]);
             lo[n] = mid[n];
             mid[n] = hi[n];
         }
@@ -491,7 +489,7 @@ template <class T> __global__ void __launch_bounds__(128) k_samples(const __grid
         const long long row = s.at + ((long long)b * C2 + j) * s.nx + a;
 #pragma unroll
         for (int q = 0; q < NIN; ++q) s.feat[row * NIN + q] = narrow(f[q]);
-        s.targ[row] = narrow(nut * s.rnu);
+        s.targ[row] = narrow(nut * s.rnu27);
     }
 }
 
@@ -1297,7 +1295,7 @@ int closure_sample(const DevState<T> &S, int lvl, ark_closure_data *d, double lx
     s.ly = ly;
     s.dy = dx[1];
     s.yplus_scale = u_tau / vis;
-    s.rnu = 1.0 / vis;
+    s.rnu27 = 1.0 / (27.0 * vis);
     const long long threads = (long long)nx * nz * ((C2 + s.jc - 1) / s.jc);
     cl::k_samples<T><<<(unsigned)((threads + 127) / 128), 128, 0, st>>>(S, lvl, s);
     CL_CUDA(cudaGetLastError());
